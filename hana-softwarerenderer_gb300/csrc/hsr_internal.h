@@ -95,7 +95,7 @@ struct __align__(128) DView {
   uint32_t clear_rgba;
   // ordering inside the batch: views this one waits for (-1 = none)
   int32_t dep0, dep1;
-  int32_t has_dependents;  // another view of the batch waits for this one's tiles
+  int32_t has_dependents;  // kTargetReaders | kTileReaders: which later views wait for this one's tiles
   uint32_t prim_base;
   // mesh (device)
   const float* px; const float* py; const float* pz;   // positions, SoA, padded to 4
@@ -126,6 +126,10 @@ struct __align__(128) DView {
   int32_t sch_base;
   int32_t cch_base;
 };
+// DView::has_dependents: a later view reads the whole target (a shadow map; this view is the last to
+// write it or one before that), and a later view draws into the same target (each of its tiles
+// waits for this view's tile at the same place).
+constexpr int32_t kTargetReaders = 1, kTileReaders = 2;
 constexpr int kVertexChunk = 2048;  // positions per vertex-stage chunk
 constexpr uint32_t kWorldPos = 1u, kWorldNormal = 2u;  // DView::world
 // The world attributes a shader's fragment() reads (IShader.cpp): the world position for the

@@ -241,8 +241,10 @@ int Runtime::plan_build(const hsr_draw_desc* descs, int n, Plan& p) {
     if (d.flags & HSR_DRAW_CLEAR) p.ncch += (int)(((size_t)tg->w * (size_t)tg->h + kClearChunk - 1) / kClearChunk);
   }
   for (int k = 0; k < n; k++) {
-    if (p.views[k].dep0 >= 0) p.views[p.views[k].dep0].has_dependents = 1;
-    if (p.views[k].dep1 >= 0) p.views[p.views[k].dep1].has_dependents = 1;
+    // the readers of a target wait for every view that writes it (a chain already marked is marked whole)
+    for (int d = p.views[k].dep0; d >= 0 && !(p.views[d].has_dependents & kTargetReaders); d = p.views[d].dep1)
+      p.views[d].has_dependents |= kTargetReaders;
+    if (p.views[k].dep1 >= 0) p.views[p.views[k].dep1].has_dependents |= kTileReaders;
   }
   if (p.total_tiles >= (size_t)kMaxBatchTiles)
     return fail(HSR_ERR_INVALID_ARG, "draw batch: too many tiles for one launch sequence (2^26)");

@@ -41,24 +41,50 @@ __device__ __forceinline__ int find_view(const DView* views, const int32_t* tbas
   return lo;
 }
 
-// Wait until every non-empty tile of view `dep` is done (its empty tiles were cleared in the
-// scatter grid, which runs before the raster).  Bounded: after the poll limit the wait sets
-// kErrWaitTimeout and returns, and once any wait of the sequence has given up the others
-// stop waiting (so a dependency that never completes costs one limit, not one per tile).
-// HSR_FAULT_DEPENDENCY_STALL makes the wait ask for one tile more than the view has.
-__device__ __forceinline__ void wait_view(const Scratch& sc, const DView* views, int dep) {
-  if (dep < 0) return;
-  const int tb = views[dep].tile_base;
-  const uint32_t need = sc.ne_off[tb + views[dep].ntiles] - sc.ne_off[tb] +
-                        ((sc.faults & HSR_FAULT_DEPENDENCY_STALL) ? 1u : 0u);
+// Poll until *p reaches `need`.  Bounded: after the poll limit the wait sets kErrWaitTimeout and
+// gives up, and once any wait of the sequence has given up the others stop waiting (so a
+// dependency that never completes costs one limit, not one per tile).
+__device__ __forceinline__ void wait_at_least(const Scratch& sc, const uint32_t* p, uint32_t need) {
   const long limit = sc.poll_limit > 0 ? (long)sc.poll_limit : kDepWaitPolls;
   long spins = 0;
-  while (*reinterpret_cast<volatile uint32_t*>(&sc.view_done[dep]) < need) {
+  while (*reinterpret_cast<const volatile uint32_t*>(p) < need) {
     if (++spins > limit || (*reinterpret_cast<volatile uint32_t*>(&sc.ctl->error) & kErrWaitTimeout)) {
       atomicOr(&sc.ctl->error, kErrWaitTimeout);
       return;
     }
-    __nanosleep(128);
+    __nanosleep(64);
+  }
+}
+
+// Wait until the target that view `dep` is the last to write (a shadow map) is complete: every
+// non-empty tile of that view and of the earlier views into the same target (its dep1 chain) is
+// done; their empty tiles were cleared in the scatter grid, which runs before the raster.
+// HSR_FAULT_DEPENDENCY_STALL makes the wait ask for one tile more than the view has.
+__device__ __forceinline__ void wait_target(const Scratch& sc, const DView* views, int dep) {
+  for (int d = dep; d >= 0; d = views[d].dep1) {
+    const int tb = views[d].tile_base;
+    const uint32_t need = sc.ne_off[tb + views[d].ntiles] - sc.ne_off[tb] +
+                          ((sc.faults & HSR_FAULT_DEPENDENCY_STALL) ? 1u : 0u);
+    wait_at_least(sc, &sc.view_done[d], need);
+  }
+  __threadfence();
+}
+
+// Wait for tile `lt` of the earlier views into this view's target.  Views of one target share their
+// tile grid and a tile reads no pixel but its own, so the last of them that has records there is
+// the only one to wait for (it waited for those before it).  A finished tile's fill cursor, spent
+// after the binning, holds kTileDone.
+constexpr uint32_t kTileDone = 0xffffffffu;
+__device__ __forceinline__ void wait_tile(const Scratch& sc, const DView* views, int dep, int lt) {
+  if (sc.faults & HSR_FAULT_DEPENDENCY_STALL) {
+    wait_target(sc, views, dep);
+    return;
+  }
+  for (int d = dep; d >= 0; d = views[d].dep1) {
+    const int t = views[d].tile_base + lt;
+    if (sc.tile_count[t] == 0u) continue;
+    wait_at_least(sc, &sc.tile_fill[t], kTileDone);
+    break;
   }
   __threadfence();
 }
@@ -126,6 +152,7 @@ struct RasterSmem {
   CandQueue cq[WARPS];
   float u8f[256], u8n[256];
   int32_t tbase[kSharedViews];
+  uint32_t claim;  // list position of the tile the CTA shares
 };
 
 // Shade the winners of one tile and write colour, depth and prim id (fused clear writes the
@@ -134,20 +161,26 @@ struct RasterSmem {
 // memory (written by the visibility pass, read back from L2), or, with no stash, are evaluated
 // again from its record: the same operations on the same values as in the visibility pass
 // either way, so the same bits.
+//
+// The warp shades the rows of 32 pixels q0, q0 + qstep, ...; `by_warp` (a tile shared by a CTA) gives
+// the warp whose stash holds each winner's weights, relative to the one `stash` belongs to.
 template <int T, int S>
 __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc, const TileState<T * T>& st, int ox,
-                                               int oy, bool clear, const ByteTables& bt, const float* stash) {
+                                               int oy, bool clear, const ByteTables& bt, const float* stash, int q0,
+                                               int qstep, const uint32_t* by_warp) {
   constexpr int PPL = T * T / 32;
   constexpr int NF4 = payload_f4_of<S>();
   const int lane = threadIdx.x & 31;
   uint32_t shaded = 0;
 #pragma unroll 1
-  for (int q = 0; q < PPL; q++) {
+  for (int q = q0; q < PPL; q += qstep) {
     const int p = lane + 32 * q;
     const int x = ox + p % T, y = oy + p / T;
     if (x >= v.W || y >= v.H) continue;
     const size_t idx = (size_t)y * v.W + x;
-    const uint32_t ri = st.rec[p];
+    uint32_t ri = st.rec[p];
+    // without the fused clear the buffer's depth enters here, after the fragments' minimum
+    if (!clear && ri != kNone && st.key[p] >= buffer_key(__ldcg(&v.depth[idx]))) ri = kNone;
     if (ri != kNone) {
       shaded++;
       float b0, b1, b2;
@@ -161,7 +194,8 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
       } else if (stash) {
         pay = ri;
         seq = 0xfffffffeu - (uint32_t)st.key[p];
-        const float4 w = __ldcg(reinterpret_cast<const float4*>(stash) + p);
+        const float* from = by_warp ? stash + (size_t)by_warp[p] * (size_t)stash_floats(T) : stash;
+        const float4 w = __ldcg(reinterpret_cast<const float4*>(from) + p);
         b0 = w.x; b1 = w.y; b2 = w.z;
       } else {
         const RasterRec r = sc.recs[ri];
@@ -203,30 +237,30 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 // The lane whose key is still the minimum after the warp's atomics records the winner's
 // record (two lanes of one step never hold the same key: one triangle covers a pixel
 // once).  Shading then runs once per pixel with a winner.
-// Four-warp CTAs are compiled for 7 per SM (72 registers a thread, fewer spills than at 8 per
-// SM's 64: measured faster on the serving batches, 1.72 -> 1.65 ms).
-template <int T, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_raster(const DView* __restrict__ views, Scratch sc) {
+//
+// A view's tiles start their coverage at once; only shading waits for what it reads of other
+// views (the shadow map; in a draw without the fused clear the depth and alpha that earlier
+// draws left at this tile).
+//
+// SHARED: a whole CTA takes one tile.  Each warp rasterises an equal share of the tile's list
+// into a tile state of its own, the states are merged by the smaller key (the order of the list
+// never matters), and the pixel rows are shaded by the warps in turn.
+template <int T, int WARPS, bool SHARED>
+__device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, const Scratch& sc,
+                                             RasterSmem<T, WARPS>& sm, const int32_t* tbase, uint32_t nlist) {
   constexpr int NPIX = T * T;
   constexpr int PPL = NPIX / 32;
-  extern __shared__ __align__(16) unsigned char raster_smem[];
-  RasterSmem<T, WARPS>& sm = *reinterpret_cast<RasterSmem<T, WARPS>*>(raster_smem);
-  build_byte_tables(sm.u8f, sm.u8n);
-  const int32_t* tbase = sc.nviews <= kSharedViews ? sm.tbase : nullptr;
-  if (tbase)
-    for (int i = threadIdx.x; i < sc.nviews; i += blockDim.x) sm.tbase[i] = views[i].tile_base;
-  __syncthreads();
+  constexpr bool kKeep = TileState<NPIX>::kKeep;
   const ByteTables bt{sm.u8f, sm.u8n};
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   TileState<NPIX>& st = sm.st[warp];
   BatchRecs& br = sm.br[warp];
   CandQueue& cq = sm.cq[warp];
   float* stash = nullptr;
-  if constexpr (!TileState<NPIX>::kKeep) {
+  if constexpr (!kKeep) {
     const uint32_t gw = blockIdx.x * (uint32_t)WARPS + (uint32_t)warp;
     if (sc.stash && gw < sc.stash_warps) stash = sc.stash + (size_t)gw * (size_t)stash_floats(T);
   }
-  if (sc.ctl->error & kErrNoDraw) return;
   const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
 
   // The non-empty tiles are handed out by one counter over their list, two ahead: while a
@@ -234,14 +268,19 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
   // is being claimed, so neither the counter's round trip nor the list lookup waits on the
   // critical path (the list is in tile order and dependencies only point to lower tile
   // indices, so holding later tiles never blocks).
-  const uint32_t nlist = min(sc.ctl->ne_tiles, (uint32_t)sc.ntiles);
   const uint32_t ntiles = (uint32_t)sc.ntiles;
   uint32_t li = 0, li_ahead = 0;  // positions in the list
-  if (lane == 0) {
-    li = atomicAdd(&sc.ctl->tile_next, 1u);
-    li_ahead = atomicAdd(&sc.ctl->tile_next, 1u);
+  if (SHARED) {
+    if (threadIdx.x == 0) sm.claim = atomicAdd(&sc.ctl->tile_next, 1u);
+    __syncthreads();
+    li = sm.claim;
+  } else {
+    if (lane == 0) {
+      li = atomicAdd(&sc.ctl->tile_next, 1u);
+      li_ahead = atomicAdd(&sc.ctl->tile_next, 1u);
+    }
+    li = __shfl_sync(kFull, li, 0);
   }
-  li = __shfl_sync(kFull, li, 0);
   uint32_t t = li < nlist ? sc.tile_list[li] : ntiles;
   uint32_t n = 0, off = 0;
   if (t < ntiles) {
@@ -250,196 +289,271 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
   }
   // views of a warp's tiles only move forward: after the first, search on from the last one
   int vi = t < ntiles ? find_view(views, tbase, sc.nviews, (int)t) : 0;
+  int ready = -1;  // the shadow map's view last seen complete
   for (;;) {
     if (t >= ntiles) break;
-    const uint32_t li_next = __shfl_sync(kFull, li_ahead, 0);
-    if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(&sc.ctl->tile_next, 1u) : nlist;
-    const uint32_t t_next = li_next < nlist ? sc.tile_list[li_next] : ntiles;
-    uint32_t n_next = 0, off_next = 0;
-    if (t_next < ntiles) {
-      n_next = sc.tile_count[t_next];
-      off_next = sc.tile_off[t_next];
-    }
-    if (t_next < ntiles) {  // warm L1 with the next tile's view descriptor line
-      const DView* vn = views + find_view(views, tbase, sc.nviews, (int)t_next);
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(vn));
-    }
-    if (tbase) {
-      while (vi + 1 < sc.nviews && tbase[vi + 1] <= (int)t) vi++;
-    } else {
-      vi = find_view(views, tbase, sc.nviews, (int)t);
+    uint32_t t_next = ntiles, n_next = 0, off_next = 0;
+    if (!SHARED) {
+      const uint32_t li_next = __shfl_sync(kFull, li_ahead, 0);
+      if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(&sc.ctl->tile_next, 1u) : nlist;
+      if (li_next < nlist) t_next = sc.tile_list[li_next];
+      if (t_next < ntiles) {
+        n_next = sc.tile_count[t_next];
+        off_next = sc.tile_off[t_next];
+      }
     }
     const DView& v = views[vi];
-    if (lane == 0) {
-      wait_view(sc, views, v.dep0);
-      wait_view(sc, views, v.dep1);
-    }
-    __syncwarp();
     const int lt = (int)t - v.tile_base;
     const int tx = lt % v.tiles_x, ty = lt / v.tiles_x;
     const int ox = tx * T, oy = ty * T;
     const bool clear = (v.flags & HSR_DRAW_CLEAR) != 0u;
 
-    if (n != 0) {  // always: the list holds the tiles with records
-      if (clear) {  // every pixel starts from the clear depth
-        const unsigned long long k0 = buffer_key(v.clear_depth);
+    // this warp's records: all of the tile's list, or its share of it
+    uint32_t b = 0, end = n;
+    if (SHARED) {
+      b = (n * (uint32_t)warp) / WARPS;
+      end = (n * (uint32_t)(warp + 1)) / WARPS;
+    }
+    {  // every pixel starts from the clear depth, or from nothing where the buffer's is read later
+      const unsigned long long k0 = clear ? buffer_key(v.clear_depth) : ~0ull;
 #pragma unroll 8
-        for (int q = 0; q < PPL; q++) {
-          st.key[lane + 32 * q] = k0;
-          st.rec[lane + 32 * q] = kNone;
-        }
-      } else {
-#pragma unroll 8
-        for (int q = 0; q < PPL; q++) {
-          const int p = lane + 32 * q;
-          const int x = ox + p % T, y = oy + p / T;
-          float d = v.clear_depth;
-          if (x < v.W && y < v.H) d = __ldcg(&v.depth[(size_t)y * v.W + x]);
-          st.key[p] = buffer_key(d);
-          st.rec[p] = kNone;
+      for (int q = 0; q < PPL; q++) {
+        st.key[lane + 32 * q] = k0;
+        st.rec[lane + 32 * q] = kNone;
+      }
+    }
+    uint32_t frags = 0;  // covered candidates of this lane
+    for (; b < end; b += 32) {
+      const uint32_t cnt = min(32u, end - b);
+      uint32_t c = 0, box = 0, ri = kNone;
+      RasterRec rr;
+      if ((uint32_t)lane < cnt) {
+        ri = sc.bins[off + b + (uint32_t)lane];
+        if (ri < nrec) {  // an index past the records never comes from a consistent bin pass
+          rr = sc.recs[ri];
+          const int lx0 = max((int)(rr.xr & 0xffffu) - ox, 0), lx1 = min((int)(rr.xr >> 16) - ox, T - 1);
+          const int ly0 = max((int)(rr.yr & 0xffffu) - oy, 0), ly1 = min((int)(rr.yr >> 16) - oy, T - 1);
+          if (lx0 <= lx1 && ly0 <= ly1) {
+            c = (uint32_t)((lx1 - lx0 + 1) * (ly1 - ly0 + 1));
+            box = (uint32_t)lx0 | ((uint32_t)ly0 << 8) | ((uint32_t)(lx1 - lx0 + 1) << 16);
+          }
         }
       }
-      uint32_t frags = 0;  // covered candidates of this lane
-      for (uint32_t b = 0; b < n; b += 32) {
-        const uint32_t cnt = min(32u, n - b);
-        uint32_t c = 0, box = 0, ri = kNone;
-        RasterRec rr;
-        if ((uint32_t)lane < cnt) {
-          ri = sc.bins[off + b + (uint32_t)lane];
-          if (ri < nrec) {  // an index past the records never comes from a consistent bin pass
-            rr = sc.recs[ri];
-            const int lx0 = max((int)(rr.xr & 0xffffu) - ox, 0), lx1 = min((int)(rr.xr >> 16) - ox, T - 1);
-            const int ly0 = max((int)(rr.yr & 0xffffu) - oy, 0), ly1 = min((int)(rr.yr >> 16) - oy, T - 1);
-            if (lx0 <= lx1 && ly0 <= ly1) {
-              c = (uint32_t)((lx1 - lx0 + 1) * (ly1 - ly0 + 1));
-              box = (uint32_t)lx0 | ((uint32_t)ly0 << 8) | ((uint32_t)(lx1 - lx0 + 1) << 16);
-            }
-          }
-        }
-        uint32_t incl = c;
+      uint32_t incl = c;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(kFull, incl, o);
-          if (lane >= o) incl += y;
-        }
-        const uint32_t W = __shfl_sync(kFull, incl, 31);
-        const uint32_t start = incl - c;
-        const unsigned ne = __ballot_sync(kFull, c > 0u);
-        __syncwarp();
-        if (c > 0u) {  // compact the non-empty runs
-          const int k = __popc(ne & ((1u << lane) - 1u));
-          const uint32_t bits = box | (((rr.view >> kRecFlagShift) & kRecExact) ? 0x80000000u : 0u);
-          br.a4[k] = make_float4(rr.ax, rr.ay, rr.e1x, rr.e1y);
-          br.b4[k] = make_float4(rr.e2x, rr.e2y, rr.uz, __uint_as_float(bits));
-          br.c2[k] = make_uint2(start, kDivMagic[box >> 16]);
-          br.d4[k] = make_float4(rr.d0, rr.d1, rr.d2, __uint_as_float(rr.seq));
-          br.ri[k] = ri;
-        }
-        __syncwarp();
-        // Visibility of `cnt` queued candidates from the ring head, one per lane: weights
-        // (the divisions of barycentric()), depth, and a 64-bit atomicMin of the key.
-        uint32_t qh = 0, qn = 0;  // ring head and queued count (warp-uniform)
-        auto resolve = [&](uint32_t cnt) {
-          __syncwarp();
-          const bool act = (uint32_t)lane < cnt;
-          unsigned long long key = 0ull, old = 0ull;
-          int p = 0, j = 0;
-          float b0 = 0.f, b1 = 0.f, b2 = 0.f;
-          if (act) {
-            const uint32_t e = (qh + (uint32_t)lane) & 63u;
-            const uint32_t jp = cq.jp[e];
-            j = (int)(jp & 31u);
-            p = (int)(jp >> 8);
-            const float2 u = cq.u[e];
-            const float4 d4 = br.d4[j];
-            cover_weights(u.x, u.y, br.b4[j].z, b0, b1, b2);
-            // interpolate_depth (graphics.cpp:186-194)
-            const float z = fa(fa(fa(0.f, fm(d4.z, b2)), fm(d4.y, b1)), fm(d4.x, b0));
-            key = ((unsigned long long)ord_bits(z) << 32) | (unsigned long long)(0xfffffffeu - __float_as_uint(d4.w));
-            old = atomicMin(&st.key[p], key);
-          }
-          __syncwarp();
-          if (act && old > key && st.key[p] == key) {
-            st.rec[p] = br.ri[j];
-            if constexpr (TileState<NPIX>::kKeep) {
-              st.b0[p] = b0;
-              st.b1[p] = b1;
-              st.b2[p] = b2;
-            } else if (stash) {
-              __stcg(reinterpret_cast<float4*>(stash) + p, make_float4(b0, b1, b2, 0.f));
-            }
-          }
-          qh = (qh + cnt) & 63u;
-          qn -= cnt;
-          __syncwarp();
-        };
-        for (uint32_t base = 0; base < W; base += 32) {
-          // runs starting before this window, and a bit per run starting inside it
-          const uint32_t before = (uint32_t)__popc(__ballot_sync(kFull, c > 0u && start < base));
-          const uint32_t here = __reduce_or_sync(
-              kFull, (c > 0u && start >= base && start - base < 32u) ? 1u << (start - base) : 0u);
-          const uint32_t i = base + (uint32_t)lane;
-          bool covered = false;
-          float ux = 0.f, uy = 0.f;
-          int p = 0, j = 0;
-          if (i < W) {
-            // owner: the last run starting at or before candidate i
-            j = (int)(before + (uint32_t)__popc(here & ((2u << lane) - 1u))) - 1;
-            const float4 a4 = br.a4[j], b4 = br.b4[j];
-            const uint2 c2 = br.c2[j];
-            const uint32_t q = i - c2.x;
-            const uint32_t bx = __float_as_uint(b4.w);
-            const uint32_t lw = (bx >> 16) & 255u;
-            const uint32_t qy = (q * c2.y) >> 16;
-            const int lx = (int)(bx & 255u) + (int)(q - qy * lw);
-            const int ly = (int)((bx >> 8) & 255u) + (int)qy;
-            p = ly * T + lx;
-            covered = cover_terms(a4.x, a4.y, a4.z, a4.w, b4.x, b4.y, b4.z, (bx >> 31) != 0u, (float)(ox + lx),
-                                  (float)(oy + ly), ux, uy);
-          }
-          const unsigned cm = __ballot_sync(kFull, covered);
-          if (covered) {  // queue behind the pending ones (at most 31 are pending here)
-            frags++;
-            const uint32_t e = (qh + qn + (uint32_t)__popc(cm & ((1u << lane) - 1u))) & 63u;
-            cq.u[e] = make_float2(ux, uy);
-            cq.jp[e] = (uint32_t)j | ((uint32_t)p << 8);
-          }
-          qn += (uint32_t)__popc(cm);
-          if (qn >= 32u) resolve(32u);
-        }
-        if (qn) resolve(qn);  // before the next batch replaces the runs the queue points to
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const uint32_t W = __shfl_sync(kFull, incl, 31);
+      const uint32_t start = incl - c;
+      const unsigned ne = __ballot_sync(kFull, c > 0u);
+      __syncwarp();
+      if (c > 0u) {  // compact the non-empty runs
+        const int k = __popc(ne & ((1u << lane) - 1u));
+        const uint32_t bits = box | (((rr.view >> kRecFlagShift) & kRecExact) ? 0x80000000u : 0u);
+        br.a4[k] = make_float4(rr.ax, rr.ay, rr.e1x, rr.e1y);
+        br.b4[k] = make_float4(rr.e2x, rr.e2y, rr.uz, __uint_as_float(bits));
+        br.c2[k] = make_uint2(start, kDivMagic[box >> 16]);
+        br.d4[k] = make_float4(rr.d0, rr.d1, rr.d2, __uint_as_float(rr.seq));
+        br.ri[k] = ri;
       }
       __syncwarp();
-      uint32_t shaded = 0;
-      switch (v.shader) {
-        case HSR_SHADER_GROUND: shaded = shade_tile<T, HSR_SHADER_GROUND>(v, sc, st, ox, oy, clear, bt, stash); break;
-        case HSR_SHADER_TOON: shaded = shade_tile<T, HSR_SHADER_TOON>(v, sc, st, ox, oy, clear, bt, stash); break;
-        case HSR_SHADER_TEXTURE: shaded = shade_tile<T, HSR_SHADER_TEXTURE>(v, sc, st, ox, oy, clear, bt, stash); break;
-        case HSR_SHADER_TEXTURE_WITH_LIGHT:
-          shaded = shade_tile<T, HSR_SHADER_TEXTURE_WITH_LIGHT>(v, sc, st, ox, oy, clear, bt, stash);
-          break;
-        case HSR_SHADER_BLINN: shaded = shade_tile<T, HSR_SHADER_BLINN>(v, sc, st, ox, oy, clear, bt, stash); break;
-        case HSR_SHADER_NORMALMAP: shaded = shade_tile<T, HSR_SHADER_NORMALMAP>(v, sc, st, ox, oy, clear, bt, stash); break;
-        case HSR_SHADER_SHADOW: shaded = shade_tile<T, HSR_SHADER_SHADOW>(v, sc, st, ox, oy, clear, bt, stash); break;
-        default: shaded = shade_tile<T, HSR_SHADER_FLAT>(v, sc, st, ox, oy, clear, bt, stash); break;
+      // Visibility of `cnt` queued candidates from the ring head, one per lane: weights
+      // (the divisions of barycentric()), depth, and a 64-bit atomicMin of the key.
+      uint32_t qh = 0, qn = 0;  // ring head and queued count (warp-uniform)
+      auto resolve = [&](uint32_t cnt) {
+        __syncwarp();
+        const bool act = (uint32_t)lane < cnt;
+        unsigned long long key = 0ull, old = 0ull;
+        int p = 0, j = 0;
+        float b0 = 0.f, b1 = 0.f, b2 = 0.f;
+        if (act) {
+          const uint32_t e = (qh + (uint32_t)lane) & 63u;
+          const uint32_t jp = cq.jp[e];
+          j = (int)(jp & 31u);
+          p = (int)(jp >> 8);
+          const float2 u = cq.u[e];
+          const float4 d4 = br.d4[j];
+          cover_weights(u.x, u.y, br.b4[j].z, b0, b1, b2);
+          // interpolate_depth (graphics.cpp:186-194)
+          const float z = fa(fa(fa(0.f, fm(d4.z, b2)), fm(d4.y, b1)), fm(d4.x, b0));
+          key = ((unsigned long long)ord_bits(z) << 32) | (unsigned long long)(0xfffffffeu - __float_as_uint(d4.w));
+          old = atomicMin(&st.key[p], key);
+        }
+        __syncwarp();
+        if (act && old > key && st.key[p] == key) {
+          st.rec[p] = br.ri[j];
+          if constexpr (kKeep) {
+            st.b0[p] = b0;
+            st.b1[p] = b1;
+            st.b2[p] = b2;
+          } else if (stash) {
+            __stcg(reinterpret_cast<float4*>(stash) + p, make_float4(b0, b1, b2, 0.f));
+          }
+        }
+        qh = (qh + cnt) & 63u;
+        qn -= cnt;
+        __syncwarp();
+      };
+      for (uint32_t base = 0; base < W; base += 32) {
+        // runs starting before this window, and a bit per run starting inside it
+        const uint32_t before = (uint32_t)__popc(__ballot_sync(kFull, c > 0u && start < base));
+        const uint32_t here = __reduce_or_sync(
+            kFull, (c > 0u && start >= base && start - base < 32u) ? 1u << (start - base) : 0u);
+        const uint32_t i = base + (uint32_t)lane;
+        bool covered = false;
+        float ux = 0.f, uy = 0.f;
+        int p = 0, j = 0;
+        if (i < W) {
+          // owner: the last run starting at or before candidate i
+          j = (int)(before + (uint32_t)__popc(here & ((2u << lane) - 1u))) - 1;
+          const float4 a4 = br.a4[j], b4 = br.b4[j];
+          const uint2 c2 = br.c2[j];
+          const uint32_t q = i - c2.x;
+          const uint32_t bx = __float_as_uint(b4.w);
+          const uint32_t lw = (bx >> 16) & 255u;
+          const uint32_t qy = (q * c2.y) >> 16;
+          const int lx = (int)(bx & 255u) + (int)(q - qy * lw);
+          const int ly = (int)((bx >> 8) & 255u) + (int)qy;
+          p = ly * T + lx;
+          covered = cover_terms(a4.x, a4.y, a4.z, a4.w, b4.x, b4.y, b4.z, (bx >> 31) != 0u, (float)(ox + lx),
+                                (float)(oy + ly), ux, uy);
+        }
+        const unsigned cm = __ballot_sync(kFull, covered);
+        if (covered) {  // queue behind the pending ones (at most 31 are pending here)
+          frags++;
+          const uint32_t e = (qh + qn + (uint32_t)__popc(cm & ((1u << lane) - 1u))) & 63u;
+          cq.u[e] = make_float2(ux, uy);
+          cq.jp[e] = (uint32_t)j | ((uint32_t)p << 8);
+        }
+        qn += (uint32_t)__popc(cm);
+        if (qn >= 32u) resolve(32u);
       }
-      shaded = __reduce_add_sync(kFull, shaded);
-      frags = __reduce_add_sync(kFull, frags);
-      if (lane == 0) {
-        if (shaded) atomicAdd(&sc.ctl->shaded_px, (unsigned long long)shaded);
-        if (frags) atomicAdd(&sc.ctl->frag_px, (unsigned long long)frags);
+      if (qn) resolve(qn);  // before the next batch replaces the runs the queue points to
+    }
+    if (lane == 0) {
+      if (v.dep0 >= 0 && v.dep0 != ready) wait_target(sc, views, v.dep0);
+      if (v.dep1 >= 0) wait_tile(sc, views, v.dep1, lt);
+    }
+    ready = v.dep0;
+    __syncwarp();
+    const TileState<NPIX>* win = &st;
+    const float* wstash = stash;
+    const uint32_t* by_warp = nullptr;
+    int q0 = 0, qstep = 1;
+    if (SHARED) {
+      // merge into the first warp's state: the smaller key per pixel (equal keys are the same
+      // buffer depth or the same triangle); the other states' record words then hold the
+      // winner's warp
+      __syncthreads();
+      for (int p = threadIdx.x; p < NPIX; p += WARPS * 32) {
+        unsigned long long k = sm.st[0].key[p];
+        int w = 0;
+#pragma unroll
+        for (int o = 1; o < WARPS; o++) {
+          const unsigned long long ko = sm.st[o].key[p];
+          if (ko < k) { k = ko; w = o; }
+        }
+        if (w) {
+          sm.st[0].key[p] = k;
+          sm.st[0].rec[p] = sm.st[w].rec[p];
+          if constexpr (kKeep) {
+            sm.st[0].b0[p] = sm.st[w].b0[p];
+            sm.st[0].b1[p] = sm.st[w].b1[p];
+            sm.st[0].b2[p] = sm.st[w].b2[p];
+          }
+        }
+        if constexpr (!kKeep) sm.st[1].rec[p] = (uint32_t)w;
       }
+      __syncthreads();
+      win = &sm.st[0];
+      q0 = warp;
+      qstep = WARPS;
+      if constexpr (!kKeep) {
+        by_warp = sm.st[1].rec;
+        if (stash) wstash = stash - (size_t)warp * (size_t)stash_floats(T);
+      }
+    }
+    uint32_t shaded = 0;
+#define HSR_SHADE(S) shaded = shade_tile<T, S>(v, sc, *win, ox, oy, clear, bt, wstash, q0, qstep, by_warp); break
+    switch (v.shader) {
+      case HSR_SHADER_GROUND: HSR_SHADE(HSR_SHADER_GROUND);
+      case HSR_SHADER_TOON: HSR_SHADE(HSR_SHADER_TOON);
+      case HSR_SHADER_TEXTURE: HSR_SHADE(HSR_SHADER_TEXTURE);
+      case HSR_SHADER_TEXTURE_WITH_LIGHT: HSR_SHADE(HSR_SHADER_TEXTURE_WITH_LIGHT);
+      case HSR_SHADER_BLINN: HSR_SHADE(HSR_SHADER_BLINN);
+      case HSR_SHADER_NORMALMAP: HSR_SHADE(HSR_SHADER_NORMALMAP);
+      case HSR_SHADER_SHADOW: HSR_SHADE(HSR_SHADER_SHADOW);
+      default: HSR_SHADE(HSR_SHADER_FLAT);
+    }
+#undef HSR_SHADE
+    shaded = __reduce_add_sync(kFull, shaded);
+    frags = __reduce_add_sync(kFull, frags);
+    if (lane == 0) {
+      if (shaded) atomicAdd(&sc.ctl->shaded_px, (unsigned long long)shaded);
+      if (frags) atomicAdd(&sc.ctl->frag_px, (unsigned long long)frags);
     }
     if (v.has_dependents) {
       // publish this tile's writes before counting it done (a later view reads them)
       __threadfence();
-      __syncwarp();
-      if (lane == 0) atomicAdd(&sc.view_done[vi], 1u);
+      if (SHARED) __syncthreads(); else __syncwarp();
+      if (SHARED ? threadIdx.x == 0 : lane == 0) {
+        if (v.has_dependents & kTargetReaders) atomicAdd(&sc.view_done[vi], 1u);
+        if (v.has_dependents & kTileReaders) atomicExch(&sc.tile_fill[t], kTileDone);
+      }
+    }
+    if (SHARED) {
+      __syncthreads();  // the merged state and the claim word are free again
+      if (threadIdx.x == 0) sm.claim = atomicAdd(&sc.ctl->tile_next, 1u);
+      __syncthreads();
+      li = sm.claim;
+      if (li < nlist) t_next = sc.tile_list[li];
+      if (t_next < ntiles) {
+        n_next = sc.tile_count[t_next];
+        off_next = sc.tile_off[t_next];
+      }
     }
     t = t_next;
     n = n_next;
     off = off_next;
+    if (t < ntiles) {
+      if (tbase) {
+        while (vi + 1 < sc.nviews && tbase[vi + 1] <= (int)t) vi++;
+      } else {
+        vi = find_view(views, tbase, sc.nviews, (int)t);
+      }
+    }
   }
+}
+
+// With few non-empty tiles most warps have none and the sequence lasts as long as its longest tile:
+// up to kSharedTilesPerCta tiles per CTA of the grid, each CTA takes a tile (tile 8, one draw each:
+// 91 tiles 24.6 -> 10.2 us, 1,026 tiles 32.8 -> 16.4 us, 1,369 tiles 34.8 -> 18.4 us; tile 16, 687
+// tiles of a served request 98 -> 31 us).  Far more tiles keep every warp busy by themselves, and
+// the barriers cost: the two are equal at about 10 tiles per CTA (86 us each at 10.6) and one
+// warp per tile wins by 1.55x at 20 (113 against 176 us) and 1.7x at 47.
+constexpr uint32_t kSharedTilesPerCta = 4;
+
+// Four-warp CTAs are compiled for 7 per SM (72 registers a thread, fewer spills than at 8 per
+// SM's 64: measured faster on the serving batches, 1.72 -> 1.65 ms).
+template <int T, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_raster(const DView* __restrict__ views, Scratch sc) {
+  extern __shared__ __align__(16) unsigned char raster_smem[];
+  RasterSmem<T, WARPS>& sm = *reinterpret_cast<RasterSmem<T, WARPS>*>(raster_smem);
+  build_byte_tables(sm.u8f, sm.u8n);
+  const int32_t* tbase = sc.nviews <= kSharedViews ? sm.tbase : nullptr;
+  if (tbase)
+    for (int i = threadIdx.x; i < sc.nviews; i += blockDim.x) sm.tbase[i] = views[i].tile_base;
+  __syncthreads();
+  if (sc.ctl->error & kErrNoDraw) return;
+  const uint32_t nlist = min(sc.ctl->ne_tiles, (uint32_t)sc.ntiles);
+  // uniform over the grid: every warp of every CTA has a stash, or none does
+  const bool stashes = TileState<T * T>::kKeep || !sc.stash || gridDim.x * (uint32_t)WARPS <= sc.stash_warps;
+  if (nlist <= kSharedTilesPerCta * gridDim.x && stashes)
+    raster_tiles<T, WARPS, true>(views, sc, sm, tbase, nlist);
+  else
+    raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist);
 }
 
 template <int T, int WARPS>

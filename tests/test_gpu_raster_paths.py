@@ -1,0 +1,88 @@
+"""The raster's two ways of handing out tiles (a warp per tile, a CTA per tile where tiles are
+few) and the order of draws into one target, against the oracle.
+
+Depth, primitive ids and alpha are exact, RGB within 1 LSB (powf)."""
+import numpy as np
+import pytest
+
+import golden_io
+import oracle
+from hsr import frame as hframe
+from hsr import scenes
+from hsr import uniforms as U
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def tuned(gpu):
+    old = gpu.get_tuning()
+    yield gpu
+    gpu.set_tuning(tile=old.tile, warps_per_cta=old.warps_per_cta, ctas_per_sm=old.ctas_per_sm)
+
+
+def _check(got, rb, label):
+    golden_io.assert_pass(got, {"depth": rb.depth, "color": rb.color, "prim": rb.prim}, "main", label, 1)
+
+
+# one CTA per SM puts the line between the paths at a few hundred tiles, eight at a few thousand
+@pytest.mark.parametrize("ctas", [1, 8])
+@pytest.mark.parametrize("tile,warps", [(8, 4), (8, 8), (16, 4), (32, 4)])
+@pytest.mark.parametrize("size", [(1, 1), (37, 29), (518, 391)])
+def test_tiles_by_warp_and_by_cta_vs_oracle(tuned, size, tile, warps, ctas):
+    """A tie soup of heavy overdraw and a shadowed normal-map frame at one tile, few and many."""
+    tuned.set_tuning(tile=tile, warps_per_cta=warps, ctas_per_sm=ctas)
+    w, h = size
+    soup = scenes.soup_frame(3000, w, h, seed=w + tile, median_edge_px=max(2.0, w / 12), dup_frac=0.05)
+    shaded = scenes.sphere_frame(3, w, h, shader=scenes.NORMALMAP, eye=(0.3, 0.4, 2.2), tex_size=32, seed=3, shadow=96,
+                                 nm_size=16)
+    for fr in (soup, shaded):
+        g = hframe.GpuFrame(fr)
+        try:
+            g.render()
+            got = g.download()
+        finally:
+            g.release()
+        for k, rb in oracle.render_frame(fr).items():
+            _check(got[k], rb, f"{fr.name} {k} tile{tile}x{warps} ctas{ctas}")
+
+
+@pytest.mark.parametrize("ctas", [1, 8])
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("size", [(90, 70), (700, 400)])
+def test_draws_into_one_target_follow_each_other(tuned, size, tile, ctas):
+    """Four objects into one target and one shadow map in one batch (only the first of each clears),
+    some tiles without records in some of them: each draw tests against what the earlier ones left,
+    and every main draw sees the whole shadow map."""
+    import hsr
+
+    tuned.set_tuning(tile=tile, warps_per_cta=4, ctas_per_sm=ctas)
+    w, h = size
+    rng = np.random.default_rng(w + tile)
+    objs, clear = [], ((0, 0, 0, 255), 1.0)
+    for k in range(4):
+        fr = scenes.sphere_frame(2 + k % 2, w, h, shader=scenes.BLINN, tex_size=16, seed=k)
+        place = U.Mat4.identity()
+        for i in range(3):
+            place.r[i][3] = np.float32(rng.uniform(-0.4, 0.4))
+            place.r[i][i] = np.float32(0.55)
+        objs.append((fr, U.shader_data((0.2, 0.3, 2.5), w, h, model=place, enable_shadow=True)))
+    main, smap = hsr.Target(w, h), hsr.Target(64, 64)
+    meshes, texs = [hsr.Mesh(f.mesh) for f, _ in objs], [hsr.Texture(f.diffuse) for f, _ in objs]
+    try:
+        descs = [hsr.make_desc(m, scenes.SHADOW, sd, smap, t, clear=clear if k == 0 else None)
+                 for k, (m, t, (_, sd)) in enumerate(zip(meshes, texs, objs))]
+        descs += [hsr.make_desc(m, scenes.BLINN, sd, main, t, shadow_map=smap, prim_base=1000 * k,
+                                clear=clear if k == 0 else None) for k, (m, t, (_, sd)) in enumerate(zip(meshes, texs, objs))]
+        hsr.draw_batch(descs)
+        got, got_s = main.download(), smap.download()
+    finally:
+        for o in [main, smap, *meshes, *texs]:
+            o.release()
+    rb, rs = oracle.Buffers(w, h, *clear), oracle.Buffers(64, 64, *clear)
+    for fr, sd in objs:
+        oracle.draw(fr.mesh, scenes.SHADOW, sd, rs, fr.diffuse)
+    for k, (fr, sd) in enumerate(objs):
+        oracle.draw(fr.mesh, scenes.BLINN, sd, rb, fr.diffuse, shadow_map=rs, prim_base=1000 * k)
+    _check(got_s, rs, "shadow map")
+    _check(got, rb, "main")
