@@ -61,32 +61,30 @@ __device__ __forceinline__ float4 mat_vec(const float* m, float x, float y, floa
 }
 
 // ---- Color (color.cpp:38-64) ------------------------------------------------------------
+// std::min(std::max(0.f, x), 1.f) gives 0 for a NaN x and +0 for -0, as the saturating forms of
+// the multiply and the add do: the clamp costs no instruction.
 struct Col { float r, g, b, a; };
 __device__ __forceinline__ Col c_add(Col a, Col b) {
-  return {std_min(std_max(0.f, fa(a.r, b.r)), 1.f), std_min(std_max(0.f, fa(a.g, b.g)), 1.f),
-          std_min(std_max(0.f, fa(a.b, b.b)), 1.f), std_min(std_max(0.f, fa(a.a, b.a)), 1.f)};
+  return {__saturatef(fa(a.r, b.r)), __saturatef(fa(a.g, b.g)), __saturatef(fa(a.b, b.b)), __saturatef(fa(a.a, b.a))};
 }
 __device__ __forceinline__ Col c_mulf(Col a, float t) {
-  t = (t > 1.f ? 1.f : (t < 0.f ? 0.f : t));
-  return {std_min(std_max(0.f, fm(a.r, t)), 1.f), std_min(std_max(0.f, fm(a.g, t)), 1.f),
-          std_min(std_max(0.f, fm(a.b, t)), 1.f), std_min(std_max(0.f, fm(a.a, t)), 1.f)};
+  // a NaN t gives 0 either way: clamped here, or as a NaN product there
+  t = __saturatef(t);
+  return {__saturatef(fm(a.r, t)), __saturatef(fm(a.g, t)), __saturatef(fm(a.b, t)), __saturatef(fm(a.a, t))};
 }
 __device__ __forceinline__ Col c_mulc(Col a, Col b) { return {fm(a.r, b.r), fm(a.g, b.g), fm(a.b, b.b), fm(a.a, b.a)}; }
 __device__ __forceinline__ Col c_of(const float* p) { return {p[0], p[1], p[2], p[3]}; }
 
 // ---- byte -> float tables --------------------------------------------------------------
-// Colour channels and normal-map components are bytes; their float values are the IEEE
-// results b/255.f (color.cpp:5, renderbuffer.cpp:46) and (b/255.f)*2.f - 1.f
-// (IShader.h:97), computed once per CTA into shared memory with the same operations.
+// Colour channels and normal-map components are bytes; their float value is the IEEE result
+// b/255.f (color.cpp:5, renderbuffer.cpp:46), computed once per CTA into shared memory with
+// the same operation; a normal-map component is (b/255.f)*2.f - 1.f from it (IShader.h:97).
 struct ByteTables {
   const float* u8f;  // b / 255.f
-  const float* u8n;  // (b / 255.f) * 2.f - 1.f
 };
-__device__ __forceinline__ void build_byte_tables(float* u8f, float* u8n) {
+__device__ __forceinline__ void build_byte_tables(float* u8f) {
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    const float f = fd((float)i, 255.f);
-    u8f[i] = f;
-    u8n[i] = fs(fm(f, 2.f), 1.f);
+    u8f[i] = fd((float)i, 255.f);
   }
 }
 
@@ -106,9 +104,9 @@ __device__ __forceinline__ Col tex_diffuse(const DView& v, float u, float t, con
 __device__ __forceinline__ F3 tex_normal(const DView& v, float u, float t, const ByteTables& bt) {
   uint32_t c = tga_get(v.normal, v.nw, v.nh, cvt_i32(fm(u, (float)v.nw)), cvt_i32(fm(t, (float)v.nh)));
   F3 r;
-  r.z = bt.u8n[c & 255u];
-  r.y = bt.u8n[(c >> 8) & 255u];
-  r.x = bt.u8n[(c >> 16) & 255u];
+  r.z = fs(fm(bt.u8f[c & 255u], 2.f), 1.f);
+  r.y = fs(fm(bt.u8f[(c >> 8) & 255u], 2.f), 1.f);
+  r.x = fs(fm(bt.u8f[(c >> 16) & 255u], 2.f), 1.f);
   return r;
 }
 
@@ -139,6 +137,22 @@ __device__ __forceinline__ bool cover_terms(float ax, float ay, float e1x, float
     const float su = fa(ux, uy);
     return (uz < 0.f) ? (su >= uz && uy <= 0.f && ux <= 0.f) : (su <= uz && uy >= 0.f && ux >= 0.f);
   }
+  float b0, b1, b2;
+  cover_weights(ux, uy, uz, b0, b1, b2);
+  return !(b0 < 0.f || b1 < 0.f || b2 < 0.f);
+}
+
+// cover_terms for edges signed so that uz > 0 (the raster's compacted records); false where uz is NaN.
+__device__ __forceinline__ bool cover_terms_pos(float ax, float ay, float e1x, float e1y, float e2x, float e2y, float uz,
+                                                float pxf, float pyf, float& ux, float& uy) {
+  const float dx = fs(ax, pxf), dy = fs(ay, pyf);
+  ux = fs(fm(e1x, dy), fm(dx, e1y));
+  uy = fs(fm(dx, e2y), fm(e2x, dy));
+  // ux + uy is NaN when either is, so the minimum may drop one
+  return fa(ux, uy) <= uz && fminf(ux, uy) >= 0.f;
+}
+// The literal divisions' decision from the cross products.
+__device__ __forceinline__ bool cover_exact(float ux, float uy, float uz) {
   float b0, b1, b2;
   cover_weights(ux, uy, uz, b0, b1, b2);
   return !(b0 < 0.f || b1 < 0.f || b2 < 0.f);

@@ -105,30 +105,32 @@ __device__ __forceinline__ unsigned long long buffer_key(float d) {
   return ((unsigned long long)ord_bits(d) << 32) | 0xffffffffull;
 }
 
-// q / d for q < 1024 and 1 <= d <= 32 by multiply-shift: ceil(65536 / d).
-__constant__ uint32_t kDivMagic[33] = {0,     65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192, 7282, 6554,
-                                       5958,  5462,  5042,  4682,  4370,  4096,  3856,  3641, 3450, 3277, 3121,
-                                       2979,  2850,  2731,  2622,  2521,  2428,  2341,  2260, 2185, 2115, 2048};
-
-// The non-empty records of one batch of a tile list, compacted.  The coverage constants a
-// candidate reads are two arrays of float4 and one of uint2 (three shared loads per candidate;
-// consecutive records are consecutive 16-byte entries, so a quarter-warp's loads of different
-// records fall in different banks); the fields resolve reads are one array each.
+// The non-empty records of one batch of a tile list, compacted.  A candidate reads three 16-byte
+// entries (consecutive records are consecutive entries, so a quarter-warp's loads of different
+// records fall in different banks).
 struct __align__(16) BatchRecs {
-  float4 a4[32];       // ax, ay, e1x, e1y
-  float4 b4[32];       // e2x, e2y, uz, box (x0 | y0 << 8 | width << 16, bit 31 = kRecExact)
-  uint2 c2[32];        // first candidate of the record's run, ceil(65536 / width)
+  float4 a4[32];       // ax, ay, e1x, e1y (edges signed so that u.z > 0)
+  float4 b4[32];       // e2x, e2y, u.z of the sign test (NaN with kRecExact: never passes), u.z
+  int4 m4[32];         // candidate -> pixel: see pixel_of
   float4 d4[32];       // screen depths d0, d1, d2 of the corners, submission order (bits)
   uint32_t ri[32];     // record index (also the index of its payload)
+  uint32_t first[32];  // a bit per remainder candidate: set where a record's candidates begin
 };
 
+// Pixel of candidate i: q = i - m.x counts a record's range in row-major order, width w;
+// m.y = ceil(65536 / w) divides by w (q < 1024, w <= 32), m.z = (first pixel) - m.x, m.w = T - w.
+__device__ __forceinline__ int pixel_of(int4 m, int i) {
+  const int row = (int)(((uint32_t)(i - m.x) * (uint32_t)m.y) >> 16);
+  return i + m.z + row * m.w;
+}
+
 // Covered candidates waiting for their weights, depth and visibility update (a ring of 64 per
-// warp): the cross products (u.x, u.y) of barycentric() and the run | pixel << 8.  The
+// warp): the cross products (u.x, u.y) of barycentric() and the record | pixel << 5.  The
 // coverage pass fills it at the rate candidates are tested; the weights' three divisions and
 // the depth test then run on full warps of covered candidates.
 struct CandQueue {
   float2 u[64];
-  uint32_t jp[64];
+  uint16_t jp[64];
 };
 
 // Per-warp tile state in shared memory: per pixel the key (ordered depth | submission) and
@@ -150,7 +152,7 @@ struct RasterSmem {
   TileState<T * T> st[WARPS];
   BatchRecs br[WARPS];
   CandQueue cq[WARPS];
-  float u8f[256], u8n[256];
+  float u8f[256];
   int32_t tbase[kSharedViews];
   uint32_t claim;  // list position of the tile the CTA shares
 };
@@ -227,11 +229,11 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 // One warp per non-empty screen tile (k_scan lists them in tile order; the scatter grid has
 // cleared the others).  For each batch of 32 records of the tile list, every record's
 // bounding-box pixels inside the tile form a run of candidates; the non-empty runs are
-// compacted and laid end to end (warp prefix sum) and the lanes walk the candidates 32 at
-// a time, so the work is proportional to the pixels the triangles can touch rather than
-// to records x 32 lanes.  The run owning a candidate is found from a ballot of the runs
-// starting in the current window of 32 candidates.  A covered candidate resolves
-// visibility with a 64-bit atomicMin on
+// compacted, and the lanes walk the candidates 32 at a time, so the work is proportional to the
+// pixels the triangles can touch rather than to records x 32 lanes: first the whole windows of
+// 32 of each record, then the remainders laid end to end (warp prefix sum), where the record
+// owning a candidate is found from a bit set at each record's first one.  A covered candidate
+// resolves visibility with a 64-bit atomicMin on
 //     (ordered depth << 32) | (0xfffffffe - seq)
 // in shared memory: smallest depth first, and among equal depths the later submission.
 // The lane whose key is still the minimum after the warp's atomics records the winner's
@@ -251,7 +253,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   constexpr int NPIX = T * T;
   constexpr int PPL = NPIX / 32;
   constexpr bool kKeep = TileState<NPIX>::kKeep;
-  const ByteTables bt{sm.u8f, sm.u8n};
+  const ByteTables bt{sm.u8f};
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   TileState<NPIX>& st = sm.st[warp];
   BatchRecs& br = sm.br[warp];
@@ -269,6 +271,8 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   // critical path (the list is in tile order and dependencies only point to lower tile
   // indices, so holding later tiles never blocks).
   const uint32_t ntiles = (uint32_t)sc.ntiles;
+  const uint32_t lane_magic = (65536u + (uint32_t)lane) / ((uint32_t)lane + 1u);  // ceil(65536 / (lane + 1))
+  const uint32_t upto = (2u << lane) - 1u;  // this lane and those below
   uint32_t li = 0, li_ahead = 0;  // positions in the list
   if (SHARED) {
     if (threadIdx.x == 0) sm.claim = atomicAdd(&sc.ctl->tile_next, 1u);
@@ -322,10 +326,11 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         st.rec[lane + 32 * q] = kNone;
       }
     }
-    uint32_t frags = 0;  // covered candidates of this lane
+    uint32_t frags = 0;  // covered candidates (warp-uniform)
     for (; b < end; b += 32) {
       const uint32_t cnt = min(32u, end - b);
-      uint32_t c = 0, box = 0, ri = kNone;
+      uint32_t c = 0, w = 1, ri = kNone;
+      int p0 = 0;  // the first pixel of the record's range in the tile
       RasterRec rr;
       if ((uint32_t)lane < cnt) {
         ri = sc.bins[off + b + (uint32_t)lane];
@@ -334,29 +339,51 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
           const int lx0 = max((int)(rr.xr & 0xffffu) - ox, 0), lx1 = min((int)(rr.xr >> 16) - ox, T - 1);
           const int ly0 = max((int)(rr.yr & 0xffffu) - oy, 0), ly1 = min((int)(rr.yr >> 16) - oy, T - 1);
           if (lx0 <= lx1 && ly0 <= ly1) {
-            c = (uint32_t)((lx1 - lx0 + 1) * (ly1 - ly0 + 1));
-            box = (uint32_t)lx0 | ((uint32_t)ly0 << 8) | ((uint32_t)(lx1 - lx0 + 1) << 16);
+            w = (uint32_t)(lx1 - lx0 + 1);
+            c = w * (uint32_t)(ly1 - ly0 + 1);
+            p0 = ly0 * T + lx0;
           }
         }
       }
-      uint32_t incl = c;
+      // whole windows of 32 candidates of one record are walked record by record; the
+      // remainders (at most 31 a record) are laid end to end and share windows.  The pass is
+      // issue-bound (73 % issue active, 87 of about 130 warp instructions a window went into
+      // finding each candidate's owner, its pixel and the sign tests), so this counts slots:
+      // raster of the 4M-triangle soup at tile 16 1,024 -> 817 us, the 1080p frame at tile 8
+      // 253 -> 219 us, 64 served requests 1,835 -> 1,744 us.
+      const uint32_t whole = c & ~31u, rest = c & 31u;
+      uint32_t incl = rest;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(kFull, incl, o);
         if (lane >= o) incl += y;
       }
-      const uint32_t W = __shfl_sync(kFull, incl, 31);
-      const uint32_t start = incl - c;
-      const unsigned ne = __ballot_sync(kFull, c > 0u);
+      const int W = (int)__shfl_sync(kFull, incl, 31);
+      const uint32_t start = incl - rest;
+      const unsigned ne = __ballot_sync(kFull, rest > 0u);
+      unsigned big = __ballot_sync(kFull, whole > 0u);
+      const unsigned exact = __ballot_sync(kFull, c > 0u && ((rr.view >> kRecFlagShift) & kRecExact) != 0u);
+      const int magic = (int)__shfl_sync(kFull, lane_magic, (int)w - 1);
+      // records with a remainder come first, in order; those without fill the entries behind them
+      const int k = rest > 0u ? __popc(ne & (upto >> 1)) : __popc(ne) + __popc((big & ~ne) & (upto >> 1));
+      br.first[lane] = 0u;
       __syncwarp();
-      if (c > 0u) {  // compact the non-empty runs
-        const int k = __popc(ne & ((1u << lane) - 1u));
-        const uint32_t bits = box | (((rr.view >> kRecFlagShift) & kRecExact) ? 0x80000000u : 0u);
-        br.a4[k] = make_float4(rr.ax, rr.ay, rr.e1x, rr.e1y);
-        br.b4[k] = make_float4(rr.e2x, rr.e2y, rr.uz, __uint_as_float(bits));
-        br.c2[k] = make_uint2(start, kDivMagic[box >> 16]);
+      if (c > 0u) {
+        // u.z made positive: the edges negated turn every cross product and u.z into their exact
+        // negatives, so the decisions and the quotients stay the same (a zero weight may change
+        // its sign, which no depth, colour or comparison shows: each is a sum with a nonzero
+        // term or one that starts from +0)
+        const uint32_t sg = __float_as_uint(rr.uz) & 0x80000000u;
+        auto flip = [sg](float f) { return __uint_as_float(__float_as_uint(f) ^ sg); };
+        const float uz = fabsf(rr.uz);
+        br.a4[k] = make_float4(rr.ax, rr.ay, flip(rr.e1x), flip(rr.e1y));
+        br.b4[k] = make_float4(flip(rr.e2x), flip(rr.e2y),
+                               ((rr.view >> kRecFlagShift) & kRecExact) ? __int_as_float(0x7fffffff) : uz, uz);
+        const int base = (int)start - (int)whole;  // candidate number of the record's first pixel
+        br.m4[k] = make_int4(base, magic, p0 - base, T - (int)w);
         br.d4[k] = make_float4(rr.d0, rr.d1, rr.d2, __uint_as_float(rr.seq));
         br.ri[k] = ri;
+        if (rest > 0u) atomicOr(&br.first[start >> 5], 1u << (start & 31u));
       }
       __syncwarp();
       // Visibility of `cnt` queued candidates from the ring head, one per lane: weights
@@ -372,10 +399,10 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
           const uint32_t e = (qh + (uint32_t)lane) & 63u;
           const uint32_t jp = cq.jp[e];
           j = (int)(jp & 31u);
-          p = (int)(jp >> 8);
+          p = (int)(jp >> 5);
           const float2 u = cq.u[e];
           const float4 d4 = br.d4[j];
-          cover_weights(u.x, u.y, br.b4[j].z, b0, b1, b2);
+          cover_weights(u.x, u.y, br.b4[j].w, b0, b1, b2);
           // interpolate_depth (graphics.cpp:186-194)
           const float z = fa(fa(fa(0.f, fm(d4.z, b2)), fm(d4.y, b1)), fm(d4.x, b0));
           key = ((unsigned long long)ord_bits(z) << 32) | (unsigned long long)(0xfffffffeu - __float_as_uint(d4.w));
@@ -396,39 +423,39 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         qn -= cnt;
         __syncwarp();
       };
-      for (uint32_t base = 0; base < W; base += 32) {
-        // runs starting before this window, and a bit per run starting inside it
-        const uint32_t before = (uint32_t)__popc(__ballot_sync(kFull, c > 0u && start < base));
-        const uint32_t here = __reduce_or_sync(
-            kFull, (c > 0u && start >= base && start - base < 32u) ? 1u << (start - base) : 0u);
-        const uint32_t i = base + (uint32_t)lane;
-        bool covered = false;
-        float ux = 0.f, uy = 0.f;
-        int p = 0, j = 0;
-        if (i < W) {
-          // owner: the last run starting at or before candidate i
-          j = (int)(before + (uint32_t)__popc(here & ((2u << lane) - 1u))) - 1;
-          const float4 a4 = br.a4[j], b4 = br.b4[j];
-          const uint2 c2 = br.c2[j];
-          const uint32_t q = i - c2.x;
-          const uint32_t bx = __float_as_uint(b4.w);
-          const uint32_t lw = (bx >> 16) & 255u;
-          const uint32_t qy = (q * c2.y) >> 16;
-          const int lx = (int)(bx & 255u) + (int)(q - qy * lw);
-          const int ly = (int)((bx >> 8) & 255u) + (int)qy;
-          p = ly * T + lx;
-          covered = cover_terms(a4.x, a4.y, a4.z, a4.w, b4.x, b4.y, b4.z, (bx >> 31) != 0u, (float)(ox + lx),
-                                (float)(oy + ly), ux, uy);
-        }
+      // One window: candidate i of record j, counted when `in`.
+      auto window = [&](int i, int j, bool in) {
+        const float4 a4 = br.a4[j], b4 = br.b4[j];
+        const int p = pixel_of(br.m4[j], i);
+        const float x = (float)(ox | (p & (T - 1))), y = (float)(oy + p / T);
+        float ux, uy;
+        bool covered = cover_terms_pos(a4.x, a4.y, a4.z, a4.w, b4.x, b4.y, b4.z, x, y, ux, uy) && in;
+        if (exact && in && b4.z != b4.z) covered = cover_exact(ux, uy, b4.w);
         const unsigned cm = __ballot_sync(kFull, covered);
         if (covered) {  // queue behind the pending ones (at most 31 are pending here)
-          frags++;
-          const uint32_t e = (qh + qn + (uint32_t)__popc(cm & ((1u << lane) - 1u))) & 63u;
+          const uint32_t e = (qh + qn + (uint32_t)__popc(cm & (upto >> 1))) & 63u;
           cq.u[e] = make_float2(ux, uy);
-          cq.jp[e] = (uint32_t)j | ((uint32_t)p << 8);
+          cq.jp[e] = (uint16_t)(j | (p << 5));
         }
         qn += (uint32_t)__popc(cm);
+        frags += (uint32_t)__popc(cm);
         if (qn >= 32u) resolve(32u);
+      };
+      // whole windows: every lane works on the same record
+      while (big) {
+        const int src = __ffs(big) - 1;
+        big &= big - 1u;
+        const int j = __shfl_sync(kFull, k, src);
+        const int first = __shfl_sync(kFull, (int)start - (int)whole, src);
+        const int n32 = __shfl_sync(kFull, (int)whole, src);
+        for (int q = 0; q < n32; q += 32) window(first + q + lane, j, true);
+      }
+      // remainders: the owner of a candidate is the last record beginning at or before it
+      int before = -1;
+      for (int base = 0; base < W; base += 32) {
+        const uint32_t here = br.first[base >> 5];
+        window(base + lane, before + __popc(here & upto), base + lane < W);
+        before += __popc(here);
       }
       if (qn) resolve(qn);  // before the next batch replaces the runs the queue points to
     }
@@ -489,7 +516,6 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     }
 #undef HSR_SHADE
     shaded = __reduce_add_sync(kFull, shaded);
-    frags = __reduce_add_sync(kFull, frags);
     if (lane == 0) {
       if (shaded) atomicAdd(&sc.ctl->shaded_px, (unsigned long long)shaded);
       if (frags) atomicAdd(&sc.ctl->frag_px, (unsigned long long)frags);
@@ -541,7 +567,7 @@ template <int T, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_raster(const DView* __restrict__ views, Scratch sc) {
   extern __shared__ __align__(16) unsigned char raster_smem[];
   RasterSmem<T, WARPS>& sm = *reinterpret_cast<RasterSmem<T, WARPS>*>(raster_smem);
-  build_byte_tables(sm.u8f, sm.u8n);
+  build_byte_tables(sm.u8f);
   const int32_t* tbase = sc.nviews <= kSharedViews ? sm.tbase : nullptr;
   if (tbase)
     for (int i = threadIdx.x; i < sc.nviews; i += blockDim.x) sm.tbase[i] = views[i].tile_base;

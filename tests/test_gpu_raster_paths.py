@@ -86,3 +86,39 @@ def test_draws_into_one_target_follow_each_other(tuned, size, tile, ctas):
         oracle.draw(fr.mesh, scenes.BLINN, sd, rb, fr.diffuse, shadow_map=rs, prim_base=1000 * k)
     _check(got_s, rs, "shadow map")
     _check(got, rb, "main")
+
+
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("edge", [1, 5, 6, 9, 17, 40])
+def test_ranges_of_every_width_and_exact_records_vs_oracle(tuned, edge, tile):
+    """Triangles whose pixel ranges hold less than a window of 32 candidates, exactly whole ones, or
+    whole ones and a remainder, every second one with a corner within 2^-8 of a pixel from the
+    left or bottom border (those records take the literal divisions)."""
+    tuned.set_tuning(tile=tile, warps_per_cta=4, ctas_per_sm=8)
+    w, h, n = 70, 52, 400
+    rng = np.random.default_rng(edge * 100 + tile)
+    p = np.empty((n, 3, 2))
+    p[:, 0] = rng.uniform(0, (w, h), (n, 2))
+    p[:, 1] = p[:, 0] + rng.uniform(0.3, edge, (n, 2)) * (1, -1)
+    p[:, 2] = p[:, 0] + rng.uniform(0.3, edge, (n, 2))
+    p = np.clip(p, 0, (w - 1e-3, h - 1e-3))
+    p[::4, 0, 0] = rng.uniform(1e-5, 3e-3, len(p[::4]))
+    p[2::4, 1, 1] = rng.uniform(1e-5, 3e-3, len(p[2::4]))
+    pos = np.zeros((n, 3, 3), np.float32)
+    pos[:, :, 0] = p[:, :, 0] / w * 2 - 1
+    pos[:, :, 1] = p[:, :, 1] / h * 2 - 1
+    pos[:, :, 2] = rng.integers(0, 40, (n, 1)) / 50  # many equal depths
+    tri = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    faces = np.zeros((n, 3, 3), np.int32)
+    faces[:, :, 0] = tri
+    mesh = scenes.Mesh(pos.reshape(-1, 3), np.array([[0, 0, 1]], np.float32), np.zeros((1, 2), np.float32), faces)
+    fr = scenes.Frame(mesh, scenes.FLAT, U.shader_data((0, 0, 1), w, h, identity_mvp=True), w, h, name=f"ranges{edge}")
+    g = hframe.GpuFrame(fr)
+    try:
+        g.render()
+        got = g.download()
+    finally:
+        g.release()
+    rb = oracle.render_frame(fr)["main"]
+    assert (rb.prim > 0).any()
+    _check(got["main"], rb, f"{fr.name} tile{tile}")
