@@ -87,6 +87,7 @@ static_assert(sizeof(RasterRec) == 64, "RasterRec must stay 64 bytes");
 // setup stages and by the shading of tiles that hold fragments.
 struct __align__(128) DView {
   // target and tiles (read per raster tile)
+  // (depth and prim may be null: planes nobody reads; depth only with the fused clear)
   uint32_t* color; float* depth; uint32_t* prim; int32_t W, H;
   int32_t tile_base, tiles_x, tiles_y, ntiles;
   int32_t shader;
@@ -149,7 +150,7 @@ static_assert(offsetof(DView, prim_base) + sizeof(uint32_t) <= 128, "per-tile fi
 struct Ctl {
   uint32_t rec_count;
   uint32_t clip_count;
-  uint32_t tile_next;
+  uint32_t tile_next;      // the one tile counter of a sequence drawn by one raster launch
   uint32_t scan_ticket;
   uint32_t error;
   uint32_t bin_total;
@@ -181,7 +182,7 @@ constexpr int kSharedViews = 256;  // views whose chunk / tile bases kernels cop
 // Scratch of one launch sequence (device pointers, sized by the host).
 struct Scratch {
   Ctl* ctl;
-  uint32_t* view_done;      // [nviews] tiles finished per view
+  uint32_t* view_done;      // [nviews] tiles finished per view, then [kRasterGroups] tile counters
   RasterRec* recs;  uint32_t rec_cap;
   Payload* pay;             // [rec_cap]
   int2* clipq;      uint32_t clip_cap;   // (view, face) of faces that need clipping
@@ -195,6 +196,9 @@ struct Scratch {
   uint32_t* bins;   uint32_t bin_cap;
   int32_t ntiles;
   int32_t nviews;
+  // the raster launch's part of the tiles, [tile_lo, tile_hi), and the counter that hands out its tiles
+  int32_t tile_lo, tile_hi;
+  uint32_t* claim;
   float* stash;             // [stash_warps][stash_floats(tile)] per raster warp (may be null)
   uint32_t stash_warps;
   uint32_t faults;          // HSR_FAULT_* injected by the host (tests of the failure paths)
@@ -204,6 +208,7 @@ struct Scratch {
 // 16-byte entry — what shading would otherwise re-derive from the record.  (The winner's record
 // index, which is also its payload index, and its submission word are in the tile's shared state.)
 __host__ __device__ constexpr int stash_floats(int tile) { return 4 * tile * tile; }
+constexpr int kRasterGroups = 4;  // raster launches of one sequence at most
 constexpr int kStashWarpsPerSm = 32;  // raster warps resident per SM at most
 
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.

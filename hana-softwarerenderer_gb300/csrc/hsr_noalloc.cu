@@ -165,6 +165,8 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   sc.bins = (uint32_t*)(dev + o_bins); sc.bin_cap = (uint32_t)bin_cap;
   sc.ntiles = (int32_t)tiles;
   sc.nviews = 1;
+  sc.tile_hi = sc.ntiles;
+  sc.claim = &sc.ctl->tile_next;
 
   // ---- the launch sequence of hsr_draw on the static scratch ------------------------------
   cudaStream_t s = rt->stream;

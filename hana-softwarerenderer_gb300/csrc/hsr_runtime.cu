@@ -135,7 +135,7 @@ int Runtime::validate(const hsr_draw_desc& d) {
 // Order the draws: a consumer of a shadow map waits for the draw that renders it; draws into
 // one target keep their array order.  Returns levels via topological order.
 int Runtime::plan_order(const hsr_draw_desc* d, int n, std::vector<int>& order, std::vector<int>& dep0,
-                        std::vector<int>& dep1) {
+                        std::vector<int>& dep1, bool in_order) {
   dep0.assign(n, -1);
   dep1.assign(n, -1);
   for (int i = 0; i < n; i++) {
@@ -161,17 +161,18 @@ int Runtime::plan_order(const hsr_draw_desc* d, int n, std::vector<int>& order, 
   }
   order.resize(n);
   for (int i = 0; i < n; i++) order[i] = i;
+  if (in_order) return HSR_OK;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return level[a] < level[b]; });
   return HSR_OK;
 }
 
-int Runtime::plan_build(const hsr_draw_desc* descs, int n, Plan& p) {
+int Runtime::plan_build(const hsr_draw_desc* descs, int n, Plan& p, bool in_order) {
   for (int i = 0; i < n; i++) {
     int rc = validate(descs[i]);
     if (rc != HSR_OK) return rc;
   }
   std::vector<int> order, dep0, dep1;
-  int rc = plan_order(descs, n, order, dep0, dep1);
+  int rc = plan_order(descs, n, order, dep0, dep1, in_order);
   if (rc != HSR_OK) return rc;
   std::vector<int> pos(n);
   for (int k = 0; k < n; k++) pos[order[k]] = k;
@@ -271,7 +272,7 @@ void Plan::layout() {
   o_vout = off; off = align_up(off + view_bytes, 256);
   o_zero = off;
   o_ctl = off; off = align_up(off + sizeof(Ctl), 256);
-  o_done = off; off = align_up(off + sizeof(uint32_t) * n, 256);
+  o_done = off; off = align_up(off + sizeof(uint32_t) * ((size_t)n + kRasterGroups), 256);
   o_cnt = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_fill = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_stat = off; off = align_up(off + sizeof(unsigned long long) * std::max(nscan, 1), 256);
@@ -312,6 +313,9 @@ void Plan::bind(char* dev_base, char* host_base) {
   sc.bins = (uint32_t*)(dev + o_bins); sc.bin_cap = (uint32_t)bin_cap;
   sc.ntiles = (int32_t)total_tiles;
   sc.nviews = n;
+  sc.tile_lo = 0;
+  sc.tile_hi = sc.ntiles;
+  sc.claim = &sc.ctl->tile_next;
   sc.stash = stash_warps ? (float*)(dev + o_stash) : nullptr;
   sc.stash_warps = stash_warps;
 }
@@ -321,7 +325,8 @@ void Plan::bind(char* dev_base, char* host_base) {
 // `ev` (may be null) holds Runtime::kEvents events: [0] before the upload and [kEvents-1]
 // after the raster are recorded whenever `ev` is given; [1] after the memset and [2+k]
 // after kernel k only where non-null (profiling).
-int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t* ev) {
+// With `split`, the raster runs group by group and records each group's event.
+int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t* ev, const RasterSplit* split) {
   const DView* dviews = (const DView*)(dev + o_views);
   auto mark = [&](int k) {
     if (ev && ev[k]) cudaEventRecord(ev[k], s);
@@ -357,8 +362,17 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
   kr = launch_scatter(dviews, tile, sc, (int)std::max<size_t>(want, 1), ncch, s);
   if (kr) return cuda_fail((cudaError_t)kr, "scatter kernel");
   mark(8);
-  kr = launch_raster(dviews, tile, sc, num_sms * tu.ctas_per_sm, tu.warps_per_cta, s);
-  if (kr) return cuda_fail((cudaError_t)kr, "raster kernel");
+  for (int g = 0, ng = split ? split->n : 1; g < ng; g++) {
+    Scratch part = sc;
+    if (split) {
+      part.tile_lo = g > 0 ? views[split->end[g - 1]].tile_base : 0;
+      part.tile_hi = split->end[g] < n ? views[split->end[g]].tile_base : sc.ntiles;
+      part.claim = sc.view_done + n + g;
+    }
+    kr = launch_raster(dviews, tile, part, num_sms * tu.ctas_per_sm, tu.warps_per_cta, s);
+    if (kr) return cuda_fail((cudaError_t)kr, "raster kernel");
+    if (split && (e = cudaEventRecord(split->done[g], s)) != cudaSuccess) return cuda_fail(e, "raster group event");
+  }
   mark(9);
   e = cudaMemcpyAsync(host + host_bytes, sc.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return cuda_fail(e, "read control block");

@@ -54,6 +54,15 @@ struct Pinned {  // grow-only pinned host staging
   int reserve(size_t bytes);
 };
 
+// A sequence rasterised in groups of consecutive views, each by a launch of its own with an event
+// after it, so that work on another stream (a server's copies) can follow the group instead of
+// the sequence.  end[g]: the plan position after the group's last view; end[n - 1] = all views.
+struct RasterSplit {
+  int n = 0;
+  int end[kRasterGroups] = {};
+  cudaEvent_t done[kRasterGroups] = {};
+};
+
 // One launch sequence: view descriptors, work chunks, scratch layout and capacities.
 struct Plan {
   struct Off { size_t clip; };
@@ -75,7 +84,7 @@ struct Plan {
 
   void layout();
   void bind(char* dev_base, char* host_base);
-  int enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t* ev);
+  int enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t* ev, const RasterSplit* split = nullptr);
   int kernel_count() const;
   bool grow(const Ctl& c);
 };
@@ -110,8 +119,9 @@ struct Runtime {
   TargetObj* target(uint64_t h);
   int validate(const hsr_draw_desc& d);
   int plan_order(const hsr_draw_desc* d, int n, std::vector<int>& order, std::vector<int>& dep0,
-                 std::vector<int>& dep1);
-  int plan_build(const hsr_draw_desc* descs, int n, Plan& p);
+                 std::vector<int>& dep1, bool in_order);
+  // `in_order`: the views keep the array's order (each after those it depends on)
+  int plan_build(const hsr_draw_desc* descs, int n, Plan& p, bool in_order = false);
   void record_result(const Plan& p, const Ctl& c);
   // A plan overflowed and grew: later plans start from at least its capacities (every path
   // that launches plans, so one overflow is not repeated by each later batch).

@@ -141,15 +141,21 @@ struct SrvReq {
 // this server will free up) is failed after this many attempts.
 constexpr int kMaxIdleAllocFailures = 8;
 
+// Bytes of results to copy per further raster group of a batch: 84 us at the link's 190 GB/s, against
+// 20-60 us for a group's launch and tail.  64 mixed requests (150 MB of colour read back, whole
+// call): 4,750 -> 4,440 us, together with the planes nobody asked for left out.
+constexpr size_t kGroupBytes = (size_t)16 << 20;
+
 struct Slot {
   cudaStream_t stream = nullptr;  // copies of results, after the batch's kernels
-  cudaEvent_t kdone = nullptr;    // the batch's kernels are done (on the compute stream)
+  RasterSplit split;              // the raster groups and their events (on the compute stream)
   cudaEvent_t done = nullptr;     // its results are copied (on the slot's stream)
   char* host = nullptr;           // the batch's descriptors and control block
   size_t host_cap = 0;
   Plan plan;
   std::vector<hsr_draw_desc> descs;
-  std::vector<SrvReq*> reqs;
+  std::vector<SrvReq*> reqs;      // in the order of their main views: group g's are [.., group_end[g])
+  int group_end[kRasterGroups] = {};
   bool busy = false;
   uint32_t batch = 0;
 };
@@ -184,6 +190,11 @@ static uint64_t g_next_obj = 1;
 
 // A target is three 256-byte aligned planes (colour, depth, prim ids) in one block.
 static size_t plane_bytes(int w, int h) { return ((size_t)w * (size_t)h * 4 + 255) / 256 * 256; }
+
+// The caller's plane k of a request (0 colour, 1 depth, 2 prim ids; null: not asked for).
+static void* out_plane(const hsr_request& r, int k) {
+  return k == 0 ? static_cast<void*>(r.out_rgba) : k == 1 ? static_cast<void*>(r.out_depth) : static_cast<void*>(r.out_prim);
+}
 
 static size_t req_bytes(const hsr_request& r) {
   return 3 * plane_bytes(r.width, r.height) + (r.shadow_size > 0 ? 3 * plane_bytes(r.shadow_size, r.shadow_size) : 0);
@@ -229,32 +240,35 @@ static int slot_enqueue(ServerObj* so, Slot& s) {
   int rc = slot_reserve(so, s, s.plan);
   if (rc != HSR_OK) return rc;
   s.plan.bind(so->dev, s.host);
-  rc = s.plan.enqueue(so->compute, so->num_sms, so->tuning, nullptr);
+  rc = s.plan.enqueue(so->compute, so->num_sms, so->tuning, nullptr, &s.split);
   if (rc != HSR_OK) return rc;
-  cudaError_t e = cudaEventRecord(s.kdone, so->compute);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(s.stream, s.kdone, 0);
-  if (e != cudaSuccess) return cuda_fail(e, "server: order copies after the batch");
   {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_rt) g_rt->launches += (uint64_t)s.plan.kernel_count();
+    if (g_rt) g_rt->launches += (uint64_t)(s.plan.kernel_count() + s.split.n - 1);
   }
-  for (SrvReq* q : s.reqs) {
-    const size_t n = (size_t)q->r.width * (size_t)q->r.height, pl = plane_bytes(q->r.width, q->r.height);
-    const char* base = q->mem;
-    if (q->r.out_rgba) cudaMemcpyAsync(q->r.out_rgba, base, 4 * n, cudaMemcpyDeviceToHost, s.stream);
-    if (q->r.out_depth) cudaMemcpyAsync(q->r.out_depth, base + pl, 4 * n, cudaMemcpyDeviceToHost, s.stream);
-    if (q->r.out_prim) cudaMemcpyAsync(q->r.out_prim, base + 2 * pl, 4 * n, cudaMemcpyDeviceToHost, s.stream);
+  size_t at = 0;
+  for (int g = 0; g < s.split.n; g++) {
+    cudaError_t e = cudaStreamWaitEvent(s.stream, s.split.done[g], 0);
+    if (e != cudaSuccess) return cuda_fail(e, "server: order copies after the batch");
+    for (; at < (size_t)s.group_end[g]; at++) {
+      SrvReq* q = s.reqs[at];
+      const size_t n = (size_t)q->r.width * (size_t)q->r.height, pl = plane_bytes(q->r.width, q->r.height);
+      for (int k = 0; k < 3; k++)
+        if (out_plane(q->r, k)) cudaMemcpyAsync(out_plane(q->r, k), q->mem + k * pl, 4 * n, cudaMemcpyDeviceToHost, s.stream);
+    }
   }
-  e = cudaEventRecord(s.done, s.stream);
+  cudaError_t e = cudaEventRecord(s.done, s.stream);
   return e == cudaSuccess ? HSR_OK : cuda_fail(e, "server: event record");
 }
 
-static TargetObj* make_pooled_target(char* mem, int w, int h) {
+// A target in the pool's block `mem`.  Every draw of a server clears, and its targets are seen
+// through the planes asked for alone: the others are neither read nor written.
+static TargetObj* make_pooled_target(char* mem, int w, int h, bool depth, bool prim) {
   TargetObj* t = new TargetObj();
   const size_t pl = plane_bytes(w, h);
   t->color = reinterpret_cast<uint32_t*>(mem);
-  t->depth = reinterpret_cast<float*>(mem + pl);
-  t->prim = reinterpret_cast<uint32_t*>(mem + 2 * pl);
+  t->depth = depth ? reinterpret_cast<float*>(mem + pl) : nullptr;
+  t->prim = prim ? reinterpret_cast<uint32_t*>(mem + 2 * pl) : nullptr;
   t->w = w;
   t->h = h;
   t->pooled = true;
@@ -288,6 +302,42 @@ static void finish(ServerObj* so, Slot& s, int status) {
   s.reqs.clear();
   s.busy = false;
   so->cv_done.notify_all();
+}
+
+// The order of a batch's main views and its raster groups.  A group's results are copied while the
+// later groups are drawn, so only the last group's copies are left when the kernels end; each
+// group costs a raster launch and its tail.  Requests without a shadow pass come first (their
+// copies run under the shadow passes), larger ones before smaller ones (so that the last group's
+// copies are short); group g also draws the shadow maps that group g + 1's main views read
+// (shadow_group[i]: the group of request i's main view), group 0 its own before them.
+static void group_requests(Slot& s, const std::vector<SrvReq*>& batch, std::vector<int>& shadow_group) {
+  auto copied = [](const SrvReq* q) {
+    size_t planes = 0;
+    for (int k = 0; k < 3; k++) planes += out_plane(q->r, k) != nullptr;
+    return planes * 4 * (size_t)q->r.width * (size_t)q->r.height;
+  };
+  s.reqs = batch;
+  std::stable_sort(s.reqs.begin(), s.reqs.end(), [&](const SrvReq* a, const SrvReq* b) {
+    const bool sa = a->r.shadow_size > 0, sb = b->r.shadow_size > 0;
+    return sa != sb ? sb : copied(a) > copied(b);
+  });
+  size_t total = 0;
+  for (const SrvReq* q : s.reqs) total += copied(q);
+  const int ng = (int)std::min<size_t>({(size_t)kRasterGroups, 1 + total / kGroupBytes, s.reqs.size()});
+  // the groups' shares of the bytes, summed: decreasing, as what the last one leaves to copy shows
+  static const double kShare[kRasterGroups][kRasterGroups] = {
+      {1.0}, {0.7, 1.0}, {0.5, 0.85, 1.0}, {0.4, 0.7, 0.9, 1.0}};
+  s.split.n = ng;
+  shadow_group.assign(s.reqs.size(), -1);
+  size_t at = 0, bytes = 0;
+  for (int g = 0; g < ng; g++) {
+    const size_t left = (size_t)(ng - 1 - g);  // every group has a request
+    do {
+      if (s.reqs[at]->r.shadow_size > 0) shadow_group[at] = g;
+      bytes += copied(s.reqs[at++]);
+    } while (at + left < s.reqs.size() && (g == ng - 1 || (double)bytes < kShare[ng - 1][g] * (double)total));
+    s.group_end[g] = (int)at;
+  }
 }
 
 // Form and launch one batch on a free slot; returns true if something was launched.
@@ -353,7 +403,8 @@ static bool try_launch(ServerObj* so, Slot& s) {
       return false;  // retried when a batch completes or after the scheduler's poll interval
     }
   }
-  s.reqs = batch;
+  std::vector<int> shadow_group;
+  group_requests(s, batch, shadow_group);
   s.batch = so->next_batch++;
   const double t = so->now();
   s.descs.clear();
@@ -361,47 +412,54 @@ static bool try_launch(ServerObj* so, Slot& s) {
   {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_rt) rc = HSR_ERR_NOT_INITIALIZED;
-    for (SrvReq* q : batch) {
-      if (rc != HSR_OK) break;
-      if (!q->mem) { rc = HSR_ERR_OUT_OF_MEMORY; break; }
-      const size_t main_bytes = 3 * plane_bytes(q->r.width, q->r.height);
-      TargetObj* tm = make_pooled_target(q->mem, q->r.width, q->r.height);
-      q->h_main = g_rt->next_handle++;
-      g_rt->targets[q->h_main] = tm;
-      hsr_target shadow = 0;
-      if (q->r.shadow_size > 0) {
-        TargetObj* ts = make_pooled_target(q->mem + main_bytes, q->r.shadow_size, q->r.shadow_size);
-        q->h_shadow = g_rt->next_handle++;
-        g_rt->targets[q->h_shadow] = ts;
-        shadow = q->h_shadow;
-        hsr_draw_desc d;
-        std::memset(&d, 0, sizeof(d));
-        d.mesh = q->r.mesh;
+    auto make_target = [&](uint64_t& h, char* mem, int w, int ht, bool depth, bool prim) {
+      h = g_rt->next_handle++;
+      g_rt->targets[h] = make_pooled_target(mem, w, ht, depth, prim);
+    };
+    auto draw_of = [](const SrvReq* q) {
+      hsr_draw_desc d;
+      std::memset(&d, 0, sizeof(d));
+      d.mesh = q->r.mesh;
+      d.flags = HSR_DRAW_CLEAR;
+      d.diffuse = q->r.diffuse;
+      d.normal = q->r.normal;
+      d.uniforms = &q->r.uniforms;
+      return d;
+    };
+    auto shadows_of_group = [&](int g) {
+      for (size_t i = 0; i < s.reqs.size(); i++) {
+        SrvReq* q = s.reqs[i];
+        if (shadow_group[i] != g) continue;
+        // a shadow map is read through its colour plane alone (is_in_shadow)
+        make_target(q->h_shadow, q->mem + 3 * plane_bytes(q->r.width, q->r.height), q->r.shadow_size, q->r.shadow_size,
+                    false, false);
+        hsr_draw_desc d = draw_of(q);
         d.shader = HSR_SHADER_SHADOW;
-        d.flags = HSR_DRAW_CLEAR;
-        d.diffuse = q->r.diffuse;
-        d.normal = q->r.normal;
-        d.target = shadow;
-        d.uniforms = &q->r.uniforms;
+        d.target = q->h_shadow;
         d.clear_depth = q->r.shadow_clear_depth;
         std::memcpy(d.clear_rgba, q->r.shadow_clear_rgba, 4);
         s.descs.push_back(d);
       }
-      hsr_draw_desc d;
-      std::memset(&d, 0, sizeof(d));
-      d.mesh = q->r.mesh;
-      d.shader = q->r.shader;
-      d.flags = HSR_DRAW_CLEAR;
-      d.diffuse = q->r.diffuse;
-      d.normal = q->r.normal;
-      d.target = q->h_main;
-      d.shadow_map = shadow;
-      d.uniforms = &q->r.uniforms;
-      d.clear_depth = q->r.clear_depth;
-      std::memcpy(d.clear_rgba, q->r.clear_rgba, 4);
-      s.descs.push_back(d);
-    }
-    if (rc == HSR_OK) rc = g_rt->plan_build(s.descs.data(), (int)s.descs.size(), s.plan);
+    };
+    size_t at = 0;
+    if (rc == HSR_OK)
+      for (int g = 0; g < s.split.n; g++) {
+        if (g == 0) shadows_of_group(0);
+        for (; at < (size_t)s.group_end[g]; at++) {
+          SrvReq* q = s.reqs[at];
+          make_target(q->h_main, q->mem, q->r.width, q->r.height, q->r.out_depth != nullptr, q->r.out_prim != nullptr);
+          hsr_draw_desc d = draw_of(q);
+          d.shader = q->r.shader;
+          d.target = q->h_main;
+          d.shadow_map = q->h_shadow;
+          d.clear_depth = q->r.clear_depth;
+          std::memcpy(d.clear_rgba, q->r.clear_rgba, 4);
+          s.descs.push_back(d);
+        }
+        shadows_of_group(g + 1);
+        s.split.end[g] = (int)s.descs.size();
+      }
+    if (rc == HSR_OK) rc = g_rt->plan_build(s.descs.data(), (int)s.descs.size(), s.plan, true);
   }
   for (SrvReq* q : batch) {
     q->st.launch_ms = t;
@@ -558,13 +616,16 @@ int hsr_server_create(const hsr_server_config* cfg, hsr_server* out) {
     bool ok = cudaStreamCreateWithFlags(&so->compute, cudaStreamNonBlocking) == cudaSuccess;
     for (Slot& s : so->slots)
       ok = ok && cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) == cudaSuccess &&
-           cudaEventCreateWithFlags(&s.kdone, cudaEventDisableTiming) == cudaSuccess &&
+           std::all_of(std::begin(s.split.done), std::end(s.split.done), [](cudaEvent_t& e) {
+             return cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+           }) &&
            cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
       cudaGetLastError();
       for (Slot& s : so->slots) {
         if (s.done) cudaEventDestroy(s.done);
-        if (s.kdone) cudaEventDestroy(s.kdone);
+        for (cudaEvent_t e : s.split.done)
+          if (e) cudaEventDestroy(e);
         if (s.stream) cudaStreamDestroy(s.stream);
       }
       if (so->compute) cudaStreamDestroy(so->compute);
@@ -684,7 +745,7 @@ int hsr_server_destroy(hsr_server s) {
     cudaStreamSynchronize(sl.stream);
     if (sl.host) cudaFreeHost(sl.host);
     cudaEventDestroy(sl.done);
-    cudaEventDestroy(sl.kdone);
+    for (cudaEvent_t e : sl.split.done) cudaEventDestroy(e);
     cudaStreamDestroy(sl.stream);
   }
   cudaStreamSynchronize(so->compute);

@@ -262,14 +262,14 @@ __device__ __forceinline__ void clear_empty_tiles(const DView* __restrict__ view
       const int i = g0 + 128 * k;
       if (m == 15u && vec) {
         *reinterpret_cast<uint4*>(v.color + i) = make_uint4(rgba, rgba, rgba, rgba);
-        *reinterpret_cast<float4*>(v.depth + i) = make_float4(depth, depth, depth, depth);
+        if (v.depth) *reinterpret_cast<float4*>(v.depth + i) = make_float4(depth, depth, depth, depth);
         if (prim) *reinterpret_cast<uint4*>(prim + i) = make_uint4(0u, 0u, 0u, 0u);
       } else {
 #pragma unroll
         for (int d = 0; d < 4; d++) {
           if (m >> d & 1u) {
             v.color[i + d] = rgba;
-            v.depth[i + d] = depth;
+            if (v.depth) v.depth[i + d] = depth;
             if (prim) prim[i + d] = 0u;
           }
         }

@@ -215,11 +215,11 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
       const uint32_t prim = v.prim_base + (seq >> 4) + 1u;
       const uint32_t alpha = clear ? v.clear_rgba : __ldcg(&v.color[idx]);
       v.color[idx] = pack_rgb(fragment_s<S>(v, P, b0, b1, b2, prim, bt), alpha);
-      v.depth[idx] = from_ord((uint32_t)(st.key[p] >> 32));
+      if (v.depth) v.depth[idx] = from_ord((uint32_t)(st.key[p] >> 32));
       if (v.prim) v.prim[idx] = prim;
     } else if (clear) {
       v.color[idx] = v.clear_rgba;
-      v.depth[idx] = v.clear_depth;
+      if (v.depth) v.depth[idx] = v.clear_depth;
       if (v.prim) v.prim[idx] = 0u;
     }
   }
@@ -249,7 +249,8 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 // never matters), and the pixel rows are shaded by the warps in turn.
 template <int T, int WARPS, bool SHARED>
 __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, const Scratch& sc,
-                                             RasterSmem<T, WARPS>& sm, const int32_t* tbase, uint32_t nlist) {
+                                             RasterSmem<T, WARPS>& sm, const int32_t* tbase, uint32_t nlist,
+                                             const uint32_t* tile_list) {
   constexpr int NPIX = T * T;
   constexpr int PPL = NPIX / 32;
   constexpr bool kKeep = TileState<NPIX>::kKeep;
@@ -275,17 +276,17 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   const uint32_t upto = (2u << lane) - 1u;  // this lane and those below
   uint32_t li = 0, li_ahead = 0;  // positions in the list
   if (SHARED) {
-    if (threadIdx.x == 0) sm.claim = atomicAdd(&sc.ctl->tile_next, 1u);
+    if (threadIdx.x == 0) sm.claim = atomicAdd(sc.claim, 1u);
     __syncthreads();
     li = sm.claim;
   } else {
     if (lane == 0) {
-      li = atomicAdd(&sc.ctl->tile_next, 1u);
-      li_ahead = atomicAdd(&sc.ctl->tile_next, 1u);
+      li = atomicAdd(sc.claim, 1u);
+      li_ahead = atomicAdd(sc.claim, 1u);
     }
     li = __shfl_sync(kFull, li, 0);
   }
-  uint32_t t = li < nlist ? sc.tile_list[li] : ntiles;
+  uint32_t t = li < nlist ? tile_list[li] : ntiles;
   uint32_t n = 0, off = 0;
   if (t < ntiles) {
     n = sc.tile_count[t];
@@ -299,8 +300,8 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     uint32_t t_next = ntiles, n_next = 0, off_next = 0;
     if (!SHARED) {
       const uint32_t li_next = __shfl_sync(kFull, li_ahead, 0);
-      if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(&sc.ctl->tile_next, 1u) : nlist;
-      if (li_next < nlist) t_next = sc.tile_list[li_next];
+      if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(sc.claim, 1u) : nlist;
+      if (li_next < nlist) t_next = tile_list[li_next];
       if (t_next < ntiles) {
         n_next = sc.tile_count[t_next];
         off_next = sc.tile_off[t_next];
@@ -531,10 +532,10 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     }
     if (SHARED) {
       __syncthreads();  // the merged state and the claim word are free again
-      if (threadIdx.x == 0) sm.claim = atomicAdd(&sc.ctl->tile_next, 1u);
+      if (threadIdx.x == 0) sm.claim = atomicAdd(sc.claim, 1u);
       __syncthreads();
       li = sm.claim;
-      if (li < nlist) t_next = sc.tile_list[li];
+      if (li < nlist) t_next = tile_list[li];
       if (t_next < ntiles) {
         n_next = sc.tile_count[t_next];
         off_next = sc.tile_off[t_next];
@@ -573,13 +574,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
     for (int i = threadIdx.x; i < sc.nviews; i += blockDim.x) sm.tbase[i] = views[i].tile_base;
   __syncthreads();
   if (sc.ctl->error & kErrNoDraw) return;
-  const uint32_t nlist = min(sc.ctl->ne_tiles, (uint32_t)sc.ntiles);
+  // this launch's part of the list (all of it unless the sequence is drawn in groups)
+  const uint32_t lo = sc.tile_lo > 0 ? sc.ne_off[sc.tile_lo] : 0u;
+  const uint32_t nlist = sc.ne_off[sc.tile_hi] - lo;
+  const uint32_t* list = sc.tile_list + lo;
   // uniform over the grid: every warp of every CTA has a stash, or none does
   const bool stashes = TileState<T * T>::kKeep || !sc.stash || gridDim.x * (uint32_t)WARPS <= sc.stash_warps;
   if (nlist <= kSharedTilesPerCta * gridDim.x && stashes)
-    raster_tiles<T, WARPS, true>(views, sc, sm, tbase, nlist);
+    raster_tiles<T, WARPS, true>(views, sc, sm, tbase, nlist, list);
   else
-    raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist);
+    raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist, list);
 }
 
 template <int T, int WARPS>
