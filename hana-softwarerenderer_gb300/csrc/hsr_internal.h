@@ -182,7 +182,8 @@ constexpr int kSharedViews = 256;  // views whose chunk / tile bases kernels cop
 // Scratch of one launch sequence (device pointers, sized by the host).
 struct Scratch {
   Ctl* ctl;
-  uint32_t* view_done;      // [nviews] tiles finished per view, then [kRasterGroups] tile counters
+  uint32_t* view_done;      // [nviews] tiles finished per view, then [kRasterGroups] tile counters and
+                            // the count of finished raster CTAs
   RasterRec* recs;  uint32_t rec_cap;
   Payload* pay;             // [rec_cap]
   int2* clipq;      uint32_t clip_cap;   // (view, face) of faces that need clipping
@@ -199,6 +200,10 @@ struct Scratch {
   // the raster launch's part of the tiles, [tile_lo, tile_hi), and the counter that hands out its tiles
   int32_t tile_lo, tile_hi;
   uint32_t* claim;
+  // where the raster's last CTA (counted by `finished`) stores the control block: mapped host
+  // memory, null for a launch that is not the sequence's last or whose host copies it itself
+  Ctl* ctl_out;
+  uint32_t* finished;
   float* stash;             // [stash_warps][stash_floats(tile)] per raster warp (may be null)
   uint32_t stash_warps;
   uint32_t faults;          // HSR_FAULT_* injected by the host (tests of the failure paths)
@@ -212,6 +217,8 @@ constexpr int kRasterGroups = 4;  // raster launches of one sequence at most
 constexpr int kStashWarpsPerSm = 32;  // raster warps resident per SM at most
 
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.
+// `from` is mapped host memory or device memory; sizes are multiples of 16.
+int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s);
 int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s);
 int launch_setup(const DView* views, int nviews, int nchunks, Scratch sc, int grid, cudaStream_t s);
 int launch_emit(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);

@@ -272,7 +272,7 @@ void Plan::layout() {
   o_vout = off; off = align_up(off + view_bytes, 256);
   o_zero = off;
   o_ctl = off; off = align_up(off + sizeof(Ctl), 256);
-  o_done = off; off = align_up(off + sizeof(uint32_t) * ((size_t)n + kRasterGroups), 256);
+  o_done = off; off = align_up(off + sizeof(uint32_t) * ((size_t)n + kRasterGroups + 1), 256);
   o_cnt = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_fill = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_stat = off; off = align_up(off + sizeof(unsigned long long) * std::max(nscan, 1), 256);
@@ -316,14 +316,16 @@ void Plan::bind(char* dev_base, char* host_base) {
   sc.tile_lo = 0;
   sc.tile_hi = sc.ntiles;
   sc.claim = &sc.ctl->tile_next;
+  sc.ctl_out = (Ctl*)(host + host_bytes);
+  sc.finished = sc.view_done + n + kRasterGroups;
   sc.stash = stash_warps ? (float*)(dev + o_stash) : nullptr;
   sc.stash_warps = stash_warps;
 }
 
-// Upload of the view descriptors, one memset, the kernels, read-back of the control
-// block: everything stream-ordered, nothing synchronous (capturable into a CUDA graph).
-// `ev` (may be null) holds Runtime::kEvents events: [0] before the upload and [kEvents-1]
-// after the raster are recorded whenever `ev` is given; [1] after the memset and [2+k]
+// View descriptors and counters (k_prep), then the kernels; the raster's last CTA writes the
+// control block into the staging.  Everything is stream-ordered, nothing synchronous (capturable
+// into a CUDA graph).  `ev` (may be null) holds Runtime::kEvents events: [0] before k_prep and
+// [kEvents-1] after the raster are recorded whenever `ev` is given; [1] after k_prep and [2+k]
 // after kernel k only where non-null (profiling).
 // With `split`, the raster runs group by group and records each group's event.
 int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t* ev, const RasterSplit* split) {
@@ -332,12 +334,11 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
     if (ev && ev[k]) cudaEventRecord(ev[k], s);
   };
   mark(0);
-  cudaError_t e = cudaMemcpyAsync(dev, host, host_bytes, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return cuda_fail(e, "upload views");
-  e = cudaMemsetAsync(dev + o_zero, 0, zero_bytes, s);
-  if (e != cudaSuccess) return cuda_fail(e, "clear scratch");
+  // (page-locked memory of cudaMallocHost is mapped at its own address)
+  int kr = launch_prep(host, dev, host_bytes, dev + o_zero, zero_bytes, num_sms * 4, s);
+  if (kr) return cuda_fail((cudaError_t)kr, "prep kernel");
   mark(1);
-  int kr = launch_vertex(dviews, n, nvch, num_sms * 8, s);
+  kr = launch_vertex(dviews, n, nvch, num_sms * 8, s);
   if (kr) return cuda_fail((cudaError_t)kr, "vertex kernel");
   mark(2);
   kr = launch_setup(dviews, n, nsch, sc, num_sms * 8, s);
@@ -368,19 +369,20 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
       part.tile_lo = g > 0 ? views[split->end[g - 1]].tile_base : 0;
       part.tile_hi = split->end[g] < n ? views[split->end[g]].tile_base : sc.ntiles;
       part.claim = sc.view_done + n + g;
+      if (g < ng - 1) part.ctl_out = nullptr;
     }
     kr = launch_raster(dviews, tile, part, num_sms * tu.ctas_per_sm, tu.warps_per_cta, s);
     if (kr) return cuda_fail((cudaError_t)kr, "raster kernel");
-    if (split && (e = cudaEventRecord(split->done[g], s)) != cudaSuccess) return cuda_fail(e, "raster group event");
+    if (!split) continue;
+    const cudaError_t e = cudaEventRecord(split->done[g], s);
+    if (e != cudaSuccess) return cuda_fail(e, "raster group event");
   }
   mark(9);
-  e = cudaMemcpyAsync(host + host_bytes, sc.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return cuda_fail(e, "read control block");
   return HSR_OK;
 }
 
 int Plan::kernel_count() const {
-  return (nvch ? 1 : 0) + (nsch ? 1 : 0) + 3 + (nscan > 0 ? 1 : 0) + 2;
+  return 1 + (nvch ? 1 : 0) + (nsch ? 1 : 0) + 3 + (nscan > 0 ? 1 : 0) + 2;
 }
 
 // Grow the capacity an overflow reported; returns false if nothing overflowed.

@@ -2,6 +2,8 @@
 // each triangle's bounding box (graphics.cpp:349-375).  Here the (record, tile) pairs are
 // laid out per tile so that one warp can own a tile in the raster.
 //
+// k_prep    the launch sequence's first kernel: view descriptors from the host's page-locked
+//           staging, counters to zero.
 // k_scan    exclusive prefix sums of the per-tile counts and of the non-empty tiles, single
 //           pass with decoupled look-back, and the list of non-empty tiles in tile order;
 //           block order comes from a ticket so a block only waits on blocks that already
@@ -9,7 +11,10 @@
 // k_scatter writes record indices into the per-tile lists with warp-aggregated atomics;
 //           a record touches at most kMaxRecordTiles tiles (k_big splits larger ones).
 //           The same grid clears the tiles no record touches, streamed in row order.
+#include <algorithm>
+
 #include "hsr_device.cuh"
+#include "hsr_launch.cuh"
 
 namespace hsr {
 
@@ -40,11 +45,29 @@ __device__ __forceinline__ unsigned long long scan_item(uint32_t count) {
   return (unsigned long long)count + (count ? kOneTile : 0ull);
 }
 
+// First kernel of a sequence: copies `copy` bytes of view descriptors from mapped host memory and
+// clears `zero` bytes of counters (both multiples of 16).  One launch in place of a copy
+// and a memset, which the kernels behind it could not overlap.
+__global__ void __launch_bounds__(256) k_prep(const uint4* __restrict__ from, uint4* __restrict__ to, size_t copy,
+                                              uint4* __restrict__ counters, size_t zero) {
+  const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = i0; i < copy / 16; i += step) to[i] = __ldcv(from + i);
+  for (size_t i = i0; i < zero / 16; i += step) counters[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s) {
+  const size_t want = (std::max(copy, zero) / 16 + 255) / 256;
+  const int grid = (int)std::min<size_t>(std::max<size_t>(want, 1), (size_t)max_grid);
+  k_prep<<<grid, 256, 0, s>>>(static_cast<const uint4*>(from), static_cast<uint4*>(to), copy, static_cast<uint4*>(counters), zero);
+  return (int)cudaGetLastError();
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_scan(Scratch sc) {
   __shared__ unsigned long long warp_sums[kScanThreads / 32];
   __shared__ unsigned long long s_prefix;
   __shared__ uint32_t s_block;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  chain_wait();
   if (threadIdx.x == 0) s_block = atomicAdd(&sc.ctl->scan_ticket, 1u);
   __syncthreads();
   const uint32_t blk = s_block;
@@ -144,8 +167,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Scratch sc) {
 int launch_scan(Scratch sc, cudaStream_t s) {
   const int nb = scan_blocks(sc.ntiles);
   if (nb <= 0) return 0;
-  k_scan<<<nb, kScanThreads, 0, s>>>(sc);
-  return (int)cudaGetLastError();
+  return launch_chained(k_scan, nb, kScanThreads, 0, s, sc);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -286,6 +308,7 @@ constexpr int kClearEvery = 2;
 __global__ void __launch_bounds__(256) k_scatter(const DView* __restrict__ views, int T, Scratch sc, int nchunks) {
   __shared__ int32_t s_cbase[kSharedViews];
   const uint32_t b = blockIdx.x, g = gridDim.x;
+  chain_wait();
   if (nchunks > 0 && b % kClearEvery == kClearEvery - 1) {  // block-uniform
     const bool in_shared = sc.nviews <= kSharedViews;
     if (in_shared)
@@ -303,8 +326,7 @@ __global__ void __launch_bounds__(256) k_scatter(const DView* __restrict__ views
 // have blocks).
 int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int nchunks, cudaStream_t s) {
   if (nchunks > 0 && grid < kClearEvery) grid = kClearEvery;
-  k_scatter<<<grid > 0 ? grid : 1, 256, 0, s>>>(views, tile, sc, nchunks);
-  return (int)cudaGetLastError();
+  return launch_chained(k_scatter, grid > 0 ? grid : 1, 256, 0, s, views, tile, sc, nchunks);
 }
 
 }  // namespace hsr

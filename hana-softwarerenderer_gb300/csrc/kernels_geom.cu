@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "hsr_device.cuh"
+#include "hsr_launch.cuh"
 
 namespace hsr {
 
@@ -204,6 +205,7 @@ __device__ __forceinline__ void vertex_chunk_work(const DView& v, const Chunk& c
 // One block per chunk (the blocks are short and many: their prologues overlap others' work).
 __global__ void __launch_bounds__(256) k_vertex(const DView* __restrict__ views, int nviews) {
   __shared__ int32_t s_base[kSharedViews];
+  chain_wait();
   const int32_t* base = share_bases(views, nviews, s_base, VchBase());
   const Chunk ch = vertex_chunk(views, base, nviews, (int)blockIdx.x);
   vertex_chunk_work(views[ch.view], ch);
@@ -212,8 +214,7 @@ __global__ void __launch_bounds__(256) k_vertex(const DView* __restrict__ views,
 int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s) {
   (void)grid;
   if (nchunks <= 0) return 0;
-  k_vertex<<<nchunks, 256, 0, s>>>(views, nviews);
-  return (int)cudaGetLastError();
+  return launch_chained(k_vertex, nchunks, 256, 0, s, views, nviews);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -489,6 +490,7 @@ __device__ __forceinline__ void cull_face(const DView& v, int f, uint32_t view, 
 __global__ void __launch_bounds__(kSetupThreads, 8) k_setup(const DView* __restrict__ views, int nviews,
                                                          int nchunks, Scratch sc) {
   __shared__ int32_t s_base[kSharedViews];
+  chain_wait();
   const int32_t* base = share_bases(views, nviews, s_base, SchBase());
   int c = (int)blockIdx.x;
   const int c_end = nchunks;
@@ -587,6 +589,7 @@ __device__ __forceinline__ void face_payload(const DView& v, int f, int nf4, int
 // the warp collectives of append_small see every lane.
 __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* __restrict__ views, int T, Scratch sc) {
   const int lane = threadIdx.x & 31;
+  chain_wait();
   if (sc.ctl->error & kErrCapacity) return;
   const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
   const uint32_t stride = gridDim.x * blockDim.x;
@@ -637,8 +640,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* __restric
 }
 
 int launch_emit(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {
-  k_emit<<<grid, kEmitThreads, 0, s>>>(views, tile, sc);
-  return (int)cudaGetLastError();
+  return launch_chained(k_emit, grid, kEmitThreads, 0, s, views, tile, sc);
 }
 
 // Homogeneous clipping (graphics.cpp:73-161), two faces per warp: each half-warp clips its own
@@ -732,6 +734,7 @@ constexpr int kPostThreads = 256;
 __global__ void __launch_bounds__(kPostThreads, 3) k_post(const DView* __restrict__ views, int T, Scratch sc) {
   __shared__ float poly[kPostThreads / 32][2][2][16 * kPolyStride];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
+  chain_wait();
   if (sc.ctl->error & kErrCapacity) return;
   const uint32_t nclip = min(sc.ctl->clip_count, sc.clip_cap);
   uint32_t item = 0, ahead = 0;
@@ -753,8 +756,7 @@ __global__ void __launch_bounds__(kPostThreads, 3) k_post(const DView* __restric
 }
 
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {
-  k_post<<<grid, kPostThreads, 0, s>>>(views, tile, sc);
-  return (int)cudaGetLastError();
+  return launch_chained(k_post, grid, kPostThreads, 0, s, views, tile, sc);
 }
 
 constexpr int kBigThreads = 512;
@@ -766,6 +768,7 @@ constexpr int kBigThreads = 512;
 // triangle's pixel range, so each pixel is still tested exactly once.
 __global__ void __launch_bounds__(kBigThreads) k_big(const DView* __restrict__ views, int T, Scratch sc) {
   __shared__ uint32_t s_base;
+  chain_wait();
   if (sc.ctl->error & kErrCapacity) return;
   const uint32_t nbig = min(sc.ctl->big_count, sc.big_cap);
   for (uint32_t item = blockIdx.x; item < nbig; item += gridDim.x) {
@@ -811,14 +814,12 @@ __global__ void __launch_bounds__(kBigThreads) k_big(const DView* __restrict__ v
 }
 
 int launch_big(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {
-  k_big<<<grid, kBigThreads, 0, s>>>(views, tile, sc);
-  return (int)cudaGetLastError();
+  return launch_chained(k_big, grid, kBigThreads, 0, s, views, tile, sc);
 }
 
 int launch_setup(const DView* views, int nviews, int nchunks, Scratch sc, int grid, cudaStream_t s) {
   if (nchunks <= 0) return 0;
-  k_setup<<<std::max(1, std::min(grid, nchunks)), kSetupThreads, 0, s>>>(views, nviews, nchunks, sc);
-  return (int)cudaGetLastError();
+  return launch_chained(k_setup, std::max(1, std::min(grid, nchunks)), kSetupThreads, 0, s, views, nviews, nchunks, sc);
 }
 
 }  // namespace hsr

@@ -23,6 +23,7 @@
 #include <float.h>
 
 #include "hsr_device.cuh"
+#include "hsr_launch.cuh"
 
 namespace hsr {
 
@@ -569,21 +570,37 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
   extern __shared__ __align__(16) unsigned char raster_smem[];
   RasterSmem<T, WARPS>& sm = *reinterpret_cast<RasterSmem<T, WARPS>*>(raster_smem);
   build_byte_tables(sm.u8f);
+  chain_wait();
   const int32_t* tbase = sc.nviews <= kSharedViews ? sm.tbase : nullptr;
   if (tbase)
     for (int i = threadIdx.x; i < sc.nviews; i += blockDim.x) sm.tbase[i] = views[i].tile_base;
   __syncthreads();
-  if (sc.ctl->error & kErrNoDraw) return;
-  // this launch's part of the list (all of it unless the sequence is drawn in groups)
-  const uint32_t lo = sc.tile_lo > 0 ? sc.ne_off[sc.tile_lo] : 0u;
-  const uint32_t nlist = sc.ne_off[sc.tile_hi] - lo;
-  const uint32_t* list = sc.tile_list + lo;
-  // uniform over the grid: every warp of every CTA has a stash, or none does
-  const bool stashes = TileState<T * T>::kKeep || !sc.stash || gridDim.x * (uint32_t)WARPS <= sc.stash_warps;
-  if (nlist <= kSharedTilesPerCta * gridDim.x && stashes)
-    raster_tiles<T, WARPS, true>(views, sc, sm, tbase, nlist, list);
-  else
-    raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist, list);
+  if (!(sc.ctl->error & kErrNoDraw)) {
+    // this launch's part of the list (all of it unless the sequence is drawn in groups)
+    const uint32_t lo = sc.tile_lo > 0 ? sc.ne_off[sc.tile_lo] : 0u;
+    const uint32_t nlist = sc.ne_off[sc.tile_hi] - lo;
+    const uint32_t* list = sc.tile_list + lo;
+    // uniform over the grid: every warp of every CTA has a stash, or none does
+    const bool stashes = TileState<T * T>::kKeep || !sc.stash || gridDim.x * (uint32_t)WARPS <= sc.stash_warps;
+    if (nlist <= kSharedTilesPerCta * gridDim.x && stashes)
+      raster_tiles<T, WARPS, true>(views, sc, sm, tbase, nlist, list);
+    else
+      raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist, list);
+  }
+  // the sequence's last CTA hands the control block to the host
+  if (sc.ctl_out) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(sc.finished, 1u) == gridDim.x - 1u) {
+        __threadfence();
+        const uint4* from = reinterpret_cast<const uint4*>(sc.ctl);
+#pragma unroll
+        for (int k = 0; k < (int)(sizeof(Ctl) / 16); k++) reinterpret_cast<uint4*>(sc.ctl_out)[k] = __ldcg(from + k);
+        __threadfence_system();
+      }
+    }
+  }
 }
 
 template <int T, int WARPS>
@@ -594,8 +611,7 @@ static int launch_t(const DView* views, Scratch sc, int grid, cudaStream_t s) {
         cudaFuncSetAttribute(k_raster<T, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  k_raster<T, WARPS><<<grid, WARPS * 32, smem, s>>>(views, sc);
-  return (int)cudaGetLastError();
+  return launch_chained(k_raster<T, WARPS>, grid, WARPS * 32, smem, s, views, sc);
 }
 
 int launch_raster(const DView* views, int tile, Scratch sc, int grid, int warps, cudaStream_t s) {

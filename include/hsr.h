@@ -292,7 +292,7 @@ HSR_API int hsr_get_stats(hsr_stats* out);
  * hsr_plan_create validates the draws (same rules as hsr_draw_batch; a plan is one launch
  * sequence, so a draw that clears a target an earlier draw of the plan writes is refused with
  * HSR_ERR_INVALID_ARG), reserves the plan's own scratch, and records the whole launch sequence
- * (descriptor upload, counter reset, eight kernels) into a CUDA graph.  Between replays only uniforms may change
+ * (descriptors and counters, then the eight kernels of the timing block) into a CUDA graph.  Between replays only uniforms may change
  * (hsr_plan_set_uniforms); meshes, textures, targets and shaders stay those of creation.
  * hsr_plan_launch replays the graph on the library stream and returns at once;
  * hsr_plan_wait blocks until it is done and re-runs it with larger scratch if the device
@@ -380,7 +380,7 @@ HSR_API int hsr_server_inject_alloc_failures(hsr_server s, int32_t n);
 typedef struct hsr_timing {
   float batch_ms;
   float kernel_ms[HSR_KERNEL_COUNT];
-  uint32_t launches;       /* kernels launched by the sequence                         */
+  uint32_t launches;       /* kernels launched by the sequence (these and the set-up)  */
   uint32_t views;          /* draws in the sequence                                    */
   uint64_t h2d_bytes;      /* host -> device bytes of the sequence (view descriptors)  */
   uint64_t d2h_bytes;      /* device -> host bytes (control block)                     */
