@@ -649,7 +649,7 @@ int launch_emit(const DView* views, int tile, Scratch sc, int grid, cudaStream_t
 // j < n-2 of the half then build the fan triangles (:394-405).  The halves run the same
 // instructions, each masked to its own polygon; every __syncwarp is reached by all 32 lanes.
 __device__ void clip_face(bool active, const DView& v, int view, int face, int T, const Scratch& sc, float* A,
-                          float* B) {
+                          float* B, uint32_t& pay_bytes) {
   const int lane = threadIdx.x & 31, hl = lane & 15;
   if (active && hl < 3) {
     const int4 iv = __ldg(&v.fv[face]), it = __ldg(&v.fvt[face]), in = __ldg(&v.fvn[face]);
@@ -712,8 +712,7 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
   const int nf4 = payload_f4(v.shader);
   const uint32_t slot = warp_reserve(valid && !big, &sc.ctl->rec_count);
   append_small(valid && !big, slot, r, pl, nf4, v, T, sc);
-  const uint32_t pb = __reduce_add_sync(kFull, (valid && !big && slot < sc.rec_cap) ? 16u * (uint32_t)nf4 : 0u);
-  if (lane == 0 && pb) atomicAdd(&sc.ctl->pay_bytes, (unsigned long long)pb);
+  if (valid && !big && slot < sc.rec_cap) pay_bytes += 16u * (uint32_t)nf4;
   const uint32_t bslot = warp_reserve(big, &sc.ctl->big_count);
   if (big) {
     if (bslot < sc.big_cap) {
@@ -728,31 +727,32 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
 
 constexpr int kPostThreads = 256;
 
-// Drains the clip queue of k_setup, two faces per warp.  Face pairs are claimed one ahead, so
-// the claim's round trip overlaps the current pair; the grid fills every SM (the queue is short
-// and each face is a chain of dependent loads, so resident warps set the throughput).
+// The clip queue of k_setup, two faces per warp: warp w of the grid begins with pair w, and where
+// there are more pairs than warps claims the next one while it works on one (a fixed order
+// leaves some warps with the faces that make many triangles: 65k faces 100 us, claimed 88 us;
+// without claims and their round trip a short queue saves 2-8 us).  The grid fills every SM: each
+// face is a chain of dependent loads, so resident warps set the throughput.
 __global__ void __launch_bounds__(kPostThreads, 3) k_post(const DView* __restrict__ views, int T, Scratch sc) {
   __shared__ float poly[kPostThreads / 32][2][2][16 * kPolyStride];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
   chain_wait();
   if (sc.ctl->error & kErrCapacity) return;
   const uint32_t nclip = min(sc.ctl->clip_count, sc.clip_cap);
-  uint32_t item = 0, ahead = 0;
-  if (lane == 0) {
-    item = atomicAdd(&sc.ctl->post_next, 2u);
-    ahead = item < nclip ? atomicAdd(&sc.ctl->post_next, 2u) : nclip;
-  }
-  item = __shfl_sync(kFull, item, 0);
-  for (;;) {
-    if (item >= nclip) break;
-    const uint32_t next = __shfl_sync(kFull, ahead, 0);
-    if (lane == 0) ahead = next < nclip ? atomicAdd(&sc.ctl->post_next, 2u) : nclip;
+  uint32_t pay_bytes = 0;  // payload bytes this lane wrote, added to the control block once (its line
+                           // serves one atomic at a time, the record slots' among them)
+  const uint32_t claimed = 2u * gridDim.x * (kPostThreads / 32);  // pairs from here on are claimed
+  uint32_t item = 2u * (blockIdx.x * (kPostThreads / 32) + (uint32_t)warp);
+  while (item < nclip) {
+    uint32_t next = nclip;
+    if (lane == 0 && claimed < nclip) next = claimed + atomicAdd(&sc.ctl->post_next, 2u);
     const uint32_t mine = item + (uint32_t)half;
     const bool active = mine < nclip;
     const int2 vf = active ? sc.clipq[mine] : make_int2(0, 0);
-    clip_face(active, views[vf.x], vf.x, vf.y, T, sc, poly[warp][half][0], poly[warp][half][1]);
-    item = next;
+    clip_face(active, views[vf.x], vf.x, vf.y, T, sc, poly[warp][half][0], poly[warp][half][1], pay_bytes);
+    item = __shfl_sync(kFull, next, 0);
   }
+  pay_bytes = __reduce_add_sync(kFull, pay_bytes);
+  if (lane == 0 && pay_bytes) atomicAdd(&sc.ctl->pay_bytes, (unsigned long long)pay_bytes);
 }
 
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {

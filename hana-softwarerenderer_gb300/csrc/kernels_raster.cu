@@ -155,6 +155,12 @@ struct RasterSmem {
   CandQueue cq[WARPS];
   float u8f[256];
   int32_t tbase[kSharedViews];
+  // pixels shaded and candidates covered in each warp's tiles, added to the control block once: its
+  // counters share a line with the claim, and atomics on one line are served one by one (two a
+  // tile besides the claim made the claim a quarter of the time with 8x8 tiles: 2560x1440
+  // close-up 127 -> 108 us, 1280x720 grid 106 -> 86 us)
+  unsigned long long shaded[WARPS], frags[WARPS];
+  uint32_t done[WARPS];  // finished tiles of the warp's view not yet counted in view_done
   uint32_t claim;  // list position of the tile the CTA shares
 };
 
@@ -295,6 +301,10 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   }
   // views of a warp's tiles only move forward: after the first, search on from the last one
   int vi = t < ntiles ? find_view(views, tbase, sc.nviews, (int)t) : 0;
+  if (lane == 0) {
+    sm.shaded[warp] = sm.frags[warp] = 0ull;
+    sm.done[warp] = 0u;
+  }
   int ready = -1;  // the shadow map's view last seen complete
   for (;;) {
     if (t >= ntiles) break;
@@ -519,16 +529,30 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
 #undef HSR_SHADE
     shaded = __reduce_add_sync(kFull, shaded);
     if (lane == 0) {
-      if (shaded) atomicAdd(&sc.ctl->shaded_px, (unsigned long long)shaded);
-      if (frags) atomicAdd(&sc.ctl->frag_px, (unsigned long long)frags);
+      sm.shaded[warp] += shaded;
+      sm.frags[warp] += frags;
     }
+    // the next tile's view: at or behind this one
+    auto view_of = [&](uint32_t tile) {
+      if (tile >= ntiles) return -1;
+      if (!tbase) return find_view(views, tbase, sc.nviews, (int)tile);
+      int k = vi;
+      while (k + 1 < sc.nviews && tbase[k + 1] <= (int)tile) k++;
+      return k;
+    };
+    int vi_next = SHARED ? vi : view_of(t_next);
     if (v.has_dependents) {
-      // publish this tile's writes before counting it done (a later view reads them)
-      __threadfence();
-      if (SHARED) __syncthreads(); else __syncwarp();
-      if (SHARED ? threadIdx.x == 0 : lane == 0) {
-        if (v.has_dependents & kTargetReaders) atomicAdd(&sc.view_done[vi], 1u);
-        if (v.has_dependents & kTileReaders) atomicExch(&sc.tile_fill[t], kTileDone);
+      // publish this tile's writes before counting it done (a later view reads them); a warp counts
+      // its tiles of a view at once when it leaves the view, which is when its last one is done
+      if (lane == 0) sm.done[warp]++;
+      if (SHARED || vi_next != vi || (v.has_dependents & kTileReaders)) {
+        __threadfence();
+        if (SHARED) __syncthreads(); else __syncwarp();
+        if (SHARED ? threadIdx.x == 0 : lane == 0) {
+          if (v.has_dependents & kTargetReaders) atomicAdd(&sc.view_done[vi], sm.done[warp]);
+          if (v.has_dependents & kTileReaders) atomicExch(&sc.tile_fill[t], kTileDone);
+          sm.done[warp] = 0u;
+        }
       }
     }
     if (SHARED) {
@@ -541,17 +565,16 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         n_next = sc.tile_count[t_next];
         off_next = sc.tile_off[t_next];
       }
+      vi_next = view_of(t_next);
     }
     t = t_next;
     n = n_next;
     off = off_next;
-    if (t < ntiles) {
-      if (tbase) {
-        while (vi + 1 < sc.nviews && tbase[vi + 1] <= (int)t) vi++;
-      } else {
-        vi = find_view(views, tbase, sc.nviews, (int)t);
-      }
-    }
+    vi = vi_next;
+  }
+  if (lane == 0) {
+    if (sm.shaded[warp]) atomicAdd(&sc.ctl->shaded_px, sm.shaded[warp]);
+    if (sm.frags[warp]) atomicAdd(&sc.ctl->frag_px, sm.frags[warp]);
   }
 }
 
