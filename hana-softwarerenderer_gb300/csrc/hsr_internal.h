@@ -150,7 +150,7 @@ static_assert(offsetof(DView, prim_base) + sizeof(uint32_t) <= 128, "per-tile fi
 struct Ctl {
   uint32_t rec_count;
   uint32_t clip_count;
-  uint32_t tile_next;      // the one tile counter of a sequence drawn by one raster launch
+  uint32_t reserved;
   uint32_t scan_ticket;
   uint32_t error;
   uint32_t bin_total;
@@ -182,8 +182,8 @@ constexpr int kSharedViews = 256;  // views whose chunk / tile bases kernels cop
 // Scratch of one launch sequence (device pointers, sized by the host).
 struct Scratch {
   Ctl* ctl;
-  uint32_t* view_done;      // [nviews] tiles finished per view, then [kRasterGroups] tile counters and
-                            // the count of finished raster CTAs
+  uint32_t* view_done;      // [nviews] tiles finished per view, then [2 * kRasterGroups] tile counters
+                            // and the count of finished raster CTAs
   RasterRec* recs;  uint32_t rec_cap;
   Payload* pay;             // [rec_cap]
   int2* clipq;      uint32_t clip_cap;   // (view, face) of faces that need clipping
@@ -197,7 +197,8 @@ struct Scratch {
   uint32_t* bins;   uint32_t bin_cap;
   int32_t ntiles;
   int32_t nviews;
-  // the raster launch's part of the tiles, [tile_lo, tile_hi), and the counter that hands out its tiles
+  // the raster launch's part of the tiles, [tile_lo, tile_hi), and the two counters that hand out its
+  // tiles (to warps, and at the end of the list to CTAs)
   int32_t tile_lo, tile_hi;
   uint32_t* claim;
   // where the raster's last CTA (counted by `finished`) stores the control block: mapped host

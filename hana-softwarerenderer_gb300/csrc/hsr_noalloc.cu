@@ -127,7 +127,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   const size_t o_clip = off; off = nal(off + sizeof(float4) * (size_t)std::max(m->npos, 1));
   const size_t o_zero = off;
   const size_t o_ctl = off; off = nal(off + sizeof(Ctl));
-  const size_t o_done = off; off = nal(off + sizeof(uint32_t));
+  const size_t o_done = off; off = nal(off + sizeof(uint32_t) * (1 + 2));
   const size_t o_cnt = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_fill = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_stat = off; off = nal(off + sizeof(unsigned long long) * (size_t)std::max(nscan, 1));
@@ -166,7 +166,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   sc.ntiles = (int32_t)tiles;
   sc.nviews = 1;
   sc.tile_hi = sc.ntiles;
-  sc.claim = &sc.ctl->tile_next;
+  sc.claim = sc.view_done + 1;
 
   // ---- the launch sequence of hsr_draw on the static scratch ------------------------------
   cudaStream_t s = rt->stream;

@@ -257,7 +257,7 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 template <int T, int WARPS, bool SHARED>
 __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, const Scratch& sc,
                                              RasterSmem<T, WARPS>& sm, const int32_t* tbase, uint32_t nlist,
-                                             const uint32_t* tile_list) {
+                                             const uint32_t* tile_list, uint32_t* claim) {
   constexpr int NPIX = T * T;
   constexpr int PPL = NPIX / 32;
   constexpr bool kKeep = TileState<NPIX>::kKeep;
@@ -283,13 +283,13 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   const uint32_t upto = (2u << lane) - 1u;  // this lane and those below
   uint32_t li = 0, li_ahead = 0;  // positions in the list
   if (SHARED) {
-    if (threadIdx.x == 0) sm.claim = atomicAdd(sc.claim, 1u);
+    if (threadIdx.x == 0) sm.claim = atomicAdd(claim, 1u);
     __syncthreads();
     li = sm.claim;
   } else {
     if (lane == 0) {
-      li = atomicAdd(sc.claim, 1u);
-      li_ahead = atomicAdd(sc.claim, 1u);
+      li = atomicAdd(claim, 1u);
+      li_ahead = atomicAdd(claim, 1u);
     }
     li = __shfl_sync(kFull, li, 0);
   }
@@ -311,7 +311,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     uint32_t t_next = ntiles, n_next = 0, off_next = 0;
     if (!SHARED) {
       const uint32_t li_next = __shfl_sync(kFull, li_ahead, 0);
-      if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(sc.claim, 1u) : nlist;
+      if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(claim, 1u) : nlist;
       if (li_next < nlist) t_next = tile_list[li_next];
       if (t_next < ntiles) {
         n_next = sc.tile_count[t_next];
@@ -557,7 +557,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     }
     if (SHARED) {
       __syncthreads();  // the merged state and the claim word are free again
-      if (threadIdx.x == 0) sm.claim = atomicAdd(sc.claim, 1u);
+      if (threadIdx.x == 0) sm.claim = atomicAdd(claim, 1u);
       __syncthreads();
       li = sm.claim;
       if (li < nlist) t_next = tile_list[li];
@@ -585,6 +585,12 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
 // the barriers cost: the two are equal at about 10 tiles per CTA (86 us each at 10.6) and one
 // warp per tile wins by 1.55x at 20 (113 against 176 us) and 1.7x at 47.
 constexpr uint32_t kSharedTilesPerCta = 4;
+// A longer list ends the same way: the warps that take its last tiles finish long after the others
+// have none left (a quarter of the warps' time of a 16-view batch).  There each CTA shares one of
+// the last gridDim.x tiles, where the lists hold at least kTailRecords records a tile on average:
+// 16 views (40 records a tile) 334 -> 315 us, 1000x600 with shadow (4.4) 70 -> 63 us, 1080p
+// frame (11) 195 -> 190 us; the 2560x1440 close-up (2.3) has nothing to share, 96 -> 99 us.
+constexpr unsigned long long kTailRecords = 3;
 
 // Four-warp CTAs are compiled for 7 per SM (72 registers a thread, fewer spills than at 8 per
 // SM's 64: measured faster on the serving batches, 1.72 -> 1.65 ms).
@@ -605,10 +611,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
     const uint32_t* list = sc.tile_list + lo;
     // uniform over the grid: every warp of every CTA has a stash, or none does
     const bool stashes = TileState<T * T>::kKeep || !sc.stash || gridDim.x * (uint32_t)WARPS <= sc.stash_warps;
-    if (nlist <= kSharedTilesPerCta * gridDim.x && stashes)
-      raster_tiles<T, WARPS, true>(views, sc, sm, tbase, nlist, list);
-    else
-      raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist, list);
+    // the tiles at the list's end that CTAs share
+    const bool long_lists = (unsigned long long)sc.ctl->bin_total >= kTailRecords * (unsigned long long)sc.ctl->ne_tiles;
+    const uint32_t shared = !stashes ? 0u : nlist <= kSharedTilesPerCta * gridDim.x ? nlist : long_lists ? gridDim.x : 0u;
+    if (shared < nlist) raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist - shared, list, sc.claim);
+    if (shared > 0u) {
+      __syncthreads();
+      raster_tiles<T, WARPS, true>(views, sc, sm, tbase, shared, list + (nlist - shared), sc.claim + 1);
+    }
   }
   // the sequence's last CTA hands the control block to the host
   if (sc.ctl_out) {
