@@ -319,6 +319,51 @@ __device__ __forceinline__ void st_v8(void* p, float4 a, float4 b) {
                "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
                : "memory");
 }
+// The (record, tile) pairs of a warp's records, 32 at a time: lane l's record covers `nt` tiles (0:
+// none, at most 32) in rows of `ntw` from tile `tile0`, `tiles_x` apart.  f(in, tile, owner) is called by
+// all lanes with one pair each (`in`: this lane has one; owner: the lane of its record).
+// Walking the pairs rather than each lane its own tiles makes the number of steps, each with an
+// atomic's round trip in the scatter, the sum of the tile counts / 32 and not their maximum; it
+// takes ten shuffles a step, so it is done where that halves the steps (emit / scatter of the
+// 4M-triangle soup 84 -> 68 / 170 -> 150 us, 1000x600 with shadow scatter 29 -> 22 us).
+template <class F>
+__device__ __forceinline__ void for_each_pair(int nt, int ntw, int tile0, int tiles_x, F f) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (!__any_sync(kAll, nt > 1)) {
+    if (__any_sync(kAll, nt > 0)) f(nt > 0, tile0, lane);
+    return;
+  }
+  const int magic = (65535 + ntw) / ntw;  // k / ntw = (k * magic) >> 16 for k < 32, ntw <= 32
+  int incl = nt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kAll, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int total = __shfl_sync(kAll, incl, 31);
+  const int most = __reduce_max_sync(kAll, nt);
+  if (total >= 16 * most) {  // even counts (the sub-records of a split triangle): each lane its own tiles
+    int kx = 0, row = tile0;
+    for (int k = 0; k < most; k++) {
+      f(k < nt, row + kx, lane);
+      if (++kx == ntw) { kx = 0; row += tiles_x; }
+    }
+    return;
+  }
+  for (int base = 0; base < total; base += 32) {
+    const int i = base + lane;
+    int own = 0;  // records whose pairs end at or before pair i
+#pragma unroll
+    for (int s = 16; s; s >>= 1)
+      if (__shfl_sync(kAll, incl, own + s - 1) <= i) own += s;
+    const int k = i - (__shfl_sync(kAll, incl - nt, own));
+    const int w = __shfl_sync(kAll, ntw, own), ky = (k * __shfl_sync(kAll, magic, own)) >> 16;
+    const int tile = __shfl_sync(kAll, tile0, own) + ky * __shfl_sync(kAll, tiles_x, own) + (k - ky * w);
+    f(i < total, tile, own);
+  }
+}
+
 // set_color (renderbuffer.cpp:38-44): R, G, B through (uchar)(c*255); alpha kept.
 __device__ __forceinline__ uint32_t pack_rgb(Col c, uint32_t alpha_word) {
   uint32_t r = (uint32_t)cvt_i32(fm(c.r, 255.f)) & 255u;

@@ -184,36 +184,30 @@ __device__ __forceinline__ void scatter_records(const DView* __restrict__ views,
   for (uint32_t i0 = block * blockDim.x + (threadIdx.x & ~31u); i0 < nrec; i0 += stride) {
     const uint32_t i = i0 + (uint32_t)lane;
     const bool ok = i < nrec;
-    int tx0 = 0, ty0 = 0, ntw = 0, nt = 0, tbase = 0, tiles_x = 0;
+    int ntw = 1, nt = 0, tile0 = 0, tiles_x = 0;
     // the record's view and pixel range: its last 16 bytes (seq, view, xr, yr) in one load
     const uint4 w = ok ? *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(&sc.recs[i]) + 48)
                        : make_uint4(0u, kRecHole << kRecFlagShift, 0u, 0u);
     if (ok && !((w.y >> kRecFlagShift) & kRecHole)) {  // holes: huge triangles split by k_big
       const uint32_t xr = w.z, yr = w.w;
       const DView& v = views[w.y & kRecViewMask];
-      tbase = v.tile_base;
       tiles_x = v.tiles_x;
-      tx0 = (int)(xr & 0xffffu) >> ts;
-      ty0 = (int)(yr & 0xffffu) >> ts;
+      const int tx0 = (int)(xr & 0xffffu) >> ts, ty0 = (int)(yr & 0xffffu) >> ts;
+      tile0 = v.tile_base + ty0 * tiles_x + tx0;
       ntw = ((int)(xr >> 16) >> ts) - tx0 + 1;
-      nt = ntw * (((int)(yr >> 16) >> ts) - ty0 + 1);
+      nt = min(ntw * (((int)(yr >> 16) >> ts) - ty0 + 1), kMaxRecordTiles);
     }
-    const int my_n = min(nt, kMaxRecordTiles);
-    const int maxn = __reduce_max_sync(kFull, my_n);
-    int kx = 0, ky = 0;  // tile k of the rectangle, row-major
-    for (int k = 0; k < maxn; k++) {
-      const int tile = (k < my_n) ? tbase + (ty0 + ky) * tiles_x + tx0 + kx : -1;
-      if (++kx == ntw) { kx = 0; ky++; }
-      const unsigned grp = __match_any_sync(kFull, tile);
+    for_each_pair(nt, ntw, tile0, tiles_x, [&](bool in, int tile, int own) {
+      const unsigned grp = __match_any_sync(kFull, in ? tile : -1);
       const int leader = __ffs(grp) - 1;
       uint32_t b = 0;
-      if (tile >= 0 && lane == leader) b = atomicAdd(&sc.tile_fill[tile], (uint32_t)__popc(grp));
+      if (in && lane == leader) b = atomicAdd(&sc.tile_fill[tile], (uint32_t)__popc(grp));
       b = __shfl_sync(kFull, b, leader);
-      if (tile >= 0) {
+      if (in) {
         const uint32_t pos = sc.tile_off[tile] + b + (uint32_t)__popc(grp & ((1u << lane) - 1u));
-        if (pos < sc.bin_cap) sc.bins[pos] = i;
+        if (pos < sc.bin_cap) sc.bins[pos] = i0 + (uint32_t)own;
       }
-    }
+    });
   }
 }
 
@@ -309,6 +303,7 @@ __global__ void __launch_bounds__(256) k_scatter(const DView* __restrict__ views
   __shared__ int32_t s_cbase[kSharedViews];
   const uint32_t b = blockIdx.x, g = gridDim.x;
   chain_wait();
+  if (sc.ctl->ne_tiles >= (uint32_t)sc.ntiles) nchunks = 0;  // every tile is the raster's: all blocks scatter
   if (nchunks > 0 && b % kClearEvery == kClearEvery - 1) {  // block-uniform
     const bool in_shared = sc.nviews <= kSharedViews;
     if (in_shared)

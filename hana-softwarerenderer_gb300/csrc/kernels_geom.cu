@@ -411,14 +411,10 @@ __device__ void append_counts(bool valid, uint32_t slot, const RasterRec& r, con
     store_payload(&sc.pay[slot], pl, nf4);
     rec_tiles(r, T, tx0, ty0, ntw, nt);
   }
-  const int maxn = __reduce_max_sync(kFull, nt);
-  int kx = 0, ky = 0;  // tile k of the rectangle = (kx, ky), row-major
-  for (int k = 0; k < maxn; k++) {
-    const int tile = (k < nt) ? v.tile_base + (ty0 + ky) * v.tiles_x + tx0 + kx : -1;
-    const unsigned grp = __match_any_sync(kFull, tile);
-    if (tile >= 0 && lane == __ffs(grp) - 1) atomicAdd(&sc.tile_count[tile], (uint32_t)__popc(grp));
-    if (++kx == ntw) { kx = 0; ky++; }
-  }
+  for_each_pair(nt, ntw, v.tile_base + ty0 * v.tiles_x + tx0, v.tiles_x, [&](bool in, int tile, int) {
+    const unsigned grp = __match_any_sync(kFull, in ? tile : -1);
+    if (in && lane == __ffs(grp) - 1) atomicAdd(&sc.tile_count[tile], (uint32_t)__popc(grp));
+  });
 }
 
 // append_counts at slots reserved by the caller, checked against the record capacity.
