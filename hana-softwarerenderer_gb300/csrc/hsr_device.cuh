@@ -326,8 +326,10 @@ __device__ __forceinline__ void st_v8(void* p, float4 a, float4 b) {
 // atomic's round trip in the scatter, the sum of the tile counts / 32 and not their maximum; it
 // takes ten shuffles a step, so it is done where that halves the steps (emit / scatter of the
 // 4M-triangle soup 84 -> 68 / 170 -> 150 us, 1000x600 with shadow scatter 29 -> 22 us).
-template <class F>
-__device__ __forceinline__ void for_each_pair(int nt, int ntw, int tile0, int tiles_x, F f) {
+// `even(most)`, where the lanes' counts are close to their maximum `most` (the sub-records of a split
+// triangle): the caller walks each lane's own tiles.
+template <class F, class E>
+__device__ __forceinline__ void for_each_pair(int nt, int ntw, int tile0, int tiles_x, F f, E even) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   if (!__any_sync(kAll, nt > 1)) {
@@ -343,12 +345,8 @@ __device__ __forceinline__ void for_each_pair(int nt, int ntw, int tile0, int ti
   }
   const int total = __shfl_sync(kAll, incl, 31);
   const int most = __reduce_max_sync(kAll, nt);
-  if (total >= 16 * most) {  // even counts (the sub-records of a split triangle): each lane its own tiles
-    int kx = 0, row = tile0;
-    for (int k = 0; k < most; k++) {
-      f(k < nt, row + kx, lane);
-      if (++kx == ntw) { kx = 0; row += tiles_x; }
-    }
+  if (total >= 16 * most) {
+    even(most);
     return;
   }
   for (int base = 0; base < total; base += 32) {

@@ -411,9 +411,17 @@ __device__ void append_counts(bool valid, uint32_t slot, const RasterRec& r, con
     store_payload(&sc.pay[slot], pl, nf4);
     rec_tiles(r, T, tx0, ty0, ntw, nt);
   }
-  for_each_pair(nt, ntw, v.tile_base + ty0 * v.tiles_x + tx0, v.tiles_x, [&](bool in, int tile, int) {
+  auto count = [&](bool in, int tile, int) {
     const unsigned grp = __match_any_sync(kFull, in ? tile : -1);
     if (in && lane == __ffs(grp) - 1) atomicAdd(&sc.tile_count[tile], (uint32_t)__popc(grp));
+  };
+  const int tile0 = v.tile_base + ty0 * v.tiles_x + tx0;
+  for_each_pair(nt, ntw, tile0, v.tiles_x, count, [&](int most) {
+    int kx = 0, row = tile0;
+    for (int k = 0; k < most; k++) {
+      count(k < nt, row + kx, lane);
+      if (++kx == ntw) { kx = 0; row += v.tiles_x; }
+    }
   });
 }
 
