@@ -148,9 +148,9 @@ constexpr int64_t kMaxBatchTiles = (int64_t)1 << 26;  // tiles of one launch seq
 static_assert(offsetof(DView, prim_base) + sizeof(uint32_t) <= 128, "per-tile fields must share one line");
 
 struct Ctl {
-  uint32_t rec_count;
+  uint32_t rec_count;      // records of the cull pass
   uint32_t clip_count;
-  uint32_t reserved;
+  uint32_t rec_extra;      // records appended behind them (clipped triangles, sub-records)
   uint32_t scan_ticket;
   uint32_t error;
   uint32_t bin_total;
@@ -222,7 +222,8 @@ constexpr int kStashWarpsPerSm = 32;  // raster warps resident per SM at most
 int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s);
 int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s);
 int launch_setup(const DView* views, int nviews, int nchunks, Scratch sc, int grid, cudaStream_t s);
-int launch_emit(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
+bool clips_with_emit(size_t faces);  // the emit pass's grid also clips (no launch_post)
+int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms, cudaStream_t s);
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
 int launch_big(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
 int launch_scan(Scratch sc, cudaStream_t s);

@@ -344,10 +344,11 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
   kr = launch_setup(dviews, n, nsch, sc, num_sms * 8, s);
   if (kr) return cuda_fail((cudaError_t)kr, "setup kernel");
   mark(3);
-  kr = launch_emit(dviews, tile, sc, num_sms * 8, s);
+  const bool one_grid = clips_with_emit(total_faces);
+  kr = launch_emit(dviews, tile, sc, one_grid, num_sms, s);
   if (kr) return cuda_fail((cudaError_t)kr, "emit kernel");
   mark(4);
-  kr = launch_post(dviews, tile, sc, num_sms * 4, s);
+  kr = one_grid ? 0 : launch_post(dviews, tile, sc, num_sms * 4, s);
   if (kr) return cuda_fail((cudaError_t)kr, "post kernel");
   mark(5);
   kr = launch_big(dviews, tile, sc, num_sms * 2, s);
@@ -382,14 +383,14 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
 }
 
 int Plan::kernel_count() const {
-  return 1 + (nvch ? 1 : 0) + (nsch ? 1 : 0) + 3 + (nscan > 0 ? 1 : 0) + 2;
+  return 1 + (nvch ? 1 : 0) + (nsch ? 1 : 0) + (clips_with_emit(total_faces) ? 2 : 3) + (nscan > 0 ? 1 : 0) + 2;
 }
 
 // Grow the capacity an overflow reported; returns false if nothing overflowed.
 bool Plan::grow(const Ctl& c) {
   if (!(c.error & kErrCapacity)) return false;
   if (c.error & kErrBigOverflow) big_cap = std::max<size_t>(big_cap * 2, (size_t)c.big_count + 256);
-  if (c.error & kErrRecOverflow) rec_cap = std::max<size_t>(rec_cap * 2, (size_t)c.rec_count + 1024);
+  if (c.error & kErrRecOverflow) rec_cap = std::max<size_t>(rec_cap * 2, (size_t)c.rec_count + c.rec_extra + 1024);
   if (c.error & kErrClipOverflow) clip_cap = std::max<size_t>(clip_cap * 2, (size_t)c.clip_count + 256);
   if (c.error & kErrBinOverflow) bin_cap = std::max<size_t>(bin_cap * 2, (size_t)c.bin_total + 4096);
   return true;
@@ -403,11 +404,11 @@ void Runtime::learn_caps(const Plan& p) {
 }
 
 void Runtime::record_result(const Plan& p, const Ctl& c) {
-  stats.records = c.rec_count;
+  stats.records = (uint64_t)c.rec_count + c.rec_extra;
   stats.clipped_faces = c.clip_count;
   stats.bin_pairs = c.bin_total;
   stats.tiles = p.total_tiles;
-  timing.records = c.rec_count;
+  timing.records = stats.records;
   timing.bin_pairs = c.bin_total;
   timing.shaded_pixels = c.shaded_px;
   timing.fragments = c.frag_px;
@@ -484,7 +485,8 @@ int Runtime::run_sequence(const hsr_draw_desc* descs, int n) {
     cudaEventElapsedTime(&ms, ev[0], ev[kEvents - 1]);
     timing.batch_ms = ms;
     for (int k = 0; k < HSR_KERNEL_COUNT; k++) {
-      float km = 0.f;
+      float km = timing.kernel_ms[k] = 0.f;
+      if (k == 3 && clips_with_emit(p.total_faces)) continue;  // clipped in the emit pass's grid
       if (profiling) cudaEventElapsedTime(&km, ev[k + 1], ev[k + 2]);
       timing.kernel_ms[k] = km;
     }

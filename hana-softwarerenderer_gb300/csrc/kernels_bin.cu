@@ -176,7 +176,7 @@ int launch_scan(Scratch sc, cudaStream_t s) {
 __device__ __forceinline__ void scatter_records(const DView* __restrict__ views, int T, const Scratch& sc, uint32_t block,
                                                 uint32_t nblocks) {
   const int lane = threadIdx.x & 31;
-  const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
+  const uint32_t nrec = min(sc.ctl->rec_count + sc.ctl->rec_extra, sc.rec_cap);
   if (sc.ctl->error & kErrNoDraw) return;
   const uint32_t stride = nblocks * blockDim.x;
   const int ts = __ffs(T) - 1;  // T is a power of two

@@ -587,73 +587,13 @@ __device__ __forceinline__ void face_payload(const DView& v, int f, int nf4, int
   pl.f[31] = 0.f;
 }
 
-// Emit pass over the records of k_setup (dense: one thread per surviving triangle): the
-// shading payload, the tile counts, and the hand-over of huge triangles to k_big (their
-// slot becomes a hole the binning skips).  Grid-stride with warp-uniform trip counts, so
-// the warp collectives of append_small see every lane.
-__global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* __restrict__ views, int T, Scratch sc) {
-  const int lane = threadIdx.x & 31;
-  chain_wait();
-  if (sc.ctl->error & kErrCapacity) return;
-  const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
-  const uint32_t stride = gridDim.x * blockDim.x;
-  uint32_t pay_bytes = 0;  // payload bytes this lane wrote for the raster (big ones: k_big)
-  for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < nrec; i0 += stride) {
-    const uint32_t i = i0 + (uint32_t)lane;
-    bool valid = false;
-    RasterRec r;
-    Payload pl;
-    int nf4 = 0;
-    const DView* v = views;
-    if (i < nrec) {
-      // the words this pass needs (seq, view, pixel range: the record's last 16 bytes); the
-      // whole record only for a huge triangle.  Every record below the count is the cull
-      // pass's: the clipper and k_big append theirs after this pass.
-      const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(&sc.recs[i]) + 48);
-      r.seq = a.x; r.view = a.y; r.xr = a.z; r.yr = a.w;
-      valid = true;
-      v = views + (r.view & kRecViewMask);
-      nf4 = payload_f4(v->shader);
-      if (nf4 > 0) {
-        const int f = (int)(r.seq >> 4);
-        face_payload(*v, f, nf4, __ldg(&v->fv[f]), pl);
-      }
-    }
-    int tx0, ty0, ntw, nt = 0;
-    if (valid) rec_tiles(r, T, tx0, ty0, ntw, nt);
-    const bool big = valid && nt > kMaxRecordTiles;
-    const bool small = valid && !big;
-    if (small) {
-      pay_bytes += 16u * (uint32_t)nf4;
-    }
-    append_counts(small, i, r, pl, nf4, *v, T, sc, true);
-    const uint32_t bslot = warp_reserve(big, &sc.ctl->big_count);
-    if (big) {
-      r = sc.recs[i];
-      sc.recs[i].view = r.view | (kRecHole << kRecFlagShift);
-      if (bslot < sc.big_cap) {
-        store_rec(&sc.bigq[bslot].rec, r);
-        store_payload(&sc.bigq[bslot].pay, pl, nf4);
-      } else {
-        atomicOr(&sc.ctl->error, kErrBigOverflow);
-      }
-    }
-  }
-  pay_bytes = __reduce_add_sync(kFull, pay_bytes);
-  if (lane == 0 && pay_bytes) atomicAdd(&sc.ctl->pay_bytes, (unsigned long long)pay_bytes);
-}
-
-int launch_emit(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {
-  return launch_chained(k_emit, grid, kEmitThreads, 0, s, views, tile, sc);
-}
-
 // Homogeneous clipping (graphics.cpp:73-161), two faces per warp: each half-warp clips its own
 // face (`active`), lane k of the half carrying varying k of the polygon through
 // Sutherland-Hodgman while every lane evaluates the plane tests on the clip coordinates; lanes
 // j < n-2 of the half then build the fan triangles (:394-405).  The halves run the same
 // instructions, each masked to its own polygon; every __syncwarp is reached by all 32 lanes.
 __device__ void clip_face(bool active, const DView& v, int view, int face, int T, const Scratch& sc, float* A,
-                          float* B, uint32_t& pay_bytes) {
+                          float* B, uint32_t rec_base, uint32_t& pay_bytes) {
   const int lane = threadIdx.x & 31, hl = lane & 15;
   if (active && hl < 3) {
     const int4 iv = __ldg(&v.fv[face]), it = __ldg(&v.fvt[face]), in = __ldg(&v.fvn[face]);
@@ -714,7 +654,7 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
   if (valid) rec_tiles(r, T, tx0, ty0, ntw, nt);
   const bool big = valid && nt > kMaxRecordTiles;
   const int nf4 = payload_f4(v.shader);
-  const uint32_t slot = warp_reserve(valid && !big, &sc.ctl->rec_count);
+  const uint32_t slot = rec_base + warp_reserve(valid && !big, &sc.ctl->rec_extra);
   append_small(valid && !big, slot, r, pl, nf4, v, T, sc);
   if (valid && !big && slot < sc.rec_cap) pay_bytes += 16u * (uint32_t)nf4;
   const uint32_t bslot = warp_reserve(big, &sc.ctl->big_count);
@@ -729,38 +669,127 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
   __syncwarp();
 }
 
-constexpr int kPostThreads = 256;
+// Emit pass over the records of k_setup (dense: one thread per surviving triangle): the
+// shading payload, the tile counts, and the hand-over of huge triangles to k_big (their
+// slot becomes a hole the binning skips).  Grid-stride with warp-uniform trip counts, so
+// the warp collectives of append_small see every lane.
+__device__ __forceinline__ void emit_records(const DView* __restrict__ views, int T, const Scratch& sc, uint32_t block,
+                                             uint32_t nblocks) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
+  const uint32_t stride = nblocks * blockDim.x;
+  uint32_t pay_bytes = 0;  // payload bytes this lane wrote for the raster (big ones: k_big)
+  for (uint32_t i0 = block * blockDim.x + (threadIdx.x & ~31u); i0 < nrec; i0 += stride) {
+    const uint32_t i = i0 + (uint32_t)lane;
+    bool valid = false;
+    RasterRec r;
+    Payload pl;
+    int nf4 = 0;
+    const DView* v = views;
+    if (i < nrec) {
+      // the words this pass needs (seq, view, pixel range: the record's last 16 bytes); the
+      // whole record only for a huge triangle.  Every record below rec_count is the
+      // cull pass's: the clipper and k_big append theirs behind it.
+      const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(&sc.recs[i]) + 48);
+      r.seq = a.x; r.view = a.y; r.xr = a.z; r.yr = a.w;
+      valid = true;
+      v = views + (r.view & kRecViewMask);
+      nf4 = payload_f4(v->shader);
+      if (nf4 > 0) {
+        const int f = (int)(r.seq >> 4);
+        face_payload(*v, f, nf4, __ldg(&v->fv[f]), pl);
+      }
+    }
+    int tx0, ty0, ntw, nt = 0;
+    if (valid) rec_tiles(r, T, tx0, ty0, ntw, nt);
+    const bool big = valid && nt > kMaxRecordTiles;
+    const bool small = valid && !big;
+    if (small) {
+      pay_bytes += 16u * (uint32_t)nf4;
+    }
+    append_counts(small, i, r, pl, nf4, *v, T, sc, true);
+    const uint32_t bslot = warp_reserve(big, &sc.ctl->big_count);
+    if (big) {
+      r = sc.recs[i];
+      sc.recs[i].view = r.view | (kRecHole << kRecFlagShift);
+      if (bslot < sc.big_cap) {
+        store_rec(&sc.bigq[bslot].rec, r);
+        store_payload(&sc.bigq[bslot].pay, pl, nf4);
+      } else {
+        atomicOr(&sc.ctl->error, kErrBigOverflow);
+      }
+    }
+  }
+  pay_bytes = __reduce_add_sync(kFull, pay_bytes);
+  if (lane == 0 && pay_bytes) atomicAdd(&sc.ctl->pay_bytes, (unsigned long long)pay_bytes);
+}
 
 // The clip queue of k_setup, two faces per warp: warp w of the grid begins with pair w, and where
 // there are more pairs than warps claims the next one while it works on one (a fixed order
 // leaves some warps with the faces that make many triangles: 65k faces 100 us, claimed 88 us;
-// without claims and their round trip a short queue saves 2-8 us).  The grid fills every SM: each
-// face is a chain of dependent loads, so resident warps set the throughput.
-__global__ void __launch_bounds__(kPostThreads, 3) k_post(const DView* __restrict__ views, int T, Scratch sc) {
-  __shared__ float poly[kPostThreads / 32][2][2][16 * kPolyStride];
+// without claims and their round trip a short queue saves 2-8 us).  Each face is a chain of
+// dependent loads, so resident warps set the throughput.
+__device__ __forceinline__ void clip_queue(const DView* __restrict__ views, int T, const Scratch& sc, uint32_t block,
+                                           uint32_t nblocks) {
+  __shared__ float poly[kEmitThreads / 32][2][2][kMaxPoly * kPolyStride];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
-  chain_wait();
-  if (sc.ctl->error & kErrCapacity) return;
   const uint32_t nclip = min(sc.ctl->clip_count, sc.clip_cap);
+  const uint32_t rec_base = sc.ctl->rec_count;  // the cull pass's records come first
   uint32_t pay_bytes = 0;  // payload bytes this lane wrote, added to the control block once (its line
                            // serves one atomic at a time, the record slots' among them)
-  const uint32_t claimed = 2u * gridDim.x * (kPostThreads / 32);  // pairs from here on are claimed
-  uint32_t item = 2u * (blockIdx.x * (kPostThreads / 32) + (uint32_t)warp);
+  const uint32_t claimed = 2u * nblocks * (kEmitThreads / 32);  // pairs from here on are claimed
+  uint32_t item = 2u * (block * (kEmitThreads / 32) + (uint32_t)warp);
   while (item < nclip) {
     uint32_t next = nclip;
     if (lane == 0 && claimed < nclip) next = claimed + atomicAdd(&sc.ctl->post_next, 2u);
     const uint32_t mine = item + (uint32_t)half;
     const bool active = mine < nclip;
     const int2 vf = active ? sc.clipq[mine] : make_int2(0, 0);
-    clip_face(active, views[vf.x], vf.x, vf.y, T, sc, poly[warp][half][0], poly[warp][half][1], pay_bytes);
+    clip_face(active, views[vf.x], vf.x, vf.y, T, sc, poly[warp][half][0], poly[warp][half][1], rec_base, pay_bytes);
     item = __shfl_sync(kFull, next, 0);
   }
   pay_bytes = __reduce_add_sync(kFull, pay_bytes);
   if (lane == 0 && pay_bytes) atomicAdd(&sc.ctl->pay_bytes, (unsigned long long)pay_bytes);
 }
 
+// Emit and clip both read what k_setup left and append independently (the clipper's records go
+// behind the cull pass's, counted apart).  CLIP: one grid, whose first `clip_blocks` blocks clip
+// while the others emit; otherwise the grid emits, and k_post clips after it.
+template <bool CLIP>
+__global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* __restrict__ views, int T, Scratch sc,
+                                                          int clip_blocks) {
+  chain_wait();
+  if (sc.ctl->error & kErrCapacity) return;
+  if (CLIP && (int)blockIdx.x < clip_blocks) {
+    clip_queue(views, T, sc, blockIdx.x, (uint32_t)clip_blocks);
+    return;
+  }
+  const uint32_t first = CLIP ? (uint32_t)clip_blocks : 0u;
+  emit_records(views, T, sc, blockIdx.x - first, gridDim.x - first);
+}
+
+__global__ void __launch_bounds__(kEmitThreads, 3) k_post(const DView* __restrict__ views, int T, Scratch sc) {
+  chain_wait();
+  if (sc.ctl->error & kErrCapacity) return;
+  clip_queue(views, T, sc, blockIdx.x, gridDim.x);
+}
+
+// For a small sequence the shorter chain counts: one grid saves a launch and the clipper's latency
+// (whole calls: 1000x600 with shadow, 10k faces, 158 -> 150 us; 1080p frame, 655k faces, 360 -> 352
+// us).  For a large one the clipper's registers and shared memory cost the emit pass more than the
+// overlap gains (16 views, 2.4M faces: equal; 4M-triangle soup 68 + 22 -> 90 us; 64 requests, 40M
+// faces, 401 + 84 -> 565 us).
+constexpr size_t kOneGridFaces = (size_t)1 << 21;
+bool clips_with_emit(size_t faces) { return faces <= kOneGridFaces; }
+
+int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms, cudaStream_t s) {
+  const int clip_blocks = clip ? num_sms * 2 : 0, grid = clip_blocks + num_sms * 8;
+  return clip ? launch_chained(k_emit<true>, grid, kEmitThreads, 0, s, views, tile, sc, clip_blocks)
+              : launch_chained(k_emit<false>, grid, kEmitThreads, 0, s, views, tile, sc, clip_blocks);
+}
+
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {
-  return launch_chained(k_post, grid, kPostThreads, 0, s, views, tile, sc);
+  return launch_chained(k_post, grid, kEmitThreads, 0, s, views, tile, sc);
 }
 
 constexpr int kBigThreads = 512;
@@ -786,7 +815,7 @@ __global__ void __launch_bounds__(kBigThreads) k_big(const DView* __restrict__ v
     const int nsub = nbx * nby;
     __syncthreads();
     if (threadIdx.x == 0) {
-      const uint32_t base = atomicAdd(&sc.ctl->rec_count, (uint32_t)nsub);
+      const uint32_t base = sc.ctl->rec_count + atomicAdd(&sc.ctl->rec_extra, (uint32_t)nsub);
       s_base = base;
       if ((uint64_t)base + (uint64_t)nsub > (uint64_t)sc.rec_cap) atomicOr(&sc.ctl->error, kErrRecOverflow);
     }

@@ -271,7 +271,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     const uint32_t gw = blockIdx.x * (uint32_t)WARPS + (uint32_t)warp;
     if (sc.stash && gw < sc.stash_warps) stash = sc.stash + (size_t)gw * (size_t)stash_floats(T);
   }
-  const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
+  const uint32_t nrec = min(sc.ctl->rec_count + sc.ctl->rec_extra, sc.rec_cap);
 
   // The non-empty tiles are handed out by one counter over their list, two ahead: while a
   // tile is rasterised, the next tile's list bounds are already loading and the one after it
