@@ -62,7 +62,8 @@ struct __align__(16) RasterRec {
   float ax, ay, e1x, e1y;   // A; e1 = B - A
   float e2x, e2y, uz, d0;   // e2 = C - A; u.z; screen depth of A
   float d1, d2;             // screen depths of B, C
-  uint32_t rsv, pad;        // reserved (zero)
+  uint32_t face;            // position of the face in the mesh's face arrays (cull pass's records)
+  uint32_t pad;             // reserved (zero)
   uint32_t seq;             // (face << 4) | (fan << 1) | clipped — submission order
   uint32_t view;            // index of the view in the batch | flags << 28 (kRec*)
   uint32_t xr, yr;          // inclusive pixel range: x0 | x1 << 16, y0 | y1 << 16
@@ -102,7 +103,9 @@ struct __align__(128) DView {
   const float* px; const float* py; const float* pz;   // positions, SoA, padded to 4
   const float* nx; const float* ny; const float* nz;   // normals, SoA, padded to 4
   const float2* uv;
-  const int4* fv; const int4* fvt; const int4* fvn;    // per-face corner indices (+pad)
+  // per-face corner indices, in an order of the library's own (near faces near one another, fv into
+  // the library's order of the positions); fv.w is the face's number in the caller's array
+  const int4* fv; const int4* fvt; const int4* fvn;
   int32_t npos, nnrm, nuv, nfaces;
   int32_t unified;  // every face corner has equal v, vt and vn indices (fvt, fvn unused)
   // the mesh's positions and normals as (x, y, z, 0), gathered per corner for the world
@@ -219,6 +222,30 @@ constexpr int kStashWarpsPerSm = 32;  // raster warps resident per SM at most
 
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.
 // `from` is mapped host memory or device memory; sizes are multiples of 16.
+// The order a mesh is kept in (see k_place_positions): raw device copies of the caller's arrays in,
+// the mesh's arrays out.
+constexpr int kMeshCells = 1 << 18;
+constexpr int kOrderedFaces = 1 << 15;  // smaller meshes keep the caller's order (they fit the caches)
+struct MeshOrder {
+  const float* pos; int npos;        // [npos][3]
+  const int32_t* faces; int nfaces;  // [nfaces][3 corners][v, vt, vn]
+  uint32_t* cells;                   // scratch: kMeshCells + 8 words
+  uint32_t* codes;                   // scratch: max(npos, nfaces) words
+  uint32_t* place;                   // scratch: npos words
+  float *px, *py, *pz;
+  float4* p4;
+  uint32_t* vorder;                  // [npos] the caller's index of each position
+  int4 *fv, *fvt, *fvn;
+};
+int launch_mesh_order(const MeshOrder& o, cudaStream_t s);
+int launch_split_normals(const float* nrm, int n, float* nx, float* ny, float* nz, float4* n4, cudaStream_t s);
+// `from` is mapped host memory or device memory; sizes are multiples of 16.
+// Bounds of `n` positions, then the mesh's faces (raw: 9 indices a face, device memory) into fv, fvt, fvn
+// grouped by the cell of a 64^3 grid that holds their centroid, cells in Morton order.
+// `cells`: kFaceCells + 8 words of scratch; `codes`: one word a face.
+constexpr int kFaceCells = 1 << 18;
+int launch_face_order(const int32_t* raw, int nfaces, const float4* p4, int npos, uint32_t* cells, uint32_t* codes,
+                      int4* fv, int4* fvt, int4* fvn, cudaStream_t s);
 int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s);
 int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s);
 int launch_setup(const DView* views, int nviews, int nchunks, Scratch sc, int grid, cudaStream_t s);

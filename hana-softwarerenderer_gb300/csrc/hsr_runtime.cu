@@ -71,7 +71,7 @@ static int dalloc(void** p, size_t bytes, const char* what) {
 }
 
 MeshObj::~MeshObj() {
-  for (void* p : {(void*)px, (void*)py, (void*)pz, (void*)nx, (void*)ny, (void*)nz, (void*)p4, (void*)n4, (void*)pk,
+  for (void* p : {(void*)px, (void*)py, (void*)pz, (void*)nx, (void*)ny, (void*)nz, (void*)p4, (void*)n4, (void*)pk, (void*)vorder,
                   (void*)uv, (void*)fv, (void*)fvt, (void*)fvn})
     if (p) cudaFree(p);
 }
@@ -495,24 +495,25 @@ int Runtime::run_sequence(const hsr_draw_desc* descs, int n) {
   return fail(HSR_ERR_BIN_OVERFLOW, "draw batch: scratch overflow persisted after retries");
 }
 
-// The packed vertex of a mesh whose corners index positions, normals and uvs alike: vertex i
-// as (x, y, z, nx), (ny, nz, u, v) from the position, normal and uv arrays (zeros where an
-// array is shorter), so a corner's attributes are one 32-byte sector.
-__global__ void k_pack_vertices(float4* __restrict__ pk, const float4* __restrict__ p4, const float4* __restrict__ n4,
-                                const float2* __restrict__ uv, int npos, int nnrm, int nuv) {
+// The packed vertex of a mesh whose corners index positions, normals and uvs alike: position i
+// with the normal and uv of the caller's index vorder[i], as (x, y, z, nx), (ny, nz, u, v) (zeros
+// where an array is shorter), so a corner's attributes are one 32-byte sector.
+__global__ void k_pack_vertices(float4* __restrict__ pk, const float4* __restrict__ p4, const uint32_t* __restrict__ vorder,
+                                const float4* __restrict__ n4, const float2* __restrict__ uv, int npos, int nnrm, int nuv) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npos; i += gridDim.x * blockDim.x) {
     const float4 p = p4[i];
-    const float4 n = i < nnrm ? n4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 t = i < nuv ? uv[i] : make_float2(0.f, 0.f);
+    const int o = (int)vorder[i];
+    const float4 n = o < nnrm ? n4[o] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2 t = o < nuv ? uv[o] : make_float2(0.f, 0.f);
     pk[2 * i] = make_float4(p.x, p.y, p.z, n.x);
     pk[2 * i + 1] = make_float4(n.y, n.z, t.x, t.y);
   }
 }
 
-int launch_pack_vertices(float4* pk, const float4* p4, const float4* n4, const float2* uv, int npos, int nnrm, int nuv,
-                         cudaStream_t s) {
+int launch_pack_vertices(float4* pk, const float4* p4, const uint32_t* vorder, const float4* n4, const float2* uv,
+                         int npos, int nnrm, int nuv, cudaStream_t s) {
   if (npos <= 0) return 0;
-  k_pack_vertices<<<std::min((npos + 255) / 256, 4096), 256, 0, s>>>(pk, p4, n4, uv, npos, nnrm, nuv);
+  k_pack_vertices<<<std::min((npos + 255) / 256, 4096), 256, 0, s>>>(pk, p4, vorder, n4, uv, npos, nnrm, nuv);
   return (int)cudaGetLastError();
 }
 
@@ -608,16 +609,66 @@ int hsr_shutdown(void) {
   return HSR_OK;
 }
 
-// (x, y, z, 0) per item of an xyz array into a device array of max(n, 1) float4s.
-static int write_xyz0(const float* src, int32_t n, float4* dst) {
-  std::vector<float4> tmp((size_t)std::max(n, 1), make_float4(0.f, 0.f, 0.f, 0.f));
-  for (int32_t i = 0; i < n; i++) tmp[i] = make_float4(src[(size_t)i * 3], src[(size_t)i * 3 + 1], src[(size_t)i * 3 + 2], 0.f);
-  cudaError_t e = cudaMemcpy(dst, tmp.data(), sizeof(float4) * tmp.size(), cudaMemcpyHostToDevice);
-  return e == cudaSuccess ? HSR_OK : cuda_fail(e, "mesh upload");
+// Host array to a temporary of the stream-ordered pool, on the library's stream (pageable memory: the
+// copy has left the host array when the call returns).
+static cudaError_t stage(const void* src, size_t bytes, void* dst) {
+  return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g_rt->stream) : cudaSuccess;
 }
-static int upload_xyz0(const float* src, int32_t n, float4** dst) {
-  int rc = dalloc((void**)dst, sizeof(float4) * (size_t)std::max(n, 1), "mesh");
-  return rc == HSR_OK ? write_xyz0(src, n, *dst) : rc;
+
+// The caller's normals into the mesh's arrays (and the packed vertices, which carry them too).
+static int place_normals(MeshObj* m, const float* nrm) {
+  cudaStream_t st = g_rt->stream;
+  const size_t bytes = sizeof(float) * 3 * (size_t)m->nnrm;
+  char* tmp = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (bytes) {
+    e = cudaMallocAsync((void**)&tmp, bytes, st);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(HSR_ERR_OUT_OF_MEMORY, "mesh: device allocation for the normals failed");
+    }
+    e = stage(nrm, bytes, tmp);
+    if (e == cudaSuccess) e = (cudaError_t)launch_split_normals((const float*)tmp, m->nnrm, m->nx, m->ny, m->nz, m->n4, st);
+    cudaFreeAsync(tmp, st);
+  }
+  if (e == cudaSuccess && m->pk)
+    e = (cudaError_t)launch_pack_vertices(m->pk, m->p4, m->vorder, m->n4, m->uv, m->npos, m->nnrm, m->nuv, st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? HSR_OK : cuda_fail(e, "normal upload");
+}
+
+// The caller's positions and faces into the mesh's arrays, in the library's order.
+static int place_mesh(MeshObj* m, const float* pos, const int32_t* faces) {
+  cudaStream_t st = g_rt->stream;
+  const size_t npos = (size_t)m->npos, nfaces = (size_t)m->nfaces;
+  const size_t b_pos = align_up(sizeof(float) * 3 * npos, 256), b_faces = align_up(sizeof(int32_t) * 9 * nfaces, 256);
+  const size_t b_cells = sizeof(uint32_t) * (kMeshCells + 64), b_codes = align_up(sizeof(uint32_t) * std::max(npos, nfaces), 256);
+  char* tmp = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&tmp, b_pos + b_faces + b_cells + b_codes + sizeof(uint32_t) * npos + 256, st);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(HSR_ERR_OUT_OF_MEMORY, "mesh: device allocation for the mesh order failed");
+  }
+  MeshOrder o = {};
+  o.pos = (const float*)tmp;
+  o.npos = m->npos;
+  o.faces = (const int32_t*)(tmp + b_pos);
+  o.nfaces = m->nfaces;
+  o.cells = (uint32_t*)(tmp + b_pos + b_faces);
+  o.codes = (uint32_t*)(tmp + b_pos + b_faces + b_cells);
+  o.place = (uint32_t*)(tmp + b_pos + b_faces + b_cells + b_codes);
+  o.px = m->px; o.py = m->py; o.pz = m->pz;
+  o.p4 = m->p4;
+  o.vorder = m->vorder;
+  o.fv = m->fv; o.fvt = m->fvt; o.fvn = m->fvn;
+  e = stage(pos, sizeof(float) * 3 * npos, tmp);
+  if (e == cudaSuccess) e = stage(faces, sizeof(int32_t) * 9 * nfaces, tmp + b_pos);
+  if (e == cudaSuccess) e = (cudaError_t)launch_mesh_order(o, st);
+  cudaFreeAsync(tmp, st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? HSR_OK : cuda_fail(e, "mesh upload");
 }
 
 int hsr_mesh_upload(const float* pos, int32_t npos, const float* nrm, int32_t nnrm, const float* uv, int32_t nuv,
@@ -627,63 +678,38 @@ int hsr_mesh_upload(const float* pos, int32_t npos, const float* nrm, int32_t nn
   if (nfaces > (1 << 27)) return fail(HSR_ERR_INVALID_ARG, "mesh: more than 2^27 faces");
   if ((npos && !pos) || (nnrm && !nrm) || (nuv && !uv) || (nfaces && !faces))
     return fail(HSR_ERR_INVALID_ARG, "mesh: null array with nonzero count");
+  bool unified = true;  // every corner has equal v, vt and vn indices
   for (int64_t i = 0; i < (int64_t)nfaces * 3; i++) {
     const int32_t* c = faces + i * 3;
     if (c[0] < 0 || c[0] >= npos || c[1] < 0 || c[1] >= nuv || c[2] < 0 || c[2] >= nnrm)
       return fail(HSR_ERR_INVALID_ARG, "mesh: face index out of range (face " + std::to_string(i / 3) + ")");
+    unified = unified && c[0] == c[1] && c[0] == c[2];
   }
   MeshObj* m = new MeshObj();
   m->npos = npos; m->nnrm = nnrm; m->nuv = nuv; m->nfaces = nfaces;
-  const size_t P = align_up((size_t)std::max(npos, 1), 4), N = align_up((size_t)std::max(nnrm, 1), 4);
-  std::vector<float> tmp(std::max(P, N), 0.f);
+  m->unified = unified;
+  // zeroed: the SoA arrays are padded to a multiple of 4, an empty array holds one item
   int rc = HSR_OK;
-  auto up_soa = [&](const float* src, int cnt, int comp, size_t padded, float** dst) -> int {
-    int r = dalloc((void**)dst, sizeof(float) * padded, "mesh");
-    if (r != HSR_OK) return r;
-    std::fill(tmp.begin(), tmp.begin() + padded, 0.f);
-    for (int i = 0; i < cnt; i++) tmp[i] = src[(size_t)i * 3 + comp];
-    cudaError_t e = cudaMemcpy(*dst, tmp.data(), sizeof(float) * padded, cudaMemcpyHostToDevice);
-    return e == cudaSuccess ? HSR_OK : cuda_fail(e, "mesh upload");
+  auto make = [&](void** p, size_t bytes, const char* what) {
+    if (rc == HSR_OK) rc = dalloc(p, bytes, what);
+    if (rc == HSR_OK && cudaMemsetAsync(*p, 0, bytes, g_rt->stream) != cudaSuccess)
+      rc = cuda_fail(cudaGetLastError(), "mesh upload");
   };
-  for (int c = 0; c < 3 && rc == HSR_OK; c++) rc = up_soa(pos, npos, c, P, c == 0 ? &m->px : (c == 1 ? &m->py : &m->pz));
-  for (int c = 0; c < 3 && rc == HSR_OK; c++) rc = up_soa(nrm, nnrm, c, N, c == 0 ? &m->nx : (c == 1 ? &m->ny : &m->nz));
-  if (rc == HSR_OK) rc = upload_xyz0(pos, npos, &m->p4);
-  if (rc == HSR_OK) rc = upload_xyz0(nrm, nnrm, &m->n4);
-  if (rc == HSR_OK) rc = dalloc((void**)&m->uv, sizeof(float2) * (size_t)std::max(nuv, 1), "mesh uv");
+  const size_t np = (size_t)std::max(npos, 1), nn = (size_t)std::max(nnrm, 1), F = (size_t)std::max(nfaces, 1);
+  for (float** p : {&m->px, &m->py, &m->pz}) make((void**)p, sizeof(float) * align_up(np, 4), "mesh positions");
+  for (float** p : {&m->nx, &m->ny, &m->nz}) make((void**)p, sizeof(float) * align_up(nn, 4), "mesh normals");
+  make((void**)&m->p4, sizeof(float4) * np, "mesh positions");
+  make((void**)&m->n4, sizeof(float4) * nn, "mesh normals");
+  make((void**)&m->vorder, sizeof(uint32_t) * np, "mesh order");
+  make((void**)&m->uv, sizeof(float2) * (size_t)std::max(nuv, 1), "mesh uv");
+  for (int4** p : {&m->fv, &m->fvt, &m->fvn}) make((void**)p, sizeof(int4) * F, "mesh faces");
   if (rc == HSR_OK && nuv) {
-    cudaError_t e = cudaMemcpy(m->uv, uv, sizeof(float2) * (size_t)nuv, cudaMemcpyHostToDevice);
+    const cudaError_t e = stage(uv, sizeof(float2) * (size_t)nuv, m->uv);
     if (e != cudaSuccess) rc = cuda_fail(e, "mesh uv upload");
   }
-  if (rc == HSR_OK) {
-    const size_t F = (size_t)std::max(nfaces, 1);
-    std::vector<int4> fv(F), ft(F), fn(F);
-    bool unified = true;
-    for (int i = 0; i < nfaces; i++) {
-      const int32_t* f = faces + (size_t)i * 9;
-      fv[i] = make_int4(f[0], f[3], f[6], 0);
-      ft[i] = make_int4(f[1], f[4], f[7], 0);
-      fn[i] = make_int4(f[2], f[5], f[8], 0);
-      for (int k = 0; k < 9; k += 3) unified = unified && f[k] == f[k + 1] && f[k] == f[k + 2];
-    }
-    m->unified = unified;
-    if (unified && npos > 0 && rc == HSR_OK) {
-      rc = dalloc((void**)&m->pk, sizeof(float4) * 2 * (size_t)npos, "packed vertices");
-      if (rc == HSR_OK) {
-        int kr = launch_pack_vertices(m->pk, m->p4, m->n4, m->uv, npos, nnrm, nuv, g_rt->stream);
-        cudaError_t e = kr ? (cudaError_t)kr : cudaStreamSynchronize(g_rt->stream);
-        if (e != cudaSuccess) rc = cuda_fail(e, "pack vertices");
-      }
-    }
-    int4** dsts[3] = {&m->fv, &m->fvt, &m->fvn};
-    std::vector<int4>* srcs[3] = {&fv, &ft, &fn};
-    for (int k = 0; k < 3 && rc == HSR_OK; k++) {
-      rc = dalloc((void**)dsts[k], sizeof(int4) * F, "mesh faces");
-      if (rc == HSR_OK) {
-        cudaError_t e = cudaMemcpy(*dsts[k], srcs[k]->data(), sizeof(int4) * F, cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) rc = cuda_fail(e, "mesh faces upload");
-      }
-    }
-  }
+  if (rc == HSR_OK) rc = place_mesh(m, pos, faces);
+  if (rc == HSR_OK && unified && npos > 0) rc = dalloc((void**)&m->pk, sizeof(float4) * 2 * np, "packed vertices");
+  if (rc == HSR_OK) rc = place_normals(m, nrm);
   if (rc != HSR_OK) { delete m; return rc; }
   const uint64_t h = g_rt->next_handle++;
   g_rt->meshes[h] = m;
@@ -696,22 +722,7 @@ int hsr_mesh_update_normals(hsr_mesh mh, const float* nrm, int32_t nnrm) {
   MeshObj* m = g_rt->mesh(mh);
   if (!m) return fail(HSR_ERR_BAD_HANDLE, "mesh_update_normals: unknown mesh");
   if (nnrm != m->nnrm || (nnrm && !nrm)) return fail(HSR_ERR_INVALID_ARG, "mesh_update_normals: count mismatch");
-  cudaStreamSynchronize(g_rt->stream);
-  const size_t N = align_up((size_t)std::max(nnrm, 1), 4);
-  std::vector<float> tmp(N, 0.f);
-  float* dst[3] = {m->nx, m->ny, m->nz};
-  for (int c = 0; c < 3; c++) {
-    for (int i = 0; i < nnrm; i++) tmp[i] = nrm[(size_t)i * 3 + c];
-    cudaError_t e = cudaMemcpy(dst[c], tmp.data(), sizeof(float) * N, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return cuda_fail(e, "normal upload");
-  }
-  int rc = write_xyz0(nrm, nnrm, m->n4);
-  if (rc == HSR_OK && m->pk) {  // the packed vertices carry the normals too
-    int kr = launch_pack_vertices(m->pk, m->p4, m->n4, m->uv, m->npos, m->nnrm, m->nuv, g_rt->stream);
-    cudaError_t e = kr ? (cudaError_t)kr : cudaStreamSynchronize(g_rt->stream);
-    if (e != cudaSuccess) rc = cuda_fail(e, "pack vertices");
-  }
-  return rc;
+  return place_normals(m, nrm);
 }
 
 int hsr_mesh_release(hsr_mesh mh) {
