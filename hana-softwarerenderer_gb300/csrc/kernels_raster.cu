@@ -305,6 +305,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     sm.shaded[warp] = sm.frags[warp] = 0ull;
     sm.done[warp] = 0u;
   }
+  uint32_t ri_ahead = !SHARED && (uint32_t)lane < n ? sc.bins[off + (uint32_t)lane] : kNone;
   int ready = -1;  // the shadow map's view last seen complete
   for (;;) {
     if (t >= ntiles) break;
@@ -313,10 +314,6 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
       const uint32_t li_next = __shfl_sync(kFull, li_ahead, 0);
       if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(claim, 1u) : nlist;
       if (li_next < nlist) t_next = tile_list[li_next];
-      if (t_next < ntiles) {
-        n_next = sc.tile_count[t_next];
-        off_next = sc.tile_off[t_next];
-      }
     }
     const DView& v = views[vi];
     const int lt = (int)t - v.tile_base;
@@ -338,14 +335,17 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         st.rec[lane + 32 * q] = kNone;
       }
     }
+    const uint32_t share = b;
     uint32_t frags = 0;  // covered candidates (warp-uniform)
     for (; b < end; b += 32) {
       const uint32_t cnt = min(32u, end - b);
-      uint32_t c = 0, w = 1, ri = kNone;
+      uint32_t c = 0, w = 1, ri = ri_ahead;
       int p0 = 0;  // the first pixel of the record's range in the tile
       RasterRec rr;
       if ((uint32_t)lane < cnt) {
-        ri = sc.bins[off + b + (uint32_t)lane];
+        // the tile's first indices came with the tile before, later ones of a 16x16 or 32x32 tile (many
+        // batches) during the batch before
+        if (SHARED ? (kKeep || b == share) : (kKeep && b > 0u)) ri = sc.bins[off + b + (uint32_t)lane];
         if (ri < nrec) {  // an index past the records never comes from a consistent bin pass
           rr = sc.recs[ri];
           const int lx0 = max((int)(rr.xr & 0xffffu) - ox, 0), lx1 = min((int)(rr.xr >> 16) - ox, T - 1);
@@ -398,6 +398,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         if (rest > 0u) atomicOr(&br.first[start >> 5], 1u << (start & 31u));
       }
       __syncwarp();
+      if (!kKeep && b + 32u + (uint32_t)lane < end) ri_ahead = sc.bins[off + b + 32u + (uint32_t)lane];
       // Visibility of `cnt` queued candidates from the ring head, one per lane: weights
       // (the divisions of barycentric()), depth, and a 64-bit atomicMin of the key.
       uint32_t qh = 0, qn = 0;  // ring head and queued count (warp-uniform)
@@ -470,6 +471,11 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         before += __popc(here);
       }
       if (qn) resolve(qn);  // before the next batch replaces the runs the queue points to
+    }
+    // the next tile's list bounds: its number, asked for before this tile's records, has come by now
+    if (!SHARED && t_next < ntiles) {
+      n_next = sc.tile_count[t_next];
+      off_next = sc.tile_off[t_next];
     }
     if (lane == 0) {
       if (v.dep0 >= 0 && v.dep0 != ready) wait_target(sc, views, v.dep0);
@@ -567,6 +573,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
       }
       vi_next = view_of(t_next);
     }
+    if (!SHARED) ri_ahead = (uint32_t)lane < n_next ? sc.bins[off_next + (uint32_t)lane] : kNone;
     t = t_next;
     n = n_next;
     off = off_next;
