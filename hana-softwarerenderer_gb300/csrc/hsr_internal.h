@@ -248,7 +248,8 @@ int launch_face_order(const int32_t* raw, int nfaces, const float4* p4, int npos
                       int4* fv, int4* fvt, int4* fvn, cudaStream_t s);
 int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s);
 int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s);
-int launch_setup(const DView* views, int nviews, int nchunks, Scratch sc, int grid, cudaStream_t s);
+bool culls_own_vertices(size_t faces);  // the cull pass needs no launch_vertex
+int launch_setup(const DView* views, int nviews, int nchunks, bool own_vertices, Scratch sc, int grid, cudaStream_t s);
 bool clips_with_emit(size_t faces);  // the emit pass's grid also clips (no launch_post)
 int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms, cudaStream_t s);
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);

@@ -175,8 +175,9 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   if (e != cudaSuccess) return cuda_fail(e, "draw_noalloc: upload");
   e = cudaMemsetAsync(dev + o_zero, 0, zero_bytes, s);  // counters start at zero every call
   if (e != cudaSuccess) return cuda_fail(e, "draw_noalloc: clear counters");
-  int kr = launch_vertex(dview, 1, nvch, rt->num_sms * 8, s);
-  if (!kr) kr = launch_setup(dview, 1, nsch, sc, rt->num_sms * 8, s);
+  const bool own = culls_own_vertices(faces);
+  int kr = own ? 0 : launch_vertex(dview, 1, nvch, rt->num_sms * 8, s);
+  if (!kr) kr = launch_setup(dview, 1, nsch, own, sc, rt->num_sms * 8, s);
   if (!kr) kr = launch_emit(dview, T, sc, clips_with_emit(faces), rt->num_sms, s);
   if (!kr && !clips_with_emit(faces)) kr = launch_post(dview, T, sc, rt->num_sms * 4, s);
   if (!kr) kr = launch_big(dview, T, sc, rt->num_sms * 2, s);
@@ -184,7 +185,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   if (!kr) kr = launch_scatter(dview, T, sc, rt->num_sms * 8, ncch, s);
   if (!kr) kr = launch_raster(dview, T, sc, rt->num_sms * rt->tuning.ctas_per_sm, rt->tuning.warps_per_cta, s);
   if (kr) return cuda_fail((cudaError_t)kr, "draw_noalloc: kernel launch");
-  rt->launches += clips_with_emit(faces) ? 7 : 8;
+  rt->launches += (own ? 6 : 7) + (clips_with_emit(faces) ? 0 : 1);
   Ctl* hc = reinterpret_cast<Ctl*>(h + host_bytes);
   e = cudaMemcpyAsync(hc, sc.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
