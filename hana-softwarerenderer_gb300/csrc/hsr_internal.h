@@ -255,7 +255,8 @@ int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
 int launch_big(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
 int launch_scan(Scratch sc, cudaStream_t s);
-int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int clear_chunks, cudaStream_t s);
+int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int clear_chunks, uint32_t plane_bytes,
+                   cudaStream_t s);
 int launch_raster(const DView* views, int tile, Scratch sc, int grid, int warps, cudaStream_t s);
 int scan_blocks(int ntiles);
 

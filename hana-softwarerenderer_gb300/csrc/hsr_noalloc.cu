@@ -182,7 +182,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   if (!kr && !clips_with_emit(faces)) kr = launch_post(dview, T, sc, rt->num_sms * 4, s);
   if (!kr) kr = launch_big(dview, T, sc, rt->num_sms * 2, s);
   if (!kr) kr = launch_scan(sc, s);
-  if (!kr) kr = launch_scatter(dview, T, sc, rt->num_sms * 8, ncch, s);
+  if (!kr) kr = launch_scatter(dview, T, sc, rt->num_sms * 8, ncch, 12u, s);
   if (!kr) kr = launch_raster(dview, T, sc, rt->num_sms * rt->tuning.ctas_per_sm, rt->tuning.warps_per_cta, s);
   if (kr) return cuda_fail((cudaError_t)kr, "draw_noalloc: kernel launch");
   rt->launches += (own ? 6 : 7) + (clips_with_emit(faces) ? 0 : 1);

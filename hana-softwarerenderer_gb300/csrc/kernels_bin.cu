@@ -323,34 +323,43 @@ __device__ __forceinline__ void clear_empty_tiles(const DView* __restrict__ view
   }
 }
 
-// Scatter and clear in one grid: every kClearEvery-th block clears (when the batch has clear
-// chunks), the others scatter, so the store-bound clear runs beside the atomic-bound scatter
-// instead of after it.
-constexpr int kClearEvery = 2;
+// Scatter and clear in one grid (when the batch has clear chunks): some blocks clear, the others
+// scatter, so the store-bound clear runs beside the atomic-bound scatter instead of after it.  Of
+// every two blocks one clears; where the pixels to clear outweigh the
+// (record, tile) pairs, two of three do (16 views, 15 pixels a pair: 92 -> 76 us; at 6 a pair, 64
+// requests, that is 299 -> 354).
+constexpr int kClearMinBlocks = 3;
+constexpr unsigned long long kClearHeavy = 10;  // pixels of three planes per pair
 
-__global__ void __launch_bounds__(256) k_scatter(const DView* __restrict__ views, int T, Scratch sc, int nchunks) {
+__global__ void __launch_bounds__(256) k_scatter(const DView* __restrict__ views, int T, Scratch sc, int nchunks,
+                                                 uint32_t plane_bytes) {
   __shared__ int32_t s_cbase[kSharedViews];
   const uint32_t b = blockIdx.x, g = gridDim.x;
   chain_wait();
-  if (sc.ctl->ne_tiles >= (uint32_t)sc.ntiles) nchunks = 0;  // every tile is the raster's: all blocks scatter
-  if (nchunks > 0 && b % kClearEvery == kClearEvery - 1) {  // block-uniform
+  const uint32_t ne = sc.ctl->ne_tiles, nt = (uint32_t)sc.ntiles;
+  if (ne >= nt) nchunks = 0;  // every tile is the raster's: all blocks scatter
+  const unsigned long long px = (unsigned long long)(nt - min(ne, nt)) * (unsigned)(T * T) * plane_bytes / 12u;
+  const uint32_t every = px >= kClearHeavy * sc.ctl->bin_total ? 3u : 2u;  // 3: two clear and one scatters
+  const uint32_t first = b / every * (every - 1u);                         // clearing blocks before this group
+  if (nchunks > 0 && b % every != 0u) {  // block-uniform
     const bool in_shared = sc.nviews <= kSharedViews;
     if (in_shared)
       for (int i = threadIdx.x; i < sc.nviews; i += blockDim.x) s_cbase[i] = views[i].cch_base;
     __syncthreads();
-    clear_empty_tiles(views, T, nchunks, sc, (int)(b / kClearEvery), (int)(g / kClearEvery), in_shared ? s_cbase : nullptr);
+    clear_empty_tiles(views, T, nchunks, sc, (int)(first + b % every - 1u), (int)(g - (g + every - 1u) / every),
+                      in_shared ? s_cbase : nullptr);
   } else if (nchunks > 0) {
-    scatter_records(views, T, sc, b - b / kClearEvery, g - g / kClearEvery);
+    scatter_records(views, T, sc, b / every, (g + every - 1u) / every);
   } else {
     scatter_records(views, T, sc, b, g);
   }
 }
 
-// `grid` blocks of 256 threads (at least kClearEvery when the batch clears, so both parts
-// have blocks).
-int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int nchunks, cudaStream_t s) {
-  if (nchunks > 0 && grid < kClearEvery) grid = kClearEvery;
-  return launch_chained(k_scatter, grid > 0 ? grid : 1, 256, 0, s, views, tile, sc, nchunks);
+// `grid` blocks of 256 threads (at least kClearMinBlocks when the batch clears, so both parts have
+// blocks); `plane_bytes`: bytes cleared per pixel on average.
+int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int nchunks, uint32_t plane_bytes, cudaStream_t s) {
+  if (nchunks > 0 && grid < kClearMinBlocks) grid = kClearMinBlocks;
+  return launch_chained(k_scatter, grid > 0 ? grid : 1, 256, 0, s, views, tile, sc, nchunks, plane_bytes);
 }
 
 }  // namespace hsr
