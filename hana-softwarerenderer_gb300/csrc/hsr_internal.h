@@ -162,7 +162,7 @@ struct Ctl {
   unsigned long long shaded_px;  // pixels whose winner was shaded by the raster
   unsigned long long frag_px;    // covered (pixel, triangle) pairs the raster depth-tested
   uint32_t ne_tiles;             // tiles with at least one record (k_scan)
-  uint32_t ctl_pad;
+  float box_px;                  // pixels of the cull pass's records' bounding boxes (k_emit)
   unsigned long long pay_bytes;  // shading payload bytes written (k_emit, k_post, k_big)
 };
 static_assert(sizeof(Ctl) == 64, "Ctl is read back whole: keep it one 64-byte block");

@@ -882,6 +882,7 @@ __device__ __forceinline__ void emit_records(const DView* __restrict__ views, in
   const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
   const uint32_t stride = nblocks * blockDim.x;
   uint32_t pay_bytes = 0;  // payload bytes this lane wrote for the raster (big ones: k_big)
+  float box_px = 0.f;      // pixels of its records' bounding boxes
   for (uint32_t i0 = block * blockDim.x + (threadIdx.x & ~31u); i0 < nrec; i0 += stride) {
     const uint32_t i = i0 + (uint32_t)lane;
     bool valid = false;
@@ -904,7 +905,10 @@ __device__ __forceinline__ void emit_records(const DView* __restrict__ views, in
       }
     }
     int tx0, ty0, ntw, nt = 0;
-    if (valid) rec_tiles(r, T, tx0, ty0, ntw, nt);
+    if (valid) {
+      rec_tiles(r, T, tx0, ty0, ntw, nt);
+      box_px += (float)(((r.xr >> 16) - (r.xr & 0xffffu) + 1u) * ((r.yr >> 16) - (r.yr & 0xffffu) + 1u));
+    }
     const bool big = valid && nt > kMaxRecordTiles;
     const bool small = valid && !big;
     if (small) {
@@ -923,8 +927,28 @@ __device__ __forceinline__ void emit_records(const DView* __restrict__ views, in
       }
     }
   }
+  // one atomic of each a block on the control block's line, which serves them one by one (a warp
+  // each: 26 -> 32 us in a 1920x1080 frame of 120k faces; now 24.6)
+  __shared__ uint32_t s_pay[kEmitThreads / 32];
+  __shared__ float s_box[kEmitThreads / 32];
   pay_bytes = __reduce_add_sync(kFull, pay_bytes);
-  if (lane == 0 && pay_bytes) atomicAdd(&sc.ctl->pay_bytes, (unsigned long long)pay_bytes);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) box_px += __shfl_down_sync(kFull, box_px, o);
+  if (lane == 0) {
+    s_pay[threadIdx.x >> 5] = pay_bytes;
+    s_box[threadIdx.x >> 5] = box_px;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long pay = 0;
+    float box = 0.f;
+    for (int w = 0; w < kEmitThreads / 32; w++) {
+      pay += s_pay[w];
+      box += s_box[w];
+    }
+    if (pay) atomicAdd(&sc.ctl->pay_bytes, pay);
+    if (box > 0.f) atomicAdd(&sc.ctl->box_px, box);
+  }
 }
 
 // The clip queue of k_setup, two faces per warp: warp w of the grid begins with pair w, and where

@@ -118,6 +118,25 @@ struct __align__(16) BatchRecs {
   uint32_t first[32];  // a bit per remainder candidate: set where a record's candidates begin
 };
 
+// Ordered bits of a depth no fragment of the record lies below (0: unknown).  interpolate_depth
+// (graphics.cpp:186-194) sums d_k b_k with weights that a covered pixel has >= 0 and that add up to
+// 1 within 4 units of 2^-24 (b0 = 1 - s / uz, b1 + b2 = s / uz, each operation rounded once), itself
+// with five roundings; so for depths >= 2^-100, where what the products lose by underflow does not
+// count, no sum is below (1 - 2^-20) times the smallest.  The literal divisions (kRecExact) may
+// underflow, and NaN compares false: no bound.
+__device__ __forceinline__ uint32_t lowest_depth(const RasterRec& r) {
+  const bool known = r.d0 >= 0x1p-100f && r.d1 >= 0x1p-100f && r.d2 >= 0x1p-100f &&
+                     !((r.view >> kRecFlagShift) & kRecExact);
+  return known ? ord_bits(fm(fminf(fminf(r.d0, r.d1), r.d2), 0x1.ffffep-1f)) : 0u;
+}
+// Candidates per pixel of the visited tiles (the records' bounding boxes, added up by the emit pass)
+// from which covered candidates are tested against lowest_depth before they are queued (HIDE): a
+// shared load and a compare a candidate, which save the divisions and the atomic of the hidden
+// ones.  The 4M-triangle soup has 26 a pixel (raster 784 -> 666 us); meshes have about 3, where
+// nearly every covered candidate wins when it is tested and the test costs 2-3 % (64 requests
+// 1,730 -> 1,786 us).
+constexpr float kHideCandidates = 10.f;
+
 // Pixel of candidate i: q = i - m.x counts a record's range in row-major order, width w;
 // m.y = ceil(65536 / w) divides by w (q < 1024, w <= 32), m.z = (first pixel) - m.x, m.w = T - w.
 __device__ __forceinline__ int pixel_of(int4 m, int i) {
@@ -155,8 +174,8 @@ struct RasterSmem {
   CandQueue cq[WARPS];
   float u8f[256];
   int32_t tbase[kSharedViews];
-  // pixels shaded and candidates covered in each warp's tiles, added to the control block once: its
-  // counters share a line with the claim, and atomics on one line are served one by one (two a
+  // pixels shaded and candidates covered in each warp's tiles, added to the control block once a CTA:
+  // its counters share a line with the claim, and atomics on one line are served one by one (two a
   // tile besides the claim made the claim a quarter of the time with 8x8 tiles: 2560x1440
   // close-up 127 -> 108 us, 1280x720 grid 106 -> 86 us)
   unsigned long long shaded[WARPS], frags[WARPS];
@@ -254,7 +273,8 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 // SHARED: a whole CTA takes one tile.  Each warp rasterises an equal share of the tile's list
 // into a tile state of its own, the states are merged by the smaller key (the order of the list
 // never matters), and the pixel rows are shaded by the warps in turn.
-template <int T, int WARPS, bool SHARED>
+// HIDE: see kHideCandidates.
+template <int T, int WARPS, bool SHARED, bool HIDE>
 __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, const Scratch& sc,
                                              RasterSmem<T, WARPS>& sm, const int32_t* tbase, uint32_t nlist,
                                              const uint32_t* tile_list, uint32_t* claim) {
@@ -301,10 +321,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   }
   // views of a warp's tiles only move forward: after the first, search on from the last one
   int vi = t < ntiles ? find_view(views, tbase, sc.nviews, (int)t) : 0;
-  if (lane == 0) {
-    sm.shaded[warp] = sm.frags[warp] = 0ull;
-    sm.done[warp] = 0u;
-  }
+  if (lane == 0) sm.done[warp] = 0u;
   uint32_t ri_ahead = !SHARED && (uint32_t)lane < n ? sc.bins[off + (uint32_t)lane] : kNone;
   int ready = -1;  // the shadow map's view last seen complete
   for (;;) {
@@ -392,7 +409,8 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         br.b4[k] = make_float4(flip(rr.e2x), flip(rr.e2y),
                                ((rr.view >> kRecFlagShift) & kRecExact) ? __int_as_float(0x7fffffff) : uz, uz);
         const int base = (int)start - (int)whole;  // candidate number of the record's first pixel
-        br.m4[k] = make_int4(base, magic, p0 - base, T - (int)w);
+        br.m4[k] = HIDE ? make_int4(base, magic | ((T - (int)w) << 20), p0 - base, (int)lowest_depth(rr))
+                        : make_int4(base, magic, p0 - base, T - (int)w);
         br.d4[k] = make_float4(rr.d0, rr.d1, rr.d2, __uint_as_float(rr.seq));
         br.ri[k] = ri;
         if (rest > 0u) atomicOr(&br.first[start >> 5], 1u << (start & 31u));
@@ -439,19 +457,29 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
       // One window: candidate i of record j, counted when `in`.
       auto window = [&](int i, int j, bool in) {
         const float4 a4 = br.a4[j], b4 = br.b4[j];
-        const int p = pixel_of(br.m4[j], i);
+        int4 m4 = br.m4[j];
+        const uint32_t lowest = (uint32_t)m4.w;
+        if (HIDE) {  // as laid out above
+          m4.w = m4.y >> 20;
+          m4.y &= 0xfffff;
+        }
+        const int p = pixel_of(m4, i);
         const float x = (float)(ox | (p & (T - 1))), y = (float)(oy + p / T);
         float ux, uy;
         bool covered = cover_terms_pos(a4.x, a4.y, a4.z, a4.w, b4.x, b4.y, b4.z, x, y, ux, uy) && in;
         if (exact && in && b4.z != b4.z) covered = cover_exact(ux, uy, b4.w);
-        const unsigned cm = __ballot_sync(kFull, covered);
+        unsigned cm = __ballot_sync(kFull, covered);
+        frags += (uint32_t)__popc(cm);
+        if (HIDE) {  // leave out what cannot win any more
+          covered = covered && lowest <= (uint32_t)(st.key[p] >> 32);
+          cm = __ballot_sync(kFull, covered);
+        }
         if (covered) {  // queue behind the pending ones (at most 31 are pending here)
           const uint32_t e = (qh + qn + (uint32_t)__popc(cm & (upto >> 1))) & 63u;
           cq.u[e] = make_float2(ux, uy);
           cq.jp[e] = (uint16_t)(j | (p << 5));
         }
         qn += (uint32_t)__popc(cm);
-        frags += (uint32_t)__popc(cm);
         if (qn >= 32u) resolve(32u);
       };
       // whole windows: every lane works on the same record
@@ -579,9 +607,16 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     off = off_next;
     vi = vi_next;
   }
-  if (lane == 0) {
-    if (sm.shaded[warp]) atomicAdd(&sc.ctl->shaded_px, sm.shaded[warp]);
-    if (sm.frags[warp]) atomicAdd(&sc.ctl->frag_px, sm.frags[warp]);
+}
+
+// The list's tiles by warps, the last `shared` of them by CTAs.
+template <int T, int WARPS, bool HIDE>
+__device__ __forceinline__ void raster_list(const DView* __restrict__ views, const Scratch& sc, RasterSmem<T, WARPS>& sm,
+                                            const int32_t* tbase, uint32_t nlist, uint32_t shared, const uint32_t* list) {
+  if (shared < nlist) raster_tiles<T, WARPS, false, HIDE>(views, sc, sm, tbase, nlist - shared, list, sc.claim);
+  if (shared > 0u) {
+    __syncthreads();
+    raster_tiles<T, WARPS, true, HIDE>(views, sc, sm, tbase, shared, list + (nlist - shared), sc.claim + 1);
   }
 }
 
@@ -606,6 +641,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
   extern __shared__ __align__(16) unsigned char raster_smem[];
   RasterSmem<T, WARPS>& sm = *reinterpret_cast<RasterSmem<T, WARPS>*>(raster_smem);
   build_byte_tables(sm.u8f);
+  if (threadIdx.x < WARPS) sm.shaded[threadIdx.x] = sm.frags[threadIdx.x] = 0ull;
   chain_wait();
   const int32_t* tbase = sc.nviews <= kSharedViews ? sm.tbase : nullptr;
   if (tbase)
@@ -621,16 +657,22 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
     // the tiles at the list's end that CTAs share
     const bool long_lists = (unsigned long long)sc.ctl->bin_total >= kTailRecords * (unsigned long long)sc.ctl->ne_tiles;
     const uint32_t shared = !stashes ? 0u : nlist <= kSharedTilesPerCta * gridDim.x ? nlist : long_lists ? gridDim.x : 0u;
-    if (shared < nlist) raster_tiles<T, WARPS, false>(views, sc, sm, tbase, nlist - shared, list, sc.claim);
-    if (shared > 0u) {
-      __syncthreads();
-      raster_tiles<T, WARPS, true>(views, sc, sm, tbase, shared, list + (nlist - shared), sc.claim + 1);
-    }
+    if (sc.ctl->box_px < kHideCandidates * (float)(T * T) * (float)sc.ctl->ne_tiles)
+      raster_list<T, WARPS, false>(views, sc, sm, tbase, nlist, shared, list);
+    else
+      raster_list<T, WARPS, true>(views, sc, sm, tbase, nlist, shared, list);
   }
-  // the sequence's last CTA hands the control block to the host
-  if (sc.ctl_out) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long shaded = 0, frags = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) {
+      shaded += sm.shaded[w];
+      frags += sm.frags[w];
+    }
+    if (shaded) atomicAdd(&sc.ctl->shaded_px, shaded);
+    if (frags) atomicAdd(&sc.ctl->frag_px, frags);
+    if (sc.ctl_out) {  // the sequence's last CTA hands the control block to the host
       __threadfence();
       if (atomicAdd(sc.finished, 1u) == gridDim.x - 1u) {
         __threadfence();

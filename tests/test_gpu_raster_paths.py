@@ -122,3 +122,46 @@ def test_ranges_of_every_width_and_exact_records_vs_oracle(tuned, edge, tile):
     rb = oracle.render_frame(fr)["main"]
     assert (rb.prim > 0).any()
     _check(got["main"], rb, f"{fr.name} tile{tile}")
+
+
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("edge", [4, 12, 60])
+def test_hidden_candidates_of_overdrawn_tiles_vs_oracle(tuned, edge, tile):
+    """Draws of few and of many candidates per pixel (the second kind leaves out what lies behind the
+    buffer): steep triangles, equal depths and neighbours one unit apart, depths of zero and next to it,
+    and a second draw over the first one's depth."""
+    import hsr
+
+    tuned.set_tuning(tile=tile, warps_per_cta=4, ctas_per_sm=8)
+    w, h, n = 75, 58, 500
+    rng = np.random.default_rng(edge + tile)
+    main = hsr.Target(w, h)
+    rb = oracle.Buffers(w, h, (0, 0, 0, 255), 1.0)
+    held = [main]
+    try:
+        for k in range(2):
+            p = np.clip(rng.uniform(0, (w, h), (n, 1, 2)) + rng.uniform(-edge / 2, edge / 2, (n, 3, 2)), 0.01, (w - 0.01, h - 0.01))
+            z = rng.uniform(-0.9, 0.95, (n, 3)).astype(np.float32)  # steep
+            flat = np.float32(0.25) + np.spacing(np.float32(0.25)) * rng.integers(-2, 3, (n, 1)).astype(np.float32)
+            z[n // 2:] = flat[n // 2:]
+            tiny = np.array([-1, -1 + 2.0**-24, -1 + 2.0**-20, -0.999, -0.5], np.float32)
+            z[::29] = tiny[rng.integers(0, 5, (len(z[::29]), 3))]
+            pos = np.zeros((n, 3, 3), np.float32)
+            pos[:, :, 0] = p[:, :, 0] / w * 2 - 1
+            pos[:, :, 1] = p[:, :, 1] / h * 2 - 1
+            pos[:, :, 2] = z
+            faces = np.zeros((n, 3, 3), np.int32)
+            faces[:, :, 0] = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+            mesh = scenes.Mesh(pos.reshape(-1, 3), np.array([[0, 0, 1]], np.float32), np.zeros((1, 2), np.float32), faces)
+            sd = U.shader_data((0, 0, 1), w, h, identity_mvp=True)
+            gm = hsr.Mesh(mesh)
+            held.append(gm)
+            hsr.draw_batch([hsr.make_desc(gm, scenes.FLAT, sd, main, clear=((0, 0, 0, 255), 1.0) if k == 0 else None,
+                                          prim_base=1000 * k)])
+            oracle.draw(mesh, scenes.FLAT, sd, rb, prim_base=1000 * k)
+        got = main.download()
+    finally:
+        for o in held:
+            o.release()
+    assert (rb.prim > 1000).any() and (rb.depth < 1.0).any()
+    _check(got, rb, f"hidden edge{edge} tile{tile}")
