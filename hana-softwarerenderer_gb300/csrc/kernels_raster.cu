@@ -192,6 +192,13 @@ struct RasterSmem {
 //
 // The warp shades the rows of 32 pixels q0, q0 + qstep, ...; `by_warp` (a tile shared by a CTA) gives
 // the warp whose stash holds each winner's weights, relative to the one `stash` belongs to.
+
+// The first and the last sector of the payload floats a shader reads, into L1.
+template <int NF4>
+__device__ __forceinline__ void prefetch_payload(const Payload* p) {
+  if constexpr (NF4 > 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+  if constexpr (NF4 > 2) asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(p) + 16 * (NF4 - 1)));
+}
 template <int T, int S>
 __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc, const TileState<T * T>& st, int ox,
                                                int oy, bool clear, const ByteTables& bt, const float* stash, int q0,
@@ -202,6 +209,12 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
   uint32_t shaded = 0;
 #pragma unroll 1
   for (int q = q0; q < PPL; q += qstep) {
+    // the next row's payloads start on their way to L1 while this row is shaded (a whole tile's at
+    // once push each other out: 64 requests at tile 16 raster 1,745 -> 1,716 us, and 1,760 then)
+    if (NF4 > 0 && q + qstep < PPL) {
+      const uint32_t rn = st.rec[lane + 32 * (q + qstep)];
+      if (rn != kNone) prefetch_payload<NF4>(&sc.pay[rn]);
+    }
     const int p = lane + 32 * q;
     const int x = ox + p % T, y = oy + p / T;
     if (x >= v.W || y >= v.H) continue;
