@@ -160,8 +160,9 @@ struct CandQueue {
 template <int NPIX>
 struct TileState {
   static constexpr bool kKeep = NPIX <= 64;
-  unsigned long long key[NPIX];
-  uint32_t rec[NPIX];
+  uint32_t z[NPIX];  // the key's upper half
+  uint2 win[NPIX];   // its lower half, the record (one store a winner)
+  __device__ __forceinline__ unsigned long long key(int p) const { return ((unsigned long long)z[p] << 32) | win[p].x; }
   float b0[kKeep ? NPIX : 1], b1[kKeep ? NPIX : 1], b2[kKeep ? NPIX : 1];
 };
 
@@ -212,16 +213,16 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
     // the next row's payloads start on their way to L1 while this row is shaded (a whole tile's at
     // once push each other out: 64 requests at tile 16 raster 1,745 -> 1,716 us, and 1,760 then)
     if (NF4 > 0 && q + qstep < PPL) {
-      const uint32_t rn = st.rec[lane + 32 * (q + qstep)];
+      const uint32_t rn = st.win[lane + 32 * (q + qstep)].y;
       if (rn != kNone) prefetch_payload<NF4>(&sc.pay[rn]);
     }
     const int p = lane + 32 * q;
     const int x = ox + p % T, y = oy + p / T;
     if (x >= v.W || y >= v.H) continue;
     const size_t idx = (size_t)y * v.W + x;
-    uint32_t ri = st.rec[p];
+    uint32_t ri = st.win[p].y;
     // without the fused clear the buffer's depth enters here, after the fragments' minimum
-    if (!clear && ri != kNone && st.key[p] >= buffer_key(__ldcg(&v.depth[idx]))) ri = kNone;
+    if (!clear && ri != kNone && st.key(p) >= buffer_key(__ldcg(&v.depth[idx]))) ri = kNone;
     if (ri != kNone) {
       shaded++;
       float b0, b1, b2;
@@ -231,10 +232,10 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
       if constexpr (TileState<T * T>::kKeep) {
         b0 = st.b0[p]; b1 = st.b1[p]; b2 = st.b2[p];
         pay = ri;
-        seq = 0xfffffffeu - (uint32_t)st.key[p];
+        seq = 0xfffffffeu - st.win[p].x;
       } else if (stash) {
         pay = ri;
-        seq = 0xfffffffeu - (uint32_t)st.key[p];
+        seq = 0xfffffffeu - st.win[p].x;
         const float* from = by_warp ? stash + (size_t)by_warp[p] * (size_t)stash_floats(T) : stash;
         const float4 w = __ldcg(reinterpret_cast<const float4*>(from) + p);
         b0 = w.x; b1 = w.y; b2 = w.z;
@@ -254,7 +255,7 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
       const uint32_t prim = v.prim_base + (seq >> 4) + 1u;
       const uint32_t alpha = clear ? v.clear_rgba : __ldcg(&v.color[idx]);
       v.color[idx] = pack_rgb(fragment_s<S>(v, P, b0, b1, b2, prim, bt), alpha);
-      if (v.depth) v.depth[idx] = from_ord((uint32_t)(st.key[p] >> 32));
+      if (v.depth) v.depth[idx] = from_ord(st.z[p]);
       if (v.prim) v.prim[idx] = prim;
     } else if (clear) {
       v.color[idx] = v.clear_rgba;
@@ -272,12 +273,16 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 // pixels the triangles can touch rather than to records x 32 lanes: first the whole windows of
 // 32 of each record, then the remainders laid end to end (warp prefix sum), where the record
 // owning a candidate is found from a bit set at each record's first one.  A covered candidate
-// resolves visibility with a 64-bit atomicMin on
+// resolves visibility by the smallest key
 //     (ordered depth << 32) | (0xfffffffe - seq)
 // in shared memory: smallest depth first, and among equal depths the later submission.
-// The lane whose key is still the minimum after the warp's atomics records the winner's
-// record (two lanes of one step never hold the same key: one triangle covers a pixel
-// once).  Shading then runs once per pixel with a winner.
+// The halves are separate words: a 32-bit atomicMin on the depth decides nearly all, and only
+// where a depth is met again does a second one decide on the submission (64-bit shared atomics
+// took 14 of the load/store unit's cycles a warp; raster of the 4M-triangle soup 669 -> 654 us,
+// 16 recorded views 306 -> 301 us, 64 requests 1,718 -> 1,708 us).
+// The lane whose key is then the minimum records the winner's record (two lanes of one step
+// never hold the same key: one triangle covers a pixel once).  Shading then runs once per pixel
+// with a winner.
 //
 // A view's tiles start their coverage at once; only shading waits for what it reads of other
 // views (the shadow map; in a draw without the fused clear the depth and alpha that earlier
@@ -361,8 +366,8 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
       const unsigned long long k0 = clear ? buffer_key(v.clear_depth) : ~0ull;
 #pragma unroll 8
       for (int q = 0; q < PPL; q++) {
-        st.key[lane + 32 * q] = k0;
-        st.rec[lane + 32 * q] = kNone;
+        st.z[lane + 32 * q] = (uint32_t)(k0 >> 32);
+        st.win[lane + 32 * q] = make_uint2((uint32_t)k0, kNone);
       }
     }
     const uint32_t share = b;
@@ -431,12 +436,12 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
       __syncwarp();
       if (!kKeep && b + 32u + (uint32_t)lane < end) ri_ahead = sc.bins[off + b + 32u + (uint32_t)lane];
       // Visibility of `cnt` queued candidates from the ring head, one per lane: weights
-      // (the divisions of barycentric()), depth, and a 64-bit atomicMin of the key.
+      // (the divisions of barycentric()), depth, and the smaller key.
       uint32_t qh = 0, qn = 0;  // ring head and queued count (warp-uniform)
       auto resolve = [&](uint32_t cnt) {
         __syncwarp();
         const bool act = (uint32_t)lane < cnt;
-        unsigned long long key = 0ull, old = 0ull;
+        uint32_t z = 0u, order = 0u, old = 0u;
         int p = 0, j = 0;
         float b0 = 0.f, b1 = 0.f, b2 = 0.f;
         if (act) {
@@ -448,13 +453,21 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
           const float4 d4 = br.d4[j];
           cover_weights(u.x, u.y, br.b4[j].w, b0, b1, b2);
           // interpolate_depth (graphics.cpp:186-194)
-          const float z = fa(fa(fa(0.f, fm(d4.z, b2)), fm(d4.y, b1)), fm(d4.x, b0));
-          key = ((unsigned long long)ord_bits(z) << 32) | (unsigned long long)(0xfffffffeu - __float_as_uint(d4.w));
-          old = atomicMin(&st.key[p], key);
+          z = ord_bits(fa(fa(fa(0.f, fm(d4.z, b2)), fm(d4.y, b1)), fm(d4.x, b0)));
+          order = 0xfffffffeu - __float_as_uint(d4.w);
+          old = atomicMin(&st.z[p], z);
         }
         __syncwarp();
-        if (act && old > key && st.key[p] == key) {
-          st.rec[p] = br.ri[j];
+        bool wins = act && old >= z && st.z[p] == z;
+        if (__any_sync(kFull, wins && old == z)) {  // an equal depth, here or in the buffer
+          if (wins && old > z) st.win[p].x = 0xffffffffu;
+          __syncwarp();
+          if (wins) wins = atomicMin(&st.win[p].x, order) > order;
+          __syncwarp();
+          wins = wins && st.win[p].x == order;
+        }
+        if (wins) {
+          st.win[p] = make_uint2(order, br.ri[j]);
           if constexpr (kKeep) {
             st.b0[p] = b0;
             st.b1[p] = b1;
@@ -484,7 +497,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
         unsigned cm = __ballot_sync(kFull, covered);
         frags += (uint32_t)__popc(cm);
         if (HIDE) {  // leave out what cannot win any more
-          covered = covered && lowest <= (uint32_t)(st.key[p] >> 32);
+          covered = covered && lowest <= st.z[p];
           cm = __ballot_sync(kFull, covered);
         }
         if (covered) {  // queue behind the pending ones (at most 31 are pending here)
@@ -530,34 +543,34 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
     int q0 = 0, qstep = 1;
     if (SHARED) {
       // merge into the first warp's state: the smaller key per pixel (equal keys are the same
-      // buffer depth or the same triangle); the other states' record words then hold the
+      // buffer depth or the same triangle); the second state's depth words then hold the
       // winner's warp
       __syncthreads();
       for (int p = threadIdx.x; p < NPIX; p += WARPS * 32) {
-        unsigned long long k = sm.st[0].key[p];
+        unsigned long long k = sm.st[0].key(p);
         int w = 0;
 #pragma unroll
         for (int o = 1; o < WARPS; o++) {
-          const unsigned long long ko = sm.st[o].key[p];
+          const unsigned long long ko = sm.st[o].key(p);
           if (ko < k) { k = ko; w = o; }
         }
         if (w) {
-          sm.st[0].key[p] = k;
-          sm.st[0].rec[p] = sm.st[w].rec[p];
+          sm.st[0].z[p] = sm.st[w].z[p];
+          sm.st[0].win[p] = sm.st[w].win[p];
           if constexpr (kKeep) {
             sm.st[0].b0[p] = sm.st[w].b0[p];
             sm.st[0].b1[p] = sm.st[w].b1[p];
             sm.st[0].b2[p] = sm.st[w].b2[p];
           }
         }
-        if constexpr (!kKeep) sm.st[1].rec[p] = (uint32_t)w;
+        if constexpr (!kKeep) sm.st[1].z[p] = (uint32_t)w;
       }
       __syncthreads();
       win = &sm.st[0];
       q0 = warp;
       qstep = WARPS;
       if constexpr (!kKeep) {
-        by_warp = sm.st[1].rec;
+        by_warp = sm.st[1].z;
         if (stash) wstash = stash - (size_t)warp * (size_t)stash_floats(T);
       }
     }
