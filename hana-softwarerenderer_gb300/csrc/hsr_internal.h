@@ -240,15 +240,9 @@ struct MeshOrder {
 int launch_mesh_order(const MeshOrder& o, cudaStream_t s);
 int launch_split_normals(const float* nrm, int n, float* nx, float* ny, float* nz, float4* n4, cudaStream_t s);
 // `from` is mapped host memory or device memory; sizes are multiples of 16.
-// Bounds of `n` positions, then the mesh's faces (raw: 9 indices a face, device memory) into fv, fvt, fvn
-// grouped by the cell of a 64^3 grid that holds their centroid, cells in Morton order.
-// `cells`: kFaceCells + 8 words of scratch; `codes`: one word a face.
-constexpr int kFaceCells = 1 << 18;
-int launch_face_order(const int32_t* raw, int nfaces, const float4* p4, int npos, uint32_t* cells, uint32_t* codes,
-                      int4* fv, int4* fvt, int4* fvn, cudaStream_t s);
 int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s);
 int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s);
-bool culls_own_vertices(size_t faces);  // the cull pass needs no launch_vertex
+bool culls_own_vertices(size_t faces, size_t positions);  // the cull pass needs no launch_vertex
 int launch_setup(const DView* views, int nviews, int nchunks, bool own_vertices, Scratch sc, int grid, cudaStream_t s);
 bool clips_with_emit(size_t faces);  // the emit pass's grid also clips (no launch_post)
 int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms, cudaStream_t s);

@@ -175,7 +175,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   if (e != cudaSuccess) return cuda_fail(e, "draw_noalloc: upload");
   e = cudaMemsetAsync(dev + o_zero, 0, zero_bytes, s);  // counters start at zero every call
   if (e != cudaSuccess) return cuda_fail(e, "draw_noalloc: clear counters");
-  const bool own = culls_own_vertices(faces);
+  const bool own = culls_own_vertices(faces, (size_t)m->npos);
   int kr = own ? 0 : launch_vertex(dview, 1, nvch, rt->num_sms * 8, s);
   if (!kr) kr = launch_setup(dview, 1, nsch, own, sc, rt->num_sms * 8, s);
   if (!kr) kr = launch_emit(dview, T, sc, clips_with_emit(faces), rt->num_sms, s);

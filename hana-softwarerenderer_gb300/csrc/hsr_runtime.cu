@@ -339,7 +339,7 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
   int kr = launch_prep(host, dev, host_bytes, dev + o_zero, zero_bytes, num_sms * 4, s);
   if (kr) return cuda_fail((cudaError_t)kr, "prep kernel");
   mark(1);
-  const bool own = culls_own_vertices(total_faces);
+  const bool own = culls_own_vertices(total_faces, total_pos);
   kr = own ? 0 : launch_vertex(dviews, n, nvch, num_sms * 8, s);
   if (kr) return cuda_fail((cudaError_t)kr, "vertex kernel");
   mark(2);
@@ -386,7 +386,7 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
 }
 
 int Plan::kernel_count() const {
-  return 1 + (nvch && !culls_own_vertices(total_faces) ? 1 : 0) + (nsch ? 1 : 0) + (clips_with_emit(total_faces) ? 2 : 3) + (nscan > 0 ? 1 : 0) + 2;
+  return 1 + (nvch && !culls_own_vertices(total_faces, total_pos) ? 1 : 0) + (nsch ? 1 : 0) + (clips_with_emit(total_faces) ? 2 : 3) + (nscan > 0 ? 1 : 0) + 2;
 }
 
 // Grow the capacity an overflow reported; returns false if nothing overflowed.
@@ -489,7 +489,7 @@ int Runtime::run_sequence(const hsr_draw_desc* descs, int n) {
     timing.batch_ms = ms;
     for (int k = 0; k < HSR_KERNEL_COUNT; k++) {
       float km = timing.kernel_ms[k] = 0.f;
-      if (k == 0 && culls_own_vertices(p.total_faces)) continue;  // part of the cull pass
+      if (k == 0 && culls_own_vertices(p.total_faces, p.total_pos)) continue;  // part of the cull pass
       if (k == 3 && clips_with_emit(p.total_faces)) continue;  // clipped in the emit pass's grid
       if (profiling) cudaEventElapsedTime(&km, ev[k + 1], ev[k + 2]);
       timing.kernel_ms[k] = km;

@@ -1080,8 +1080,11 @@ int launch_big(const DView* views, int tile, Scratch sc, int grid, cudaStream_t 
 // A small sequence's cull pass transforms the corners itself: each vertex about six times, but the
 // vertex stage's launch and its write and read of the screen vertices are saved (whole calls: 2,048
 // faces 68.6 -> 65.9 us, 5,120 faces 81 -> 77.5, 262,144 faces 181 -> 179.5; 655,364 faces equal).
+// So does a large one with a position a face or more, where a vertex serves three corners or
+// fewer (vertex + cull of 4M faces with 3 positions each 176 -> 133 us, with 1.5 144 -> 127, with
+// 1.06 134 -> 123; closed meshes have half a position a face: 64 requests 793 -> 1,000 us).
 constexpr size_t kOwnVertexFaces = (size_t)1 << 18;
-bool culls_own_vertices(size_t faces) { return faces <= kOwnVertexFaces; }
+bool culls_own_vertices(size_t faces, size_t positions) { return faces <= kOwnVertexFaces || positions >= faces; }
 
 int launch_setup(const DView* views, int nviews, int nchunks, bool own_vertices, Scratch sc, int grid, cudaStream_t s) {
   if (nchunks <= 0) return 0;

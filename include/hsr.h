@@ -368,8 +368,8 @@ HSR_API int hsr_server_inject_alloc_failures(hsr_server s, int32_t n);
  * batch_ms spans the upload of the view descriptors to the end of the raster kernel;
  * kernel_ms holds one entry per kernel of the launch sequence, in launch order, filled when
  * profiling is on:
- *   [0] vertex   screen vertices (k_vertex; 0 for a sequence of at most 2^18 faces, whose cull pass
- *                computes them)
+ *   [0] vertex   screen vertices (k_vertex; 0 for a sequence of at most 2^18 faces or of a position a face
+ *                or more, whose cull pass computes them)
  *   [1] cull     fast accept, cull, viewport, bounding box, record (k_setup)
  *   [2] emit     shading payloads and tile counts of the surviving triangles (k_emit)
  *   [3] clip     homogeneous clipper for faces crossing a plane (k_post; 0 for a sequence of at most

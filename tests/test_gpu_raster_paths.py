@@ -165,3 +165,30 @@ def test_hidden_candidates_of_overdrawn_tiles_vs_oracle(tuned, edge, tile):
             o.release()
     assert (rb.prim > 1000).any() and (rb.depth < 1.0).any()
     _check(got, rb, f"hidden edge{edge} tile{tile}")
+
+
+@pytest.mark.parametrize("more", [-1, 0, 1])
+def test_large_meshes_around_a_position_a_face_vs_oracle(gpu, more):
+    """More than 2^18 faces: with fewer positions than faces the screen vertices are computed first,
+    else by the pass that culls the faces."""
+    w, h, n = 640, 360, (1 << 18) + 37
+    rng = np.random.default_rng(7 + more)
+    npos = n + more
+    walk = np.cumsum(rng.normal(0, 2.5, (npos, 2)), axis=0) + rng.uniform(0, 100, 2)
+    p = np.abs((walk + (w, h)) % (2 * w, 2 * h) - (w, h)) * (1.02, 1.02) - (0.01 * w, 0.01 * h)  # some leave the target
+    pos = np.empty((npos, 3), np.float32)
+    pos[:, 0], pos[:, 1] = p[:, 0] / w * 2 - 1, p[:, 1] / h * 2 - 1
+    pos[:, 2] = rng.uniform(-1.001, 1.0, npos)
+    faces = np.zeros((n, 3, 3), np.int32)
+    faces[:, :, 0] = (np.arange(n)[:, None] + np.arange(3)) % npos
+    mesh = scenes.Mesh(pos, np.array([[0, 0, 1]], np.float32), np.zeros((1, 2), np.float32), faces)
+    fr = scenes.Frame(mesh, scenes.FLAT, U.shader_data((0, 0, 1), w, h, identity_mvp=True), w, h, name=f"walk{more}")
+    g = hframe.GpuFrame(fr)
+    try:
+        g.render()
+        got = g.download()
+    finally:
+        g.release()
+    rb = oracle.render_frame(fr)["main"]
+    assert (rb.prim > 0).mean() > 0.5
+    _check(got["main"], rb, fr.name)
