@@ -588,6 +588,8 @@ int hsr_init(int device) {
   }
   e = cudaStreamCreateWithFlags(&rt->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete rt; return cuda_fail(e, "cudaStreamCreate"); }
+  e = cudaMallocHost((void**)&rt->fixed_host, kFixedHostBytes);
+  if (e != cudaSuccess) { delete rt; return cuda_fail(e, "hsr_init: page-locked staging"); }
   for (int k = 0; k < Runtime::kEvents; k++) {
     e = cudaEventCreate(&rt->ev[k]);
     if (e != cudaSuccess) { delete rt; return cuda_fail(e, "cudaEventCreate"); }
@@ -606,6 +608,7 @@ int hsr_shutdown(void) {
   for (auto& kv : g_rt->targets) delete kv.second;
   if (g_rt->arena.base) cudaFree(g_rt->arena.base);
   if (g_rt->staging.base) cudaFreeHost(g_rt->staging.base);
+  cudaFreeHost(g_rt->fixed_host);
   for (int k = 0; k < Runtime::kEvents; k++) cudaEventDestroy(g_rt->ev[k]);
   cudaStreamDestroy(g_rt->stream);
   delete g_rt;

@@ -95,6 +95,8 @@ struct Plan {
 // a batch runs as one launch sequence up to there.
 int first_reclear(const hsr_draw_desc* d, int n);
 
+constexpr size_t kFixedHostBytes = 4096;
+
 struct Runtime {
   int device = 0;
   int num_sms = 1;
@@ -105,6 +107,7 @@ struct Runtime {
   std::unordered_map<uint64_t, TargetObj*> targets;
   Arena arena;
   Pinned staging;
+  char* fixed_host = nullptr;  // page-locked, kFixedHostBytes: hsr_draw_noalloc's view descriptor and control block
   hsr_tuning tuning = {8, 4, 8, 4.0f};
   hsr_stats stats = {};
   uint64_t launches = 0;
