@@ -319,6 +319,39 @@ __device__ __forceinline__ void st_v8(void* p, float4 a, float4 b) {
                "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
                : "memory");
 }
+__device__ __forceinline__ void store_rec(RasterRec* dst, const RasterRec& r) {
+  const float4* s = reinterpret_cast<const float4*>(&r);
+  st_v8(dst, s[0], s[1]);
+  st_v8(reinterpret_cast<char*>(dst) + 32, s[2], s[3]);
+}
+
+// Payload floats a shader reads, rounded up to whole float4s (see the Payload layout).
+__device__ __forceinline__ int payload_f4(int shader) {
+  switch (shader) {
+    case HSR_SHADER_FLAT: return 0;
+    case HSR_SHADER_SHADOW: case HSR_SHADER_GROUND: case HSR_SHADER_TOON: return 2;
+    case HSR_SHADER_TEXTURE: return 3;
+    case HSR_SHADER_TEXTURE_WITH_LIGHT: return 6;
+    default: return 8;
+  }
+}
+
+// Sub-records of a triangle over ntw x nth tiles.
+__device__ __forceinline__ uint32_t sub_records(int ntw, int nth) {
+  return (uint32_t)((ntw + kSubTilesX - 1) / kSubTilesX) * (uint32_t)((nth + kSubTilesY - 1) / kSubTilesY);
+}
+
+// Tile rectangle of a record; T is a power of two (8 or 16).
+__device__ __forceinline__ void rec_tiles(const RasterRec& r, int T, int& tx0, int& ty0, int& ntw, int& nt) {
+  const int ts = __ffs(T) - 1;
+  const int x0 = (int)(r.xr & 0xffffu), x1 = (int)(r.xr >> 16);
+  const int y0 = (int)(r.yr & 0xffffu), y1 = (int)(r.yr >> 16);
+  tx0 = x0 >> ts;
+  ty0 = y0 >> ts;
+  ntw = (x1 >> ts) - tx0 + 1;
+  nt = ntw * ((y1 >> ts) - ty0 + 1);
+}
+
 // The (record, tile) pairs of a warp's records, 32 at a time: lane l's record covers `nt` tiles (0:
 // none, at most 32) in rows of `ntw` from tile `tile0`, `tiles_x` apart.  f(in, tile, owner) is called by
 // all lanes with one pair each (`in`: this lane has one; owner: the lane of its record).

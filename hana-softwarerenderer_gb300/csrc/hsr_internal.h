@@ -51,7 +51,7 @@ constexpr long kScanWaitPolls = 1L << 22;  // scan: a predecessor block's prefix
 enum : uint32_t {
   kRecExact = 1u,  // coordinates outside the range where the division-free coverage test is
                    // exact: the raster evaluates the reference's divisions instead
-  kRecHole = 2u,   // slot of a huge triangle handed to k_big: binned nowhere
+  kRecHole = 2u,   // slot of a huge triangle handed to k_scan: binned nowhere
 };
 
 // One triangle that reached the raster (64 bytes).  A, B-A, C-A are the per-triangle
@@ -163,12 +163,12 @@ struct Ctl {
   unsigned long long frag_px;    // covered (pixel, triangle) pairs the raster depth-tested
   uint32_t ne_tiles;             // tiles with at least one record (k_scan)
   float box_px;                  // pixels of the cull pass's records' bounding boxes (k_emit)
-  unsigned long long pay_bytes;  // shading payload bytes written (k_emit, k_post, k_big)
+  unsigned long long pay_bytes;  // shading payload bytes written (k_emit, k_post, k_scan)
 };
 static_assert(sizeof(Ctl) == 64, "Ctl is read back whole: keep it one 64-byte block");
 
-// A triangle whose bounding box touches more than kMaxRecordTiles tiles, queued by setup
-// and expanded into sub-records by k_post.
+// A triangle whose bounding box touches more than kMaxRecordTiles tiles, queued by
+// the emit and clip passes and expanded into sub-records by k_scan.
 struct __align__(16) BigItem {
   RasterRec rec;
   Payload pay;
@@ -196,6 +196,7 @@ struct Scratch {
   uint32_t* tile_off;       // [ntiles]
   uint32_t* ne_off;         // [ntiles + 1] non-empty tiles before each tile
   uint32_t* tile_list;      // [ntiles] the non-empty tiles in tile order (ne_tiles of them)
+  unsigned long long* split;        // parts of huge triangles split, their sub-records (two words behind scan_status)
   unsigned long long* scan_status;  // [scan blocks]
   uint32_t* bins;   uint32_t bin_cap;
   int32_t ntiles;
@@ -247,11 +248,10 @@ int launch_setup(const DView* views, int nviews, int nchunks, bool own_vertices,
 bool clips_with_emit(size_t faces);  // the emit pass's grid also clips (no launch_post)
 int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms, cudaStream_t s);
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
-int launch_big(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
-int launch_scan(Scratch sc, cudaStream_t s);
+int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStream_t s);
 int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int clear_chunks, uint32_t plane_bytes,
                    cudaStream_t s);
 int launch_raster(const DView* views, int tile, Scratch sc, int grid, int warps, cudaStream_t s);
-int scan_blocks(int ntiles);
+int scan_words(int ntiles);  // 64-bit words of Scratch::scan_status
 
 }  // namespace hsr

@@ -13,7 +13,7 @@
 // allocating routine.  As in hsr_draw, k_prep reads the view descriptor from the staging and
 // zeroes the counters, and the raster's last CTA writes the control block back into it, so the
 // kernels follow each other in one chain (with a copy, a memset and a copy back from a plain host
-// array a 641x359 frame of 20,480 faces took 86 us a call, now 82.5).
+// array a 641x359 frame of 20,480 faces took 86 us a call, then 82.5).
 //
 // Limits and sharing:
 //   - the success path allocates nothing on the device or the host (a failing call only
@@ -122,7 +122,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   const size_t faces = (size_t)m->nfaces, tiles = (size_t)v.ntiles;
   const size_t rec_cap = faces + faces / 4 + 1024, clip_cap = faces / 16 + 256, big_cap = faces / 64 + 256;
   const size_t bin_cap = (size_t)(rt->tuning.bin_factor * (double)(faces + tiles)) + 4096;
-  const int nscan = scan_blocks((int)tiles);
+  const int nscan = scan_words((int)tiles);
   size_t off = 0;
   const size_t o_view = off; off = nal(off + sizeof(DView));
   const size_t host_bytes = off;
@@ -132,7 +132,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   const size_t o_done = off; off = nal(off + sizeof(uint32_t) * (1 + 2 + 1));
   const size_t o_cnt = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_fill = off; off = nal(off + sizeof(uint32_t) * tiles);
-  const size_t o_stat = off; off = nal(off + sizeof(unsigned long long) * (size_t)std::max(nscan, 1));
+  const size_t o_stat = off; off = nal(off + sizeof(unsigned long long) * (size_t)nscan);
   const size_t zero_bytes = off - o_zero;
   const size_t o_toff = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_neoff = off; off = nal(off + sizeof(uint32_t) * (tiles + 1));
@@ -164,6 +164,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   sc.ne_off = (uint32_t*)(dev + o_neoff);
   sc.tile_list = (uint32_t*)(dev + o_list);
   sc.scan_status = (unsigned long long*)(dev + o_stat);
+  sc.split = sc.scan_status + (nscan - 2);
   sc.bins = (uint32_t*)(dev + o_bins); sc.bin_cap = (uint32_t)bin_cap;
   sc.ntiles = (int32_t)tiles;
   sc.nviews = 1;
@@ -182,12 +183,11 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   if (!kr) kr = launch_setup(dview, 1, nsch, own, sc, rt->num_sms * 8, s);
   if (!kr) kr = launch_emit(dview, T, sc, clips_with_emit(faces), rt->num_sms, s);
   if (!kr && !clips_with_emit(faces)) kr = launch_post(dview, T, sc, rt->num_sms * 4, s);
-  if (!kr) kr = launch_big(dview, T, sc, rt->num_sms * 2, s);
-  if (!kr) kr = launch_scan(sc, s);
+  if (!kr) kr = launch_scan(dview, T, sc, rt->num_sms * 2, s);
   if (!kr) kr = launch_scatter(dview, T, sc, rt->num_sms * 8, ncch, 12u, s);
   if (!kr) kr = launch_raster(dview, T, sc, rt->num_sms * rt->tuning.ctas_per_sm, rt->tuning.warps_per_cta, s);
   if (kr) return cuda_fail((cudaError_t)kr, "draw_noalloc: kernel launch");
-  rt->launches += (own ? 7 : 8) + (clips_with_emit(faces) ? 0 : 1);
+  rt->launches += (own ? 6 : 7) + (clips_with_emit(faces) ? 0 : 1);
   const Ctl* hc = reinterpret_cast<const Ctl*>(h + host_bytes);
   const cudaError_t e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "draw_noalloc");

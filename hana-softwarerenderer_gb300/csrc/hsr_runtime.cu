@@ -264,7 +264,7 @@ void Plan::layout() {
   clip_cap = std::min<size_t>(clip_cap, 0xfffff000u);
   big_cap = std::min<size_t>(big_cap, 0xfffff000u);
   bin_cap = std::min<size_t>(bin_cap, 0xfffff000u);
-  nscan = scan_blocks((int)total_tiles);
+  nscan = scan_words((int)total_tiles);
   // [views | chunks | per-view vertex outputs | ctl | view_done | tile_count | tile_fill |
   //  scan_status | tile_off | ne_off | tile_list | recs | clipbuf | bins]; the zeroed part is one memset
   size_t off = 0;
@@ -276,7 +276,7 @@ void Plan::layout() {
   o_done = off; off = align_up(off + sizeof(uint32_t) * ((size_t)n + 2 * kRasterGroups + 1), 256);
   o_cnt = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_fill = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
-  o_stat = off; off = align_up(off + sizeof(unsigned long long) * std::max(nscan, 1), 256);
+  o_stat = off; off = align_up(off + sizeof(unsigned long long) * nscan, 256);
   zero_bytes = off - o_zero;
   o_toff = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_neoff = off; off = align_up(off + sizeof(uint32_t) * (total_tiles + 1), 256);
@@ -311,6 +311,7 @@ void Plan::bind(char* dev_base, char* host_base) {
   sc.ne_off = (uint32_t*)(dev + o_neoff);
   sc.tile_list = (uint32_t*)(dev + o_list);
   sc.scan_status = (unsigned long long*)(dev + o_stat);
+  sc.split = sc.scan_status + (nscan - 2);
   sc.bins = (uint32_t*)(dev + o_bins); sc.bin_cap = (uint32_t)bin_cap;
   sc.ntiles = (int32_t)total_tiles;
   sc.nviews = n;
@@ -353,10 +354,8 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
   kr = one_grid ? 0 : launch_post(dviews, tile, sc, num_sms * 4, s);
   if (kr) return cuda_fail((cudaError_t)kr, "post kernel");
   mark(5);
-  kr = launch_big(dviews, tile, sc, num_sms * 2, s);
-  if (kr) return cuda_fail((cudaError_t)kr, "big-triangle kernel");
   mark(6);
-  kr = launch_scan(sc, s);
+  kr = launch_scan(dviews, tile, sc, num_sms * 2, s);
   if (kr) return cuda_fail((cudaError_t)kr, "scan kernel");
   mark(7);
   // grid-stride over the records: one full wave of 256-thread blocks (fewer when there are
@@ -386,7 +385,7 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
 }
 
 int Plan::kernel_count() const {
-  return 1 + (nvch && !culls_own_vertices(total_faces, total_pos) ? 1 : 0) + (nsch ? 1 : 0) + (clips_with_emit(total_faces) ? 2 : 3) + (nscan > 0 ? 1 : 0) + 2;
+  return 1 + (nvch && !culls_own_vertices(total_faces, total_pos) ? 1 : 0) + (nsch ? 1 : 0) + (clips_with_emit(total_faces) ? 1 : 2) + 3;
 }
 
 // Grow the capacity an overflow reported; returns false if nothing overflowed.
@@ -490,6 +489,7 @@ int Runtime::run_sequence(const hsr_draw_desc* descs, int n) {
     for (int k = 0; k < HSR_KERNEL_COUNT; k++) {
       float km = timing.kernel_ms[k] = 0.f;
       if (k == 0 && culls_own_vertices(p.total_faces, p.total_pos)) continue;  // part of the cull pass
+      if (k == 4) continue;  // split in the scan's grid
       if (k == 3 && clips_with_emit(p.total_faces)) continue;  // clipped in the emit pass's grid
       if (profiling) cudaEventElapsedTime(&km, ev[k + 1], ev[k + 2]);
       timing.kernel_ms[k] = km;

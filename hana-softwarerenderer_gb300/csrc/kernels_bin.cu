@@ -4,12 +4,12 @@
 //
 // k_prep    the launch sequence's first kernel: view descriptors from the host's page-locked
 //           staging, counters to zero.
-// k_scan    exclusive prefix sums of the per-tile counts and of the non-empty tiles, single
+// k_scan    sub-records of triangles that touch more than kMaxRecordTiles tiles, then exclusive prefix sums of the per-tile counts and of the non-empty tiles, single
 //           pass with decoupled look-back, and the list of non-empty tiles in tile order;
 //           block order comes from a ticket so a block only waits on blocks that already
 //           run, and every wait is bounded (error bit + give up, never a hang).
 // k_scatter writes record indices into the per-tile lists with warp-aggregated atomics;
-//           a record touches at most kMaxRecordTiles tiles (k_big splits larger ones).
+//           a record touches at most kMaxRecordTiles tiles (k_scan splits larger ones).
 //           The same grid clears the tiles no record touches, streamed in row order.
 #include <algorithm>
 
@@ -19,15 +19,15 @@
 namespace hsr {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
+constexpr int kScanThreads = 512;
+constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;  // tiles per scan block
 constexpr unsigned long long kFlagAgg = 1ull << 62;
 constexpr unsigned long long kFlagPre = 2ull << 62;
 constexpr unsigned long long kValMask = (1ull << 62) - 1;
 
 __host__ __device__ __forceinline__ int scan_blocks_hd(int ntiles) { return (ntiles + kScanTile - 1) / kScanTile; }
-int scan_blocks(int ntiles) { return scan_blocks_hd(ntiles); }
+int scan_words(int ntiles) { return scan_blocks_hd(ntiles) + 2; }  // and Scratch::split
 
 __device__ __forceinline__ unsigned long long ld_volatile64(const unsigned long long* p) {
   return *reinterpret_cast<const volatile unsigned long long*>(p);
@@ -62,23 +62,130 @@ int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t 
   return (int)cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan(Scratch sc) {
+// A huge triangle's tile rectangle splits into sub-records over blocks of kSubTilesX x kSubTilesY
+// tiles (same triangle constants and seq, pixel range clipped to the block, each with its own copy
+// of the payload, since a record's payload index is its own index), and every tile of the
+// rectangle is counted once.  The sub-ranges partition the triangle's pixel range, so each pixel is
+// still tested exactly once.  `parts` warps share the triangle.  Returns a lane's number of tiles.
+// (A warp and not a CTA each: most queued triangles have some tens of tiles, and what takes the time
+// is the chain of loads from the queue to the view.)
+__device__ __forceinline__ uint32_t split_triangle(const DView* __restrict__ views, int T, const Scratch& sc, const BigItem& bi,
+                                                   uint32_t first, int part, int parts) {
+  const RasterRec b = bi.rec;
+  const DView& v = views[b.view & kRecViewMask];
+  int tx0, ty0, ntw, nt;
+  rec_tiles(b, T, tx0, ty0, ntw, nt);
+  const int nth = nt / ntw;
+  const int nbx = (ntw + kSubTilesX - 1) / kSubTilesX;
+  const int nsub = (int)sub_records(ntw, nth);
+  const uint32_t base = first + b.pad;
+  const int i0 = part * 32 + (int)(threadIdx.x & 31u), step = parts * 32;
+  if ((uint64_t)base + (uint64_t)nsub > (uint64_t)sc.rec_cap) {
+    if (i0 == 0) atomicOr(&sc.ctl->error, kErrRecOverflow);
+    return 0u;
+  }
+  const int nf4 = payload_f4(v.shader);
+  for (int k = i0; k < nsub * nf4; k += step)
+    reinterpret_cast<float4*>(&sc.pay[base + (uint32_t)(k / nf4)])[k % nf4] =
+        reinterpret_cast<const float4*>(&bi.pay)[k % nf4];
+  if (i0 == 0 && nf4) atomicAdd(&sc.ctl->pay_bytes, 16ull * (unsigned long long)(nf4 * nsub));
+  const int x0 = (int)(b.xr & 0xffffu), x1 = (int)(b.xr >> 16);
+  const int y0 = (int)(b.yr & 0xffffu), y1 = (int)(b.yr >> 16);
+  for (int sidx = i0; sidx < nsub; sidx += step) {
+    const int bx = sidx % nbx, by = sidx / nbx;
+    const int stx0 = tx0 + bx * kSubTilesX, stx1 = min(tx0 + ntw - 1, stx0 + kSubTilesX - 1);
+    const int sty0 = ty0 + by * kSubTilesY, sty1 = min(ty0 + nth - 1, sty0 + kSubTilesY - 1);
+    RasterRec w = b;
+    w.xr = (uint32_t)max(x0, stx0 * T) | ((uint32_t)min(x1, stx1 * T + T - 1) << 16);
+    w.yr = (uint32_t)max(y0, sty0 * T) | ((uint32_t)min(y1, sty1 * T + T - 1) << 16);
+    w.pad = 0u;
+    store_rec(&sc.recs[base + (uint32_t)sidx], w);
+  }
+  for (int k = i0; k < nt; k += step)
+    atomicAdd(&sc.tile_count[v.tile_base + (ty0 + k / ntw) * v.tiles_x + tx0 + k % ntw], 1u);
+  return (uint32_t)(nt / step) + 1u;
+}
+
+// Sub-records of the queued huge triangles, then the scan, in one grid: blocks take tickets; where
+// triangles are queued the first ones split them (up to kMaxParts warps each), and a scan block waits,
+// bounded, until all are split, which only blocks with lower tickets do.  Most draws queue none and
+// scan at once.
+//
+// A launch less and no wait where nothing is split, the look-back over 32 predecessors at a time (one
+// per lane; it was one after the other) and a triangle split by up to 256 warps (it was a CTA): split
+// and scan 12.1 -> 6.0 us for 91 tiles, 22 -> 14 for a 1920x1080 frame over a ground plane (four
+// triangles of 8,000 to 32,000 tiles), 24.5 -> 12 for 64 requests; whole calls of a 128x128 draw
+// 65.8 -> 64.2 us, of six objects in 1280x720 224 -> 219, of a recorded 1280x720 frame 178.7 -> 175.9.
+constexpr uint32_t kMaxParts = 256;
+constexpr uint32_t kScanWarps = kScanThreads / 32;
+constexpr uint32_t kStepsToReport = 4096;  // a splitter reports at least every few milliseconds
+__global__ void __launch_bounds__(kScanThreads) k_scan(const DView* __restrict__ views, int T, Scratch sc, uint32_t splitters) {
   __shared__ unsigned long long warp_sums[kScanThreads / 32];
   __shared__ unsigned long long s_prefix;
   __shared__ uint32_t s_block;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nblocks = scan_blocks_hd(sc.ntiles);
+  unsigned long long* split_done = sc.split;  // parts of triangles split
+  const long limit = sc.poll_limit > 0 ? (long)sc.poll_limit : kScanWaitPolls;
   chain_wait();
   if (threadIdx.x == 0) s_block = atomicAdd(&sc.ctl->scan_ticket, 1u);
   __syncthreads();
-  const uint32_t blk = s_block;
+  uint32_t blk = s_block;
+  const uint32_t nbig = min(sc.ctl->big_count, sc.big_cap);
+  if (nbig > 0u) {
+    const uint32_t parts = min(max(splitters * kScanWarps / nbig, 1u), kMaxParts), units = nbig * parts;
+    const uint32_t first = min(splitters, (units + kScanWarps - 1) / kScanWarps);
+    if (blk < first) {
+      const bool skip = (sc.ctl->error & kErrCapacity) != 0u;  // nothing will be drawn
+      // (the clipper's count is final, and grows by the sub-records' only when all parts are done)
+      const uint32_t base = sc.ctl->rec_count + sc.ctl->rec_extra;
+      uint32_t mine = 0, steps = 0;  // the CTA's parts done, and a thread's tiles in them
+      for (uint32_t u0 = blk * kScanWarps; u0 < units; u0 += first * kScanWarps) {
+        const uint32_t u = u0 + (uint32_t)warp;
+        if (!skip && u < units) steps += split_triangle(views, T, sc, sc.bigq[u / parts], base, (int)(u % parts), (int)parts);
+        mine += min((uint32_t)kScanWarps, units - u0);
+        if (!__syncthreads_or(steps >= kStepsToReport || u0 + first * kScanWarps >= units)) continue;
+        if (threadIdx.x == 0) {
+          __threadfence();
+          atomicAdd(split_done, (unsigned long long)mine);
+        }
+        mine = steps = 0;
+      }
+      return;
+    }
+    blk -= first;
+    if (blk >= (uint32_t)nblocks) return;
+    if (threadIdx.x == 0) {
+      unsigned long long seen = 0;
+      for (long spins = 0;;) {  // the limit counts from the last report
+        const unsigned long long s = ld_volatile64(split_done);
+        if (s >= units) break;
+        if (s != seen) { seen = s; spins = 0; }
+        if (++spins > limit) {
+          atomicOr(&sc.ctl->error, kErrScanTimeout);
+          break;
+        }
+        __nanosleep(64);
+      }
+      __threadfence();
+      if ((int)blk == nblocks - 1) sc.ctl->rec_extra += (uint32_t)ld_volatile64(sc.split + 1);
+    }
+    __syncthreads();
+  }
+  if (blk >= (uint32_t)nblocks) return;
   const int base = (int)blk * kScanTile + (int)threadIdx.x * kScanItems;
   uint32_t vals[kScanItems];
+  static_assert(kScanItems == 4, "one 16-byte load");
+  if (base + kScanItems <= sc.ntiles) {
+    const uint4 c = __ldcg(reinterpret_cast<const uint4*>(sc.tile_count + base));
+    vals[0] = c.x; vals[1] = c.y; vals[2] = c.z; vals[3] = c.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) vals[k] = base + k < sc.ntiles ? __ldcg(sc.tile_count + base + k) : 0u;
+  }
   unsigned long long local = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++) {
-    vals[k] = (base + k < sc.ntiles) ? sc.tile_count[base + k] : 0u;
-    local += scan_item(vals[k]);
-  }
+  for (int k = 0; k < kScanItems; k++) local += scan_item(vals[k]);
   // block-wide exclusive scan of the thread sums
   unsigned long long incl = local;
 #pragma unroll
@@ -97,14 +204,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Scratch sc) {
       if (lane >= o) wi += y;
     }
     if (lane < kScanThreads / 32) warp_sums[lane] = wi - w;  // exclusive per warp
-    if (lane == kScanThreads / 32 - 1) {
-      // lane 7 holds the block aggregate; publish and look back
-      const unsigned long long agg = wi;
-      unsigned long long* st = sc.scan_status;
-      unsigned long long prefix = 0;
-      const long limit = sc.poll_limit > 0 ? (long)sc.poll_limit : kScanWaitPolls;
-      if (blk == 0 && (sc.faults & HSR_FAULT_SCAN_STALL)) {
-        // injected stall: withhold the prefix and wait on a word nothing sets (its own)
+    const unsigned long long agg = __shfl_sync(kFull, wi, kScanThreads / 32 - 1);  // the block's; publish, look back
+    unsigned long long* st = sc.scan_status;
+    unsigned long long prefix = 0;
+    if (blk == 0 && (sc.faults & HSR_FAULT_SCAN_STALL)) {
+      // injected stall: withhold the prefix and wait on a word nothing sets (its own)
+      if (lane == 0) {
         long spins = 0;
         while ((ld_volatile64(&st[0]) >> 62) == 0) {
           if (++spins > limit) {
@@ -113,32 +218,37 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Scratch sc) {
           }
           __nanosleep(64);
         }
-      } else if (blk == 0) {
-        atomicExch(&st[0], kFlagPre | agg);
-      } else {
-        atomicExch(&st[blk], kFlagAgg | agg);
-        unsigned long long acc = 0;
-        int p = (int)blk - 1;
-        long spins = 0;
-        while (p >= 0) {
-          const unsigned long long s = ld_volatile64(&st[p]);
-          if ((s >> 62) == 0) {
-            if (++spins > limit) {
-              atomicOr(&sc.ctl->error, kErrScanTimeout);
-              break;
-            }
-            __nanosleep(64);
-            continue;
-          }
-          acc += s & kValMask;
-          if ((s >> 62) == 2) break;
-          p--;
-        }
-        prefix = acc;
-        atomicExch(&st[blk], kFlagPre | (acc + agg));
       }
+    } else if (blk == 0) {
+      if (lane == 0) atomicExch(&st[0], kFlagPre | agg);
+    } else {
+      if (lane == 0) atomicExch(&st[blk], kFlagAgg | agg);
+      long spins = 0;
+      for (int p = (int)blk - 1; p >= 0;) {
+        // lane l looks at the l-th predecessor; before block 0 there is a prefix of nothing
+        const unsigned long long s = p >= lane ? ld_volatile64(&st[p - lane]) : kFlagPre;
+        const unsigned pre = __ballot_sync(kFull, (s >> 62) == 2), none = __ballot_sync(kFull, (s >> 62) == 0);
+        const unsigned use = pre ? (pre & -pre) | ((pre & -pre) - 1u) : kFull;  // up to the nearest prefix
+        if (none & use) {
+          if (++spins > limit) {
+            if (lane == 0) atomicOr(&sc.ctl->error, kErrScanTimeout);
+            break;
+          }
+          __nanosleep(64);
+          continue;
+        }
+        unsigned long long sum = (use >> lane & 1u) ? s & kValMask : 0ull;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+        prefix += sum;
+        if (pre) break;
+        p -= 32;
+      }
+      if (lane == 0) atomicExch(&st[blk], kFlagPre | (prefix + agg));
+    }
+    if (lane == 0) {
       s_prefix = prefix;
-      if ((int)blk == scan_blocks_hd(sc.ntiles) - 1) {
+      if ((int)blk == nblocks - 1) {
         const unsigned long long total = prefix + agg;
         const unsigned long long pairs = total & kCntMask;
         const uint32_t ne = (uint32_t)(total >> kCntBits);
@@ -164,10 +274,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Scratch sc) {
   }
 }
 
-int launch_scan(Scratch sc, cudaStream_t s) {
-  const int nb = scan_blocks(sc.ntiles);
-  if (nb <= 0) return 0;
-  return launch_chained(k_scan, nb, kScanThreads, 0, s, sc);
+int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStream_t s) {
+  return launch_chained(k_scan, splitters + scan_blocks_hd(sc.ntiles), kScanThreads, 0, s, views, tile, sc, (uint32_t)splitters);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -188,7 +296,7 @@ __device__ __forceinline__ void scatter_records(const DView* __restrict__ views,
     // the record's view and pixel range: its last 16 bytes (seq, view, xr, yr) in one load
     const uint4 w = ok ? *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(&sc.recs[i]) + 48)
                        : make_uint4(0u, kRecHole << kRecFlagShift, 0u, 0u);
-    if (ok && !((w.y >> kRecFlagShift) & kRecHole)) {  // holes: huge triangles split by k_big
+    if (ok && !((w.y >> kRecFlagShift) & kRecHole)) {  // holes: huge triangles split by k_scan
       const uint32_t xr = w.z, yr = w.w;
       const DView& v = views[w.y & kRecViewMask];
       tiles_x = v.tiles_x;

@@ -18,8 +18,8 @@
 // surviving triangle; faces that need the clipper are queued.  k_emit writes the surviving
 // records' shading payloads and tile counts on dense warps; k_post clips the queued faces (two
 // per warp: lane k of a half-warp carries varying k of the polygon through Sutherland-Hodgman)
-// and emits their fan triangles; k_big splits triangles that touch more than kMaxRecordTiles
-// tiles into sub-records.
+// and emits their fan triangles.  Triangles that touch more than kMaxRecordTiles tiles are queued
+// for the scan (kernels_bin.cu), which splits them into sub-records.
 #include <float.h>
 
 #include <algorithm>
@@ -498,23 +498,6 @@ __device__ __forceinline__ bool build_rec(const DView& v, F3 n0, F3 n1, F3 n2, u
   return true;
 }
 
-__device__ __forceinline__ void store_rec(RasterRec* dst, const RasterRec& r) {
-  const float4* s = reinterpret_cast<const float4*>(&r);
-  st_v8(dst, s[0], s[1]);
-  st_v8(reinterpret_cast<char*>(dst) + 32, s[2], s[3]);
-}
-
-// Payload floats a shader reads, rounded up to whole float4s (see the Payload layout).
-__device__ __forceinline__ int payload_f4(int shader) {
-  switch (shader) {
-    case HSR_SHADER_FLAT: return 0;
-    case HSR_SHADER_SHADOW: case HSR_SHADER_GROUND: case HSR_SHADER_TOON: return 2;
-    case HSR_SHADER_TEXTURE: return 3;
-    case HSR_SHADER_TEXTURE_WITH_LIGHT: return 6;
-    default: return 8;
-  }
-}
-
 // Corner varyings c[k] in shader_struct_v2f order (13 floats) -> payload.
 __device__ __forceinline__ void make_payload(int shader, const float* c0, const float* c1, const float* c2,
                                              Payload& p) {
@@ -543,17 +526,6 @@ __device__ __forceinline__ void store_payload(Payload* dst, const Payload& p, in
     if (q + 1 < nf4) st_v8(d + q, s[q], s[q + 1]);
     else if (q < nf4) d[q] = s[q];
   }
-}
-
-// Tile rectangle of a record; T is a power of two (8 or 16).
-__device__ __forceinline__ void rec_tiles(const RasterRec& r, int T, int& tx0, int& ty0, int& ntw, int& nt) {
-  const int ts = __ffs(T) - 1;
-  const int x0 = (int)(r.xr & 0xffffu), x1 = (int)(r.xr >> 16);
-  const int y0 = (int)(r.yr & 0xffffu), y1 = (int)(r.yr >> 16);
-  tx0 = x0 >> ts;
-  ty0 = y0 >> ts;
-  ntw = (x1 >> ts) - tx0 + 1;
-  nt = ntw * ((y1 >> ts) - ty0 + 1);
 }
 
 // Slot of this lane's item when `want`, one atomicAdd per warp (~0u otherwise).
@@ -630,6 +602,23 @@ __device__ void append_small(bool valid, uint32_t slot, RasterRec r, const Paylo
   const bool ok = valid && slot < sc.rec_cap;
   if (valid && !ok) atomicOr(&sc.ctl->error, kErrRecOverflow);
   append_counts(ok, slot, r, pl, nf4, v, T, sc);
+}
+
+// Hand over a triangle that touches more than kMaxRecordTiles tiles at the queue slot `bslot`:
+// the places of its sub-records among all (behind the clipper's records) are reserved here, in
+// RasterRec::pad of the queued record, so that several CTAs can split one triangle without talking to
+// each other.
+__device__ __forceinline__ void queue_big(uint32_t bslot, RasterRec& r, const Payload& pl, int nf4, int T,
+                                          const Scratch& sc) {
+  const int ts = __ffs(T) - 1;
+  auto tiles = [ts](uint32_t range) { return (int)((range >> 16 >> ts) - ((range & 0xffffu) >> ts)) + 1; };
+  r.pad = (uint32_t)atomicAdd(sc.split + 1, (unsigned long long)sub_records(tiles(r.xr), tiles(r.yr)));
+  if (bslot < sc.big_cap) {
+    store_rec(&sc.bigq[bslot].rec, r);
+    store_payload(&sc.bigq[bslot].pay, pl, nf4);
+  } else {
+    atomicOr(&sc.ctl->error, kErrBigOverflow);
+  }
 }
 
 // True when the reference's clipper returns 0 vertices for this face without creating any
@@ -861,19 +850,12 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
   append_small(valid && !big, slot, r, pl, nf4, v, T, sc);
   if (valid && !big && slot < sc.rec_cap) pay_bytes += 16u * (uint32_t)nf4;
   const uint32_t bslot = warp_reserve(big, &sc.ctl->big_count);
-  if (big) {
-    if (bslot < sc.big_cap) {
-      store_rec(&sc.bigq[bslot].rec, r);
-      store_payload(&sc.bigq[bslot].pay, pl, nf4);
-    } else {
-      atomicOr(&sc.ctl->error, kErrBigOverflow);
-    }
-  }
+  if (big) queue_big(bslot, r, pl, nf4, T, sc);
   __syncwarp();
 }
 
 // Emit pass over the records of k_setup (dense: one thread per surviving triangle): the
-// shading payload, the tile counts, and the hand-over of huge triangles to k_big (their
+// shading payload, the tile counts, and the hand-over of huge triangles to k_scan (their
 // slot becomes a hole the binning skips).  Grid-stride with warp-uniform trip counts, so
 // the warp collectives of append_small see every lane.
 __device__ __forceinline__ void emit_records(const DView* __restrict__ views, int T, const Scratch& sc, uint32_t block,
@@ -881,7 +863,7 @@ __device__ __forceinline__ void emit_records(const DView* __restrict__ views, in
   const int lane = threadIdx.x & 31;
   const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
   const uint32_t stride = nblocks * blockDim.x;
-  uint32_t pay_bytes = 0;  // payload bytes this lane wrote for the raster (big ones: k_big)
+  uint32_t pay_bytes = 0;  // payload bytes this lane wrote for the raster (split ones: k_scan)
   float box_px = 0.f;      // pixels of its records' bounding boxes
   for (uint32_t i0 = block * blockDim.x + (threadIdx.x & ~31u); i0 < nrec; i0 += stride) {
     const uint32_t i = i0 + (uint32_t)lane;
@@ -893,7 +875,7 @@ __device__ __forceinline__ void emit_records(const DView* __restrict__ views, in
     if (i < nrec) {
       // the words this pass needs (the face, and seq, view, pixel range in the last 16 bytes); the
       // whole record only for a huge triangle.  Every record below rec_count is the
-      // cull pass's: the clipper and k_big append theirs behind it.
+      // cull pass's: the clipper's and the sub-records come behind it.
       const uint4 a = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(&sc.recs[i]) + 48);
       const int f = (int)sc.recs[i].face;
       r.seq = a.x; r.view = a.y; r.xr = a.z; r.yr = a.w;
@@ -919,12 +901,7 @@ __device__ __forceinline__ void emit_records(const DView* __restrict__ views, in
     if (big) {
       r = sc.recs[i];
       sc.recs[i].view = r.view | (kRecHole << kRecFlagShift);
-      if (bslot < sc.big_cap) {
-        store_rec(&sc.bigq[bslot].rec, r);
-        store_payload(&sc.bigq[bslot].pay, pl, nf4);
-      } else {
-        atomicOr(&sc.ctl->error, kErrBigOverflow);
-      }
+      queue_big(bslot, r, pl, nf4, T, sc);
     }
   }
   // one atomic of each a block on the control block's line, which serves them one by one (a warp
@@ -1017,64 +994,6 @@ int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms
 
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {
   return launch_chained(k_post, grid, kEmitThreads, 0, s, views, tile, sc);
-}
-
-constexpr int kBigThreads = 512;
-
-// Expands each queued huge triangle with a whole CTA: its tile rectangle splits into
-// sub-records over blocks of kSubTilesX x kSubTilesY tiles (same triangle constants and
-// seq, pixel range clipped to the block, one shared payload at the first sub-record's
-// slot), and every tile of the rectangle is counted once.  The sub-ranges partition the
-// triangle's pixel range, so each pixel is still tested exactly once.
-__global__ void __launch_bounds__(kBigThreads) k_big(const DView* __restrict__ views, int T, Scratch sc) {
-  __shared__ uint32_t s_base;
-  chain_wait();
-  if (sc.ctl->error & kErrCapacity) return;
-  const uint32_t nbig = min(sc.ctl->big_count, sc.big_cap);
-  for (uint32_t item = blockIdx.x; item < nbig; item += gridDim.x) {
-    const BigItem& bi = sc.bigq[item];
-    const RasterRec b = bi.rec;
-    const DView& v = views[b.view & kRecViewMask];
-    int tx0, ty0, ntw, nt;
-    rec_tiles(b, T, tx0, ty0, ntw, nt);
-    const int nth = nt / ntw;
-    const int nbx = (ntw + kSubTilesX - 1) / kSubTilesX, nby = (nth + kSubTilesY - 1) / kSubTilesY;
-    const int nsub = nbx * nby;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const uint32_t base = sc.ctl->rec_count + atomicAdd(&sc.ctl->rec_extra, (uint32_t)nsub);
-      s_base = base;
-      if ((uint64_t)base + (uint64_t)nsub > (uint64_t)sc.rec_cap) atomicOr(&sc.ctl->error, kErrRecOverflow);
-    }
-    __syncthreads();
-    const uint32_t base = s_base;
-    if ((uint64_t)base + (uint64_t)nsub > (uint64_t)sc.rec_cap) continue;
-    // every sub-record carries its own copy of the payload, so that a record's payload index is
-    // its own index (the raster loads the payload from the record index in shared memory)
-    const int nf4 = payload_f4(v.shader);
-    for (int k = threadIdx.x; k < nsub * nf4; k += kBigThreads)
-      reinterpret_cast<float4*>(&sc.pay[base + (uint32_t)(k / nf4)])[k % nf4] =
-          reinterpret_cast<const float4*>(&bi.pay)[k % nf4];
-    if (threadIdx.x == 0 && nf4) atomicAdd(&sc.ctl->pay_bytes, 16ull * (unsigned long long)(nf4 * nsub));
-    const int x0 = (int)(b.xr & 0xffffu), x1 = (int)(b.xr >> 16);
-    const int y0 = (int)(b.yr & 0xffffu), y1 = (int)(b.yr >> 16);
-    for (int sidx = threadIdx.x; sidx < nsub; sidx += kBigThreads) {
-      const int bx = sidx % nbx, by = sidx / nbx;
-      const int stx0 = tx0 + bx * kSubTilesX, stx1 = min(tx0 + ntw - 1, stx0 + kSubTilesX - 1);
-      const int sty0 = ty0 + by * kSubTilesY, sty1 = min(ty0 + nth - 1, sty0 + kSubTilesY - 1);
-      RasterRec w = b;
-      w.xr = (uint32_t)max(x0, stx0 * T) | ((uint32_t)min(x1, stx1 * T + T - 1) << 16);
-      w.yr = (uint32_t)max(y0, sty0 * T) | ((uint32_t)min(y1, sty1 * T + T - 1) << 16);
-      w.pad = 0u;
-      store_rec(&sc.recs[base + (uint32_t)sidx], w);
-    }
-    for (int k = threadIdx.x; k < nt; k += kBigThreads)
-      atomicAdd(&sc.tile_count[v.tile_base + (ty0 + k / ntw) * v.tiles_x + tx0 + k % ntw], 1u);
-  }
-}
-
-int launch_big(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s) {
-  return launch_chained(k_big, grid, kBigThreads, 0, s, views, tile, sc);
 }
 
 // A small sequence's cull pass transforms the corners itself: each vertex about six times, but the

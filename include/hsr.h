@@ -374,8 +374,8 @@ HSR_API int hsr_server_inject_alloc_failures(hsr_server s, int32_t n);
  *   [2] emit     shading payloads and tile counts of the surviving triangles (k_emit)
  *   [3] clip     homogeneous clipper for faces crossing a plane (k_post; 0 for a sequence of at most
  *                2^21 faces, which clips in the emit pass's grid)
- *   [4] split    sub-records of triangles touching many tiles (k_big)
- *   [5] scan     prefix sums over the tile counts (k_scan)
+ *   [4] split    0: the scan's grid splits the triangles that touch many tiles
+ *   [5] scan     sub-records of those, prefix sums over the tile counts (k_scan)
  *   [6] scatter  tile lists, and the clear of tiles without triangles (k_scatter)
  *   [7] raster   coverage, depth test, shading, writes (k_raster) */
 #define HSR_KERNEL_COUNT 8

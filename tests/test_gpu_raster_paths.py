@@ -192,3 +192,35 @@ def test_large_meshes_around_a_position_a_face_vs_oracle(gpu, more):
     rb = oracle.render_frame(fr)["main"]
     assert (rb.prim > 0).mean() > 0.5
     _check(got["main"], rb, fr.name)
+
+
+@pytest.mark.parametrize("size", [(200, 160), (2100, 2090)])
+@pytest.mark.parametrize("nbig", [0, 1, 3, 300, 6000])
+def test_split_triangles_and_the_scan_behind_them_vs_oracle(tuned, nbig, size):
+    """No, few (many warps each) and many (several rounds of warps) triangles that are split, small and
+    clipped ones among them, before a scan of one block and of more than 32 (8x8 tiles)."""
+    tuned.set_tuning(tile=8, warps_per_cta=4, ctas_per_sm=8)
+    w, h = size
+    rng = np.random.default_rng(nbig + w)
+    n = nbig + 500
+    edge = np.full(n, 5.0)
+    edge[rng.permutation(n)[:nbig]] = min(w, h) if nbig < 10 else 110.0
+    c = rng.uniform(0, (w, h), (n, 1, 2)) if nbig >= 10 else rng.uniform(0.3, 0.7, (n, 1, 2)) * (w, h)
+    ang = rng.uniform(0, 2 * np.pi, (n, 1)) + np.arange(3) * (2 * np.pi / 3)
+    p = c + edge[:, None, None] / 2 * np.stack([np.cos(ang), np.sin(ang)], axis=2)
+    pos = np.empty((n, 3, 3), np.float32)
+    pos[:, :, 0], pos[:, :, 1] = p[:, :, 0] / w * 2 - 1, p[:, :, 1] / h * 2 - 1
+    pos[:, :, 2] = rng.uniform(-0.9, 0.9, (n, 1)).astype(np.float32)
+    faces = np.zeros((n, 3, 3), np.int32)
+    faces[:, :, 0] = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+    mesh = scenes.Mesh(pos.reshape(-1, 3), np.array([[0, 0, 1]], np.float32), np.zeros((1, 2), np.float32), faces)
+    fr = scenes.Frame(mesh, scenes.FLAT, U.shader_data((0, 0, 1), w, h, identity_mvp=True), w, h, name=f"split{nbig}")
+    g = hframe.GpuFrame(fr)
+    try:
+        g.render()
+        split = tuned.last_timing()["split_triangles"]
+        got = g.download()
+    finally:
+        g.release()
+    assert split >= nbig // 3 if nbig else split == 0
+    _check(got["main"], oracle.render_frame(fr)["main"], fr.name)
