@@ -311,24 +311,23 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   }
   const uint32_t nrec = min(sc.ctl->rec_count + sc.ctl->rec_extra, sc.rec_cap);
 
-  // The non-empty tiles are handed out by one counter over their list, two ahead: while a
-  // tile is rasterised, the next tile's list bounds are already loading and the one after it
-  // is being claimed, so neither the counter's round trip nor the list lookup waits on the
-  // critical path (the list is in tile order and dependencies only point to lower tile
-  // indices, so holding later tiles never blocks).
+  // The non-empty tiles are handed out by one counter over their list, each when its warp is ready
+  // for it: the list is in tile order and dependencies only point to lower tile indices, so
+  // nobody waits for a tile that is not yet being drawn.  (Claimed two tiles ahead, to hide the
+  // counter and the lists, tiles lay with warps that were busy or waiting while others were done
+  // or waited for them: 64 requests 1,705 -> 1,523 us, six objects 135 -> 92, 16 views 301 -> 272,
+  // 1080p frame 184 -> 166, the 4M-triangle soup 653 -> 600.  To claim one before the shading
+  // waits gave half of that.)
   const uint32_t ntiles = (uint32_t)sc.ntiles;
   const uint32_t lane_magic = (65536u + (uint32_t)lane) / ((uint32_t)lane + 1u);  // ceil(65536 / (lane + 1))
   const uint32_t upto = (2u << lane) - 1u;  // this lane and those below
-  uint32_t li = 0, li_ahead = 0;  // positions in the list
+  uint32_t li = 0;  // position in the list
   if (SHARED) {
     if (threadIdx.x == 0) sm.claim = atomicAdd(claim, 1u);
     __syncthreads();
     li = sm.claim;
   } else {
-    if (lane == 0) {
-      li = atomicAdd(claim, 1u);
-      li_ahead = atomicAdd(claim, 1u);
-    }
+    if (lane == 0) li = atomicAdd(claim, 1u);
     li = __shfl_sync(kFull, li, 0);
   }
   uint32_t t = li < nlist ? tile_list[li] : ntiles;
@@ -345,11 +344,6 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   for (;;) {
     if (t >= ntiles) break;
     uint32_t t_next = ntiles, n_next = 0, off_next = 0;
-    if (!SHARED) {
-      const uint32_t li_next = __shfl_sync(kFull, li_ahead, 0);
-      if (lane == 0) li_ahead = li_next < nlist ? atomicAdd(claim, 1u) : nlist;
-      if (li_next < nlist) t_next = tile_list[li_next];
-    }
     const DView& v = views[vi];
     const int lt = (int)t - v.tile_base;
     const int tx = lt % v.tiles_x, ty = lt / v.tiles_x;
@@ -526,11 +520,6 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
       }
       if (qn) resolve(qn);  // before the next batch replaces the runs the queue points to
     }
-    // the next tile's list bounds: its number, asked for before this tile's records, has come by now
-    if (!SHARED && t_next < ntiles) {
-      n_next = sc.tile_count[t_next];
-      off_next = sc.tile_off[t_next];
-    }
     if (lane == 0) {
       if (v.dep0 >= 0 && v.dep0 != ready) wait_target(sc, views, v.dep0);
       if (v.dep1 >= 0) wait_tile(sc, views, v.dep1, lt);
@@ -592,6 +581,15 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
       sm.shaded[warp] += shaded;
       sm.frags[warp] += frags;
     }
+    if (!SHARED) {
+      if (lane == 0) li = atomicAdd(claim, 1u);
+      li = __shfl_sync(kFull, li, 0);
+      if (li < nlist) {
+        t_next = tile_list[li];
+        n_next = sc.tile_count[t_next];
+        off_next = sc.tile_off[t_next];
+      }
+    }
     // the next tile's view: at or behind this one
     auto view_of = [&](uint32_t tile) {
       if (tile >= ntiles) return -1;
@@ -635,7 +633,8 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
   }
 }
 
-// The list's tiles by warps, the last `shared` of them by CTAs.
+// The list's tiles by warps, or (`shared` of them: all or none) by CTAs.  Written as if both could run:
+// as one branch the compiler lays the loops out together, and the first one is 1-2 % slower.
 template <int T, int WARPS, bool HIDE>
 __device__ __forceinline__ void raster_list(const DView* __restrict__ views, const Scratch& sc, RasterSmem<T, WARPS>& sm,
                                             const int32_t* tbase, uint32_t nlist, uint32_t shared, const uint32_t* list) {
@@ -653,12 +652,6 @@ __device__ __forceinline__ void raster_list(const DView* __restrict__ views, con
 // the barriers cost: the two are equal at about 10 tiles per CTA (86 us each at 10.6) and one
 // warp per tile wins by 1.55x at 20 (113 against 176 us) and 1.7x at 47.
 constexpr uint32_t kSharedTilesPerCta = 4;
-// A longer list ends the same way: the warps that take its last tiles finish long after the others
-// have none left (a quarter of the warps' time of a 16-view batch).  There each CTA shares one of
-// the last gridDim.x tiles, where the lists hold at least kTailRecords records a tile on average:
-// 16 views (40 records a tile) 334 -> 315 us, 1000x600 with shadow (4.4) 70 -> 63 us, 1080p
-// frame (11) 195 -> 190 us; the 2560x1440 close-up (2.3) has nothing to share, 96 -> 99 us.
-constexpr unsigned long long kTailRecords = 3;
 
 // Four-warp CTAs are compiled for 7 per SM (72 registers a thread, fewer spills than at 8 per
 // SM's 64: measured faster on the serving batches, 1.72 -> 1.65 ms).
@@ -680,9 +673,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
     const uint32_t* list = sc.tile_list + lo;
     // uniform over the grid: every warp of every CTA has a stash, or none does
     const bool stashes = TileState<T * T>::kKeep || !sc.stash || gridDim.x * (uint32_t)WARPS <= sc.stash_warps;
-    // the tiles at the list's end that CTAs share
-    const bool long_lists = (unsigned long long)sc.ctl->bin_total >= kTailRecords * (unsigned long long)sc.ctl->ne_tiles;
-    const uint32_t shared = !stashes ? 0u : nlist <= kSharedTilesPerCta * gridDim.x ? nlist : long_lists ? gridDim.x : 0u;
+    const uint32_t shared = stashes && nlist <= kSharedTilesPerCta * gridDim.x ? nlist : 0u;
     if (sc.ctl->box_px < kHideCandidates * (float)(T * T) * (float)sc.ctl->ne_tiles)
       raster_list<T, WARPS, false>(views, sc, sm, tbase, nlist, shared, list);
     else
