@@ -361,12 +361,13 @@ __device__ __forceinline__ void rec_tiles(const RasterRec& r, int T, int& tx0, i
 // 4M-triangle soup 84 -> 68 / 170 -> 150 us, 1000x600 with shadow scatter 29 -> 22 us).
 // `even(most)`, where the lanes' counts are close to their maximum `most` (the sub-records of a split
 // triangle): the caller walks each lane's own tiles.
+// Several warps may hold the same records (`part` of `parts`) and take every parts-th step each.
 template <class F, class E>
-__device__ __forceinline__ void for_each_pair(int nt, int ntw, int tile0, int tiles_x, F f, E even) {
+__device__ __forceinline__ void for_each_pair(int nt, int ntw, int tile0, int tiles_x, F f, E even, int part = 0, int parts = 1) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   if (!__any_sync(kAll, nt > 1)) {
-    if (__any_sync(kAll, nt > 0)) f(nt > 0, tile0, lane);
+    if (part == 0 && __any_sync(kAll, nt > 0)) f(nt > 0, tile0, lane);
     return;
   }
   const int magic = (65535 + ntw) / ntw;  // k / ntw = (k * magic) >> 16 for k < 32, ntw <= 32
@@ -382,7 +383,7 @@ __device__ __forceinline__ void for_each_pair(int nt, int ntw, int tile0, int ti
     even(most);
     return;
   }
-  for (int base = 0; base < total; base += 32) {
+  for (int base = 32 * part; base < total; base += 32 * parts) {
     const int i = base + lane;
     int own = 0;  // records whose pairs end at or before pair i
 #pragma unroll
