@@ -1,17 +1,19 @@
 // hsr_internal.h — data layout shared by the host runtime and the sm_103a kernels.
 //
 // Pipeline of one launch sequence (a batch of views = draws):
-//   k_vertex  : SoA positions -> screen vertex per view (world attributes are transformed per
-//               corner where a triangle survives: k_emit, and the clipper)
-//   k_setup   : per face: fast accept or homogeneous clip (graphics.cpp:132-161), then per
-//               fan triangle divide / cull / viewport / bbox (graphics.cpp:314-347) -> one
-//               64-byte RasterRec, plus per-tile counts (warp-aggregated atomics)
-//   k_scan    : exclusive prefix sums of the per-tile counts and of the non-empty tiles
+//   k_prep    : view descriptors from the host's page-locked staging, counters to zero
+//   k_vertex  : (large sequences of shared vertices) SoA positions -> screen vertex per view (world
+//               attributes are transformed per corner where a triangle survives)
+//   k_setup   : per face: fast accept or the clip queue (graphics.cpp:132-161), divide / cull /
+//               viewport / bbox (graphics.cpp:314-347) -> one 64-byte RasterRec
+//   k_emit    : shading payloads and per-tile counts (warp-aggregated atomics) of the records; in
+//               sequences of up to 2^21 faces the same grid clips (larger ones: k_post after it)
+//   k_scan    : sub-records of triangles that touch many tiles, then exclusive prefix sums of the per-tile counts and of the non-empty tiles
 //               (decoupled look-back), and the list of non-empty tiles in tile order
 //   k_scatter : (record, tile) pairs into per-tile lists; beside it, in the same grid, the
 //               fused clear of the tiles no triangle touches, streamed row by row
-//   k_raster  : persistent over the non-empty tiles; one warp owns one screen tile,
-//               resolves visibility per pixel as min over (depth, later-submitted) — the
+//   k_raster  : persistent over the non-empty tiles; one warp owns one screen tile (a CTA
+//               where tiles are few), resolves visibility per pixel as min over (depth, later-submitted) — the
 //               sequential loop's result — then shades the winners and writes colour /
 //               depth / prim id once.
 #pragma once
@@ -166,6 +168,7 @@ struct Ctl {
   unsigned long long pay_bytes;  // shading payload bytes written (k_emit, k_post, k_scan)
 };
 static_assert(sizeof(Ctl) == 64, "Ctl is read back whole: keep it one 64-byte block");
+constexpr size_t kSplitWords = 128;  // Scratch::split, in the zeroed 256 bytes that hold Ctl, on a line of its own
 
 // A triangle whose bounding box touches more than kMaxRecordTiles tiles, queued by
 // the emit and clip passes and expanded into sub-records by k_scan.
@@ -196,7 +199,7 @@ struct Scratch {
   uint32_t* tile_off;       // [ntiles]
   uint32_t* ne_off;         // [ntiles + 1] non-empty tiles before each tile
   uint32_t* tile_list;      // [ntiles] the non-empty tiles in tile order (ne_tiles of them)
-  unsigned long long* split;        // parts of huge triangles split, their sub-records (two words behind scan_status)
+  unsigned long long* split;        // parts of huge triangles split, their sub-records (two words, kSplitWords bytes behind ctl)
   unsigned long long* scan_status;  // [scan blocks]
   uint32_t* bins;   uint32_t bin_cap;
   int32_t ntiles;
@@ -252,6 +255,6 @@ int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStr
 int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int clear_chunks, uint32_t plane_bytes,
                    cudaStream_t s);
 int launch_raster(const DView* views, int tile, Scratch sc, int grid, int warps, cudaStream_t s);
-int scan_words(int ntiles);  // 64-bit words of Scratch::scan_status
+int scan_blocks(int ntiles);
 
 }  // namespace hsr

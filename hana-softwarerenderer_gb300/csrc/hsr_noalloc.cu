@@ -122,7 +122,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   const size_t faces = (size_t)m->nfaces, tiles = (size_t)v.ntiles;
   const size_t rec_cap = faces + faces / 4 + 1024, clip_cap = faces / 16 + 256, big_cap = faces / 64 + 256;
   const size_t bin_cap = (size_t)(rt->tuning.bin_factor * (double)(faces + tiles)) + 4096;
-  const int nscan = scan_words((int)tiles);
+  const int nscan = scan_blocks((int)tiles);
   size_t off = 0;
   const size_t o_view = off; off = nal(off + sizeof(DView));
   const size_t host_bytes = off;
@@ -132,7 +132,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   const size_t o_done = off; off = nal(off + sizeof(uint32_t) * (1 + 2 + 1));
   const size_t o_cnt = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_fill = off; off = nal(off + sizeof(uint32_t) * tiles);
-  const size_t o_stat = off; off = nal(off + sizeof(unsigned long long) * (size_t)nscan);
+  const size_t o_stat = off; off = nal(off + sizeof(unsigned long long) * (size_t)std::max(nscan, 1));
   const size_t zero_bytes = off - o_zero;
   const size_t o_toff = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_neoff = off; off = nal(off + sizeof(uint32_t) * (tiles + 1));
@@ -164,7 +164,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   sc.ne_off = (uint32_t*)(dev + o_neoff);
   sc.tile_list = (uint32_t*)(dev + o_list);
   sc.scan_status = (unsigned long long*)(dev + o_stat);
-  sc.split = sc.scan_status + (nscan - 2);
+  sc.split = (unsigned long long*)(dev + o_ctl + kSplitWords);
   sc.bins = (uint32_t*)(dev + o_bins); sc.bin_cap = (uint32_t)bin_cap;
   sc.ntiles = (int32_t)tiles;
   sc.nviews = 1;

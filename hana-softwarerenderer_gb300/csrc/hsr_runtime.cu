@@ -2,8 +2,8 @@
 //
 // Replaces graphics_draw_triangle(DrawData*) (graphics.h:15, graphics.cpp:378-407) by
 // handle-based calls.  Meshes, textures and targets live in device memory; hsr_draw_batch
-// turns a list of draws into one launch sequence of eight kernels (vertex, cull, emit, clip,
-// split, scan, scatter, raster) over all of them, or into several in array order where a draw
+// turns a list of draws into one launch sequence (set-up, [vertex], cull, emit, [clip], scan, scatter,
+// raster) over all of them, or into several in array order where a draw
 // clears a target an earlier draw of the list writes.  Scratch is a grow-only arena; an
 // overflow detected on the device
 // leaves the targets untouched (the raster checks the error word first) and the batch is
@@ -264,7 +264,7 @@ void Plan::layout() {
   clip_cap = std::min<size_t>(clip_cap, 0xfffff000u);
   big_cap = std::min<size_t>(big_cap, 0xfffff000u);
   bin_cap = std::min<size_t>(bin_cap, 0xfffff000u);
-  nscan = scan_words((int)total_tiles);
+  nscan = scan_blocks((int)total_tiles);
   // [views | chunks | per-view vertex outputs | ctl | view_done | tile_count | tile_fill |
   //  scan_status | tile_off | ne_off | tile_list | recs | clipbuf | bins]; the zeroed part is one memset
   size_t off = 0;
@@ -276,7 +276,7 @@ void Plan::layout() {
   o_done = off; off = align_up(off + sizeof(uint32_t) * ((size_t)n + 2 * kRasterGroups + 1), 256);
   o_cnt = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_fill = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
-  o_stat = off; off = align_up(off + sizeof(unsigned long long) * nscan, 256);
+  o_stat = off; off = align_up(off + sizeof(unsigned long long) * std::max(nscan, 1), 256);
   zero_bytes = off - o_zero;
   o_toff = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_neoff = off; off = align_up(off + sizeof(uint32_t) * (total_tiles + 1), 256);
@@ -311,7 +311,7 @@ void Plan::bind(char* dev_base, char* host_base) {
   sc.ne_off = (uint32_t*)(dev + o_neoff);
   sc.tile_list = (uint32_t*)(dev + o_list);
   sc.scan_status = (unsigned long long*)(dev + o_stat);
-  sc.split = sc.scan_status + (nscan - 2);
+  sc.split = (unsigned long long*)(dev + o_ctl + kSplitWords);
   sc.bins = (uint32_t*)(dev + o_bins); sc.bin_cap = (uint32_t)bin_cap;
   sc.ntiles = (int32_t)total_tiles;
   sc.nviews = n;

@@ -27,7 +27,7 @@ constexpr unsigned long long kFlagPre = 2ull << 62;
 constexpr unsigned long long kValMask = (1ull << 62) - 1;
 
 __host__ __device__ __forceinline__ int scan_blocks_hd(int ntiles) { return (ntiles + kScanTile - 1) / kScanTile; }
-int scan_words(int ntiles) { return scan_blocks_hd(ntiles) + 2; }  // and Scratch::split
+int scan_blocks(int ntiles) { return scan_blocks_hd(ntiles); }
 
 __device__ __forceinline__ unsigned long long ld_volatile64(const unsigned long long* p) {
   return *reinterpret_cast<const volatile unsigned long long*>(p);

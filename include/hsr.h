@@ -292,8 +292,8 @@ HSR_API int hsr_get_stats(hsr_stats* out);
  * hsr_plan_create validates the draws (same rules as hsr_draw_batch; a plan is one launch
  * sequence, so a draw that clears a target an earlier draw of the plan writes is refused with
  * HSR_ERR_INVALID_ARG), reserves the plan's own scratch, and records the whole launch sequence
- * (descriptors and counters, then the eight kernels of the timing block) into a CUDA graph.  Between replays only uniforms may change
- * (hsr_plan_set_uniforms); meshes, textures, targets and shaders stay those of creation.
+ * (descriptors and counters, then the kernels of the timing block) into a CUDA graph.  Between
+ * replays only uniforms may change (hsr_plan_set_uniforms); meshes, textures, targets and shaders stay those of creation.
  * hsr_plan_launch replays the graph on the library stream and returns at once;
  * hsr_plan_wait blocks until it is done and re-runs it with larger scratch if the device
  * reported an overflow (the targets are left untouched by an overflowing run). */
