@@ -26,7 +26,11 @@
 
 namespace hsr {
 
-constexpr int kMaxPoly = 10;              // 3 vertices + one per clip plane (7 planes)
+// Vertices of a clipped polygon: 3 + one per clip plane (7) in exact arithmetic, more where rounding
+// bends a polygon that lies along a corner line of the frustum (12 seen).  Vertices past the last
+// place are dropped.
+constexpr int kMaxPoly = 16;
+constexpr int kMaxMeshFaces = 1 << 27;    // hsr_mesh_upload refuses more
 constexpr int kVaryings = 13;             // floats in shader_struct_v2f (IShader.h:41-47)
 constexpr int kMaxRecordTiles = 32;       // records never touch more tiles (big ones are split)
 constexpr int kSubTilesX = 8, kSubTilesY = 4;  // tile block of one sub-record
@@ -66,7 +70,7 @@ struct __align__(16) RasterRec {
   float d1, d2;             // screen depths of B, C
   uint32_t face;            // position of the face in the mesh's face arrays (cull pass's records)
   uint32_t pad;             // reserved (zero)
-  uint32_t seq;             // (face << 4) | (fan << 1) | clipped — submission order
+  uint32_t seq;             // (face << kSeqFaceShift) | (fan << 1) | clipped — submission order
   uint32_t view;            // index of the view in the batch | flags << 28 (kRec*)
   uint32_t xr, yr;          // inclusive pixel range: x0 | x1 << 16, y0 | y1 << 16
 };
@@ -83,6 +87,11 @@ constexpr int kRecFlagShift = 28;
 struct __align__(16) Payload {
   float f[kPayloadFloats];
 };
+constexpr int kSeqFaceShift = 5;
+static_assert(kMaxPoly - 2 <= 1 << (kSeqFaceShift - 1), "the fan index must not reach the face's bits");
+// (below 2^32 - 1: the raster's keys hold 0xfffffffe - seq, and 0xffffffff stands for the buffer's depth)
+static_assert(((uint64_t)kMaxMeshFaces << kSeqFaceShift) - (1u << kSeqFaceShift) + 2 * (kMaxPoly - 3) + 1 <= 0xfffffffeull,
+              "submission words must fit 32 bits");
 static_assert(sizeof(RasterRec) == 64, "RasterRec must stay 64 bytes");
 
 // Per-draw descriptor on the device.  The fields every raster tile reads come first, in

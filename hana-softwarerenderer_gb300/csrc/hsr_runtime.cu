@@ -682,7 +682,7 @@ int hsr_mesh_upload(const float* pos, int32_t npos, const float* nrm, int32_t nn
                     const int32_t* faces, int32_t nfaces, hsr_mesh* out) {
   RT_OR_FAIL();
   if (!out || npos < 0 || nnrm < 0 || nuv < 0 || nfaces < 0) return fail(HSR_ERR_INVALID_ARG, "mesh: bad arguments");
-  if (nfaces > (1 << 27)) return fail(HSR_ERR_INVALID_ARG, "mesh: more than 2^27 faces");
+  if (nfaces > kMaxMeshFaces) return fail(HSR_ERR_INVALID_ARG, "mesh: more than 2^27 faces");
   if ((npos && !pos) || (nnrm && !nrm) || (nuv && !uv) || (nfaces && !faces))
     return fail(HSR_ERR_INVALID_ARG, "mesh: null array with nonzero count");
   bool unified = true;  // every corner has equal v, vt and vn indices

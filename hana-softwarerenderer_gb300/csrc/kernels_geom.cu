@@ -678,7 +678,7 @@ __device__ __forceinline__ void cull_face(const DView& v, int f, uint32_t view, 
   }
   if (accept)
     valid = build_rec(v, {sv[0].x, sv[0].y, sv[0].z}, {sv[1].x, sv[1].y, sv[1].z}, {sv[2].x, sv[2].y, sv[2].z},
-                      (uint32_t)iv.w << 4, view, r);
+                      (uint32_t)iv.w << kSeqFaceShift, view, r);
   r.face = (uint32_t)f;
 }
 
@@ -815,12 +815,12 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
         const float* prev = src + (i == 0 ? n - 1 : i - 1) * kPolyStride;
         const float* curr = src + i * kPolyStride;
         const bool pin = inside_plane(prev, plane), cin = inside_plane(curr, plane);
-        if (pin != cin) {
+        if (pin != cin && m < kMaxPoly) {
           const float t = intersect_ratio(prev, curr, plane);
           if (hl < kVaryings) dst[m * kPolyStride + hl] = fa(prev[hl], fm(fs(curr[hl], prev[hl]), t));
           m++;
         }
-        if (cin) {
+        if (cin && m < kMaxPoly) {
           if (hl < kVaryings) dst[m * kPolyStride + hl] = curr[hl];
           m++;
         }
@@ -837,9 +837,9 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
     const float* p0 = src;
     const float* p1 = src + (hl + 1) * kPolyStride;
     const float* p2 = src + (hl + 2) * kPolyStride;
+    const uint32_t seq = ((uint32_t)__ldg(&v.fv[face].w) << kSeqFaceShift) | ((uint32_t)hl << 1) | 1u;
     valid = build_rec(v, ndc_of(make_float4(p0[0], p0[1], p0[2], p0[3])), ndc_of(make_float4(p1[0], p1[1], p1[2], p1[3])),
-                      ndc_of(make_float4(p2[0], p2[1], p2[2], p2[3])), ((uint32_t)__ldg(&v.fv[face].w) << 4) | ((uint32_t)hl << 1) | 1u,
-                      (uint32_t)view, r);
+                      ndc_of(make_float4(p2[0], p2[1], p2[2], p2[3])), seq, (uint32_t)view, r);
     if (valid) make_payload(v.shader, p0, p1, p2, pl);
   }
   int tx0, ty0, ntw, nt = 0;

@@ -252,7 +252,7 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 #pragma unroll
         for (int k = 0; k < NF4; k++) reinterpret_cast<float4*>(P)[k] = src[k];
       }
-      const uint32_t prim = v.prim_base + (seq >> 4) + 1u;
+      const uint32_t prim = v.prim_base + (seq >> kSeqFaceShift) + 1u;
       const uint32_t alpha = clear ? v.clear_rgba : __ldcg(&v.color[idx]);
       v.color[idx] = pack_rgb(fragment_s<S>(v, P, b0, b1, b2, prim, bt), alpha);
       if (v.depth) v.depth[idx] = from_ord(st.z[p]);

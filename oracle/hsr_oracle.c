@@ -9,9 +9,11 @@
  * the GPU path:
  *   - float -> int conversions follow x86 cvttss2si: truncation, INT_MIN when the value
  *     is NaN or out of range (texture coordinates, bounding-box start);
- *   - the homogeneous clipper gets ping-pong buffers large enough for 10 vertices (the
- *     reference writes the odd planes' output into a 3-element array, graphics.cpp:379
- *     with :153,:155,:157);
+ *   - the homogeneous clipper gets ping-pong buffers of MAX_POLY vertices (the reference
+ *     writes the odd planes' output into a 3-element array, graphics.cpp:379 with
+ *     :153,:155,:157).  Exact arithmetic makes at most 10, rounding more (a polygon along
+ *     a corner line of the frustum is cut more than twice by one plane); vertices past
+ *     the last place are dropped;
  *   - is_in_shadow treats a NaN light-space position as lit (the reference would index
  *     the shadow map with (int)NaN).
  */
@@ -28,6 +30,7 @@
 
 #define EPSILON 1e-5f /* maths.h:6 */
 #define NV 13         /* floats in shader_struct_v2f (IShader.h:41-47) */
+#define MAX_POLY 16   /* vertices of a clipped polygon */
 
 typedef struct { float x, y; } v2;
 typedef struct { float x, y, z; } v3;
@@ -357,23 +360,26 @@ static int clip_against_plane(int plane, int n, const v2f* in, v2f* out) { /* :7
     int cin = is_inside_plane(curr->f, plane);
     if (pin != cin) {
       float t = intersect_ratio(prev->f, curr->f, plane);
-      for (int k = 0; k < NV; k++) out[m].f[k] = prev->f[k] + (curr->f[k] - prev->f[k]) * t; /* :7-17 */
-      m++;
+      if (m < MAX_POLY) {
+        for (int k = 0; k < NV; k++) out[m].f[k] = prev->f[k] + (curr->f[k] - prev->f[k]) * t; /* :7-17 */
+        m++;
+      }
     }
-    if (cin) out[m++] = *curr;
+    if (cin && m < MAX_POLY) out[m++] = *curr;
   }
   return m;
 }
 static int is_vertex_visible(const float* c) { /* :132-134 */
   return fabsf(c[0]) <= c[3] && fabsf(c[1]) <= c[3] && fabsf(c[2]) <= c[3];
 }
-/* clip_triangle (:136-161); poly receives the result, at most 10 vertices. */
-static int clip_triangle(const v2f* tri, v2f* poly) {
+/* clip_triangle (:136-161); poly receives the result, at most MAX_POLY vertices, and counts (may
+ * be NULL) the number of vertices after each plane (0 for the planes after a dropped polygon). */
+static int clip_triangle(const v2f* tri, v2f* poly, int32_t* counts) {
   if (is_vertex_visible(tri[0].f) && is_vertex_visible(tri[1].f) && is_vertex_visible(tri[2].f)) {
     poly[0] = tri[0]; poly[1] = tri[1]; poly[2] = tri[2];
     return 3;
   }
-  v2f a[16], b[16];
+  v2f a[MAX_POLY], b[MAX_POLY];
   a[0] = tri[0]; a[1] = tri[1]; a[2] = tri[2];
   int n = 3;
   static const int planes[7] = {PW, PX, NX, PY, NY, PZ, NZ};
@@ -381,6 +387,7 @@ static int clip_triangle(const v2f* tri, v2f* poly) {
   v2f* dst = b;
   for (int k = 0; k < 7; k++) {
     n = clip_against_plane(planes[k], n, src, dst);
+    if (counts) counts[k] = n;
     if (n < 3) return 0;
     v2f* t = src; src = dst; dst = t;
   }
@@ -481,7 +488,7 @@ static int draw_mesh(const hsro_mesh* mesh, int32_t shader, const hsr_shader_dat
    * for every corner, so computing it once gives the same bits. */
   mat_mul(shader == HSR_SHADER_SHADOW ? sd->light_vp_matrix : sd->camera_vp_matrix,
           sd->model_matrix, c.mvp);
-  v2f tri[3], poly[10];
+  v2f tri[3], poly[MAX_POLY];
   for (int32_t i = 0; i < mesh->nfaces; i++) {
     for (int j = 0; j < 3; j++) {
       const int32_t* corner = &mesh->faces[((size_t)i * 3 + (size_t)j) * 3];
@@ -495,13 +502,21 @@ static int draw_mesh(const hsro_mesh* mesh, int32_t shader, const hsr_shader_dat
       }
       tri[j] = vertex(&c, p, n, uv);
     }
-    int nv = clip_triangle(tri, poly);
+    int nv = clip_triangle(tri, poly, NULL);
     for (int j = 0; j < nv - 2; j++) {
       v2f t[3] = {poly[0], poly[j + 1], poly[j + 2]};
       rasterize_triangle(&c, t, prim_base + (uint32_t)i + 1u);
     }
   }
   return 0;
+}
+
+void hsro_clip_counts(const float clip[12], int32_t counts[7]) {
+  v2f tri[3], poly[MAX_POLY];
+  memset(tri, 0, sizeof(tri));
+  for (int j = 0; j < 3; j++) memcpy(tri[j].f, clip + 4 * j, 4 * sizeof(float));
+  for (int k = 0; k < 7; k++) counts[k] = 0;
+  clip_triangle(tri, poly, counts);
 }
 
 int hsro_draw(const hsro_mesh* mesh, int32_t shader, const hsr_shader_data* sd,

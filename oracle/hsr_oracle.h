@@ -49,6 +49,10 @@ int hsro_draw_stored_normals(const hsro_mesh* mesh, int32_t shader, const hsr_sh
                              const hsro_texture* diffuse, const hsro_texture* normal,
                              const hsro_target* shadow_map, hsro_target* target, uint32_t prim_base);
 
+/* Vertices of a triangle's polygon after each clip plane, from the corners' clip positions
+ * (x, y, z, w each); all 0 where the triangle is wholly visible and is not clipped. */
+void hsro_clip_counts(const float clip[12], int32_t counts[7]);
+
 /* renderbuffer_clear_color / renderbuffer_clear_depth with explicit bytes; prim -> 0. */
 void hsro_clear(hsro_target* t, const uint8_t rgba[4], float depth);
 

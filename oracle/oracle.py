@@ -57,6 +57,8 @@ def lib():
                                         ctypes.POINTER(_Tex), ctypes.POINTER(_Tex),
                                         ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                         ctypes.c_int32, ctypes.c_int32]
+        L.hsro_clip_counts.restype = None
+        L.hsro_clip_counts.argtypes = [_f32p, _i32p]
         L.hsro_no_contraction.restype = ctypes.c_int
         if not L.hsro_no_contraction():
             raise RuntimeError("liboracle.so was built with floating-point contraction")
@@ -116,6 +118,15 @@ def draw(mesh, shader: int, sd: np.ndarray, target: Buffers, diffuse=None, norma
     if rc != 0:
         raise ValueError(f"hsro_draw failed ({rc})")
     del keep
+
+
+def clip_counts(clip) -> np.ndarray:
+    """Vertices after each of the seven clip planes, for [n][3][4] clip positions -> [n][7]."""
+    c = np.ascontiguousarray(clip, np.float32).reshape(-1, 12)
+    out = np.zeros((len(c), 7), np.int32)
+    for a, b in zip(c, out):
+        lib().hsro_clip_counts(a.ctypes.data_as(_f32p), b.ctypes.data_as(_i32p))
+    return out
 
 
 def render_frame(frame) -> dict:
