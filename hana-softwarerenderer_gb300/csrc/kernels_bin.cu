@@ -69,7 +69,7 @@ int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t 
 // still tested exactly once.  `parts` warps share the triangle.  Returns a lane's number of tiles.
 // (A warp and not a CTA each: most queued triangles have some tens of tiles, and what takes the time
 // is the chain of loads from the queue to the view.)
-__device__ __forceinline__ uint32_t split_triangle(const DView* __restrict__ views, int T, const Scratch& sc, const BigItem& bi,
+__device__ __forceinline__ uint32_t split_triangle(const DView* views, int T, const Scratch& sc, const BigItem& bi,
                                                    uint32_t first, int part, int parts) {
   const RasterRec b = bi.rec;
   const DView& v = views[b.view & kRecViewMask];
@@ -119,7 +119,7 @@ __device__ __forceinline__ uint32_t split_triangle(const DView* __restrict__ vie
 constexpr uint32_t kMaxParts = 256;
 constexpr uint32_t kScanWarps = kScanThreads / 32;
 constexpr uint32_t kStepsToReport = 4096;  // a splitter reports at least every few milliseconds
-__global__ void __launch_bounds__(kScanThreads) k_scan(const DView* __restrict__ views, int T, Scratch sc, uint32_t splitters) {
+__global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T, Scratch sc, uint32_t splitters) {
   __shared__ unsigned long long warp_sums[kScanThreads / 32];
   __shared__ unsigned long long s_prefix;
   __shared__ uint32_t s_block;
@@ -284,7 +284,7 @@ int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStr
 // with an atomic's round trip (1000x600 with shadow, 3,779 records of 15 tiles each: 22.5 -> 12.3 us, 2560x1440
 // close-up 16.4 -> 10.2 us; a quarter million records and more keep their warps to themselves).
 constexpr uint32_t kMaxSharers = 16;
-__device__ __forceinline__ void scatter_records(const DView* __restrict__ views, int T, const Scratch& sc, uint32_t block,
+__device__ __forceinline__ void scatter_records(const DView* views, int T, const Scratch& sc, uint32_t block,
                                                 uint32_t nblocks) {
   const int lane = threadIdx.x & 31;
   const uint32_t nrec = min(sc.ctl->rec_count + sc.ctl->rec_extra, sc.rec_cap);
@@ -363,7 +363,7 @@ __device__ __forceinline__ void scatter_records(const DView* __restrict__ views,
 // to T neighbours) decides whether it is written.
 // Block `block` of the `nblocks` clearing blocks takes chunks warp by warp; `cbase` holds the
 // views' chunk bases when the batch has at most kSharedViews views (else null).
-__device__ __forceinline__ void clear_empty_tiles(const DView* __restrict__ views, int T, int nchunks, const Scratch& sc,
+__device__ __forceinline__ void clear_empty_tiles(const DView* views, int T, int nchunks, const Scratch& sc,
                                                   int block, int nblocks, const int32_t* cbase) {
   if (sc.ctl->error & kErrNoDraw) return;  // an overflowing or stalled sequence draws nothing
   const int ts = __ffs(T) - 1;
@@ -446,7 +446,7 @@ __device__ __forceinline__ void clear_empty_tiles(const DView* __restrict__ view
 constexpr int kClearMinBlocks = 3;
 constexpr unsigned long long kClearHeavy = 10;  // pixels of three planes per pair
 
-__global__ void __launch_bounds__(256) k_scatter(const DView* __restrict__ views, int T, Scratch sc, int nchunks,
+__global__ void __launch_bounds__(256) k_scatter(const DView* views, int T, Scratch sc, int nchunks,
                                                  uint32_t plane_bytes) {
   __shared__ int32_t s_cbase[kSharedViews];
   const uint32_t b = blockIdx.x, g = gridDim.x;

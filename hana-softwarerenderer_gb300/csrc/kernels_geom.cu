@@ -402,7 +402,7 @@ __device__ __forceinline__ void vertex_chunk_work(const DView& v, const Chunk& c
 }
 
 // One block per chunk (the blocks are short and many: their prologues overlap others' work).
-__global__ void __launch_bounds__(256) k_vertex(const DView* __restrict__ views, int nviews) {
+__global__ void __launch_bounds__(256) k_vertex(const DView* views, int nviews) {
   __shared__ int32_t s_base[kSharedViews];
   chain_wait();
   const int32_t* base = share_bases(views, nviews, s_base, VchBase());
@@ -660,7 +660,7 @@ __device__ __forceinline__ void cull_face(const DView& v, int f, uint32_t view, 
   const int pi[3] = {iv.x, iv.y, iv.z};
   float4 sv[3];
 #pragma unroll
-  for (int k = 0; k < 3; k++) sv[k] = OWN ? screen_vertex(clip_of(v, pi[k])) : __ldg(&v.sv[pi[k]]);
+  for (int k = 0; k < 3; k++) sv[k] = OWN ? screen_vertex(clip_of(v, pi[k])) : v.sv[pi[k]];
   bool accept = sv_normal(sv[0]) && sv_normal(sv[1]) && sv_normal(sv[2]);
   if (!accept) {
     const uint32_t m0 = sv_mask(sv[0]), m1 = sv_mask(sv[1]), m2 = sv_mask(sv[2]);
@@ -683,7 +683,7 @@ __device__ __forceinline__ void cull_face(const DView& v, int f, uint32_t view, 
 }
 
 template <bool OWN>
-__global__ void __launch_bounds__(kSetupThreads, 8) k_setup(const DView* __restrict__ views, int nviews,
+__global__ void __launch_bounds__(kSetupThreads, 8) k_setup(const DView* views, int nviews,
                                                          int nchunks, Scratch sc) {
   __shared__ int32_t s_base[kSharedViews];
   chain_wait();
@@ -858,7 +858,7 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
 // shading payload, the tile counts, and the hand-over of huge triangles to k_scan (their
 // slot becomes a hole the binning skips).  Grid-stride with warp-uniform trip counts, so
 // the warp collectives of append_small see every lane.
-__device__ __forceinline__ void emit_records(const DView* __restrict__ views, int T, const Scratch& sc, uint32_t block,
+__device__ __forceinline__ void emit_records(const DView* views, int T, const Scratch& sc, uint32_t block,
                                              uint32_t nblocks) {
   const int lane = threadIdx.x & 31;
   const uint32_t nrec = min(sc.ctl->rec_count, sc.rec_cap);
@@ -933,7 +933,7 @@ __device__ __forceinline__ void emit_records(const DView* __restrict__ views, in
 // leaves some warps with the faces that make many triangles: 65k faces 100 us, claimed 88 us;
 // without claims and their round trip a short queue saves 2-8 us).  Each face is a chain of
 // dependent loads, so resident warps set the throughput.
-__device__ __forceinline__ void clip_queue(const DView* __restrict__ views, int T, const Scratch& sc, uint32_t block,
+__device__ __forceinline__ void clip_queue(const DView* views, int T, const Scratch& sc, uint32_t block,
                                            uint32_t nblocks) {
   __shared__ float poly[kEmitThreads / 32][2][2][kMaxPoly * kPolyStride];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
@@ -960,7 +960,7 @@ __device__ __forceinline__ void clip_queue(const DView* __restrict__ views, int 
 // behind the cull pass's, counted apart).  CLIP: one grid, whose first `clip_blocks` blocks clip
 // while the others emit; otherwise the grid emits, and k_post clips after it.
 template <bool CLIP>
-__global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* __restrict__ views, int T, Scratch sc,
+__global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* views, int T, Scratch sc,
                                                           int clip_blocks) {
   chain_wait();
   if (sc.ctl->error & kErrCapacity) return;
@@ -972,7 +972,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* __restric
   emit_records(views, T, sc, blockIdx.x - first, gridDim.x - first);
 }
 
-__global__ void __launch_bounds__(kEmitThreads, 3) k_post(const DView* __restrict__ views, int T, Scratch sc) {
+__global__ void __launch_bounds__(kEmitThreads, 3) k_post(const DView* views, int T, Scratch sc) {
   chain_wait();
   if (sc.ctl->error & kErrCapacity) return;
   clip_queue(views, T, sc, blockIdx.x, gridDim.x);

@@ -293,7 +293,7 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 // never matters), and the pixel rows are shaded by the warps in turn.
 // HIDE: see kHideCandidates.
 template <int T, int WARPS, bool SHARED, bool HIDE>
-__device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, const Scratch& sc,
+__device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& sc,
                                              RasterSmem<T, WARPS>& sm, const int32_t* tbase, uint32_t nlist,
                                              const uint32_t* tile_list, uint32_t* claim) {
   constexpr int NPIX = T * T;
@@ -636,7 +636,7 @@ __device__ __forceinline__ void raster_tiles(const DView* __restrict__ views, co
 // The list's tiles by warps, or (`shared` of them: all or none) by CTAs.  Written as if both could run:
 // as one branch the compiler lays the loops out together, and the first one is 1-2 % slower.
 template <int T, int WARPS, bool HIDE>
-__device__ __forceinline__ void raster_list(const DView* __restrict__ views, const Scratch& sc, RasterSmem<T, WARPS>& sm,
+__device__ __forceinline__ void raster_list(const DView* views, const Scratch& sc, RasterSmem<T, WARPS>& sm,
                                             const int32_t* tbase, uint32_t nlist, uint32_t shared, const uint32_t* list) {
   if (shared < nlist) raster_tiles<T, WARPS, false, HIDE>(views, sc, sm, tbase, nlist - shared, list, sc.claim);
   if (shared > 0u) {
@@ -656,7 +656,7 @@ constexpr uint32_t kSharedTilesPerCta = 4;
 // Four-warp CTAs are compiled for 7 per SM (72 registers a thread, fewer spills than at 8 per
 // SM's 64: measured faster on the serving batches, 1.72 -> 1.65 ms).
 template <int T, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_raster(const DView* __restrict__ views, Scratch sc) {
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_raster(const DView* views, Scratch sc) {
   extern __shared__ __align__(16) unsigned char raster_smem[];
   RasterSmem<T, WARPS>& sm = *reinterpret_cast<RasterSmem<T, WARPS>*>(raster_smem);
   build_byte_tables(sm.u8f);
