@@ -963,7 +963,9 @@ template <bool CLIP>
 __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const DView* views, int T, Scratch sc,
                                                           int clip_blocks) {
   chain_wait();
-  if (sc.ctl->error & kErrCapacity) return;
+  // as one block: another block of this grid may set the word meanwhile, and the blocks that emit meet
+  // at a barrier
+  if (__syncthreads_or((sc.ctl->error & kErrCapacity) != 0u)) return;
   if (CLIP && (int)blockIdx.x < clip_blocks) {
     clip_queue(views, T, sc, blockIdx.x, (uint32_t)clip_blocks);
     return;

@@ -32,3 +32,11 @@ def test_read_only_loads_are_of_meshes_and_textures():
     for name in ("kernels_geom.cu", "kernels_bin.cu", "kernels_raster.cu", "hsr_device.cuh"):
         for at in re.findall(r"__ldg\(([^()]*(?:\[[^\]]*\])?)", SRC[name]):
             assert set(re.findall(r"\w+", at)) & STATIC and "sv" not in re.findall(r"\w+", at), (name, at)
+
+
+def test_emit_leaves_on_an_overflow_as_one_block():
+    """Clipping blocks set the error word while emitting blocks of the same grid begin; those add up
+    their warps' sums behind a barrier, so their warps must not part over it."""
+    body = re.search(r"k_emit\(const DView\* views.*?\n}\n", SRC["kernels_geom.cu"], re.S).group(0)
+    assert re.search(r"if \(__syncthreads_or\(\(sc\.ctl->error & kErrCapacity\) != 0u\)\) return;", body)
+    assert body.count("ctl->error") == 1
