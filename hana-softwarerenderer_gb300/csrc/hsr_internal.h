@@ -233,6 +233,13 @@ __host__ __device__ constexpr int stash_floats(int tile) { return 4 * tile * til
 constexpr int kRasterGroups = 4;  // raster launches of one sequence at most
 constexpr int kStashWarpsPerSm = 32;  // raster warps resident per SM at most
 
+// Blocks of 256 threads that walk a mesh array of n items.  (The walks count in 64 bits: an array may
+// have up to 2^31 - 1 items, and an int would wrap on the last step.)
+inline int item_blocks(int n) {
+  const size_t want = ((size_t)(n > 0 ? n : 1) + 255) / 256;
+  return (int)(want < 4096 ? want : 4096);
+}
+
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.
 // `from` is mapped host memory or device memory; sizes are multiples of 16.
 // The order a mesh is kept in (see k_place_positions): raw device copies of the caller's arrays in,

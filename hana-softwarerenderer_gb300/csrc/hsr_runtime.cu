@@ -504,7 +504,7 @@ int Runtime::run_sequence(const hsr_draw_desc* descs, int n) {
 // where an array is shorter), so a corner's attributes are one 32-byte sector.
 __global__ void k_pack_vertices(float4* __restrict__ pk, const float4* __restrict__ p4, const uint32_t* __restrict__ vorder,
                                 const float4* __restrict__ n4, const float2* __restrict__ uv, int npos, int nnrm, int nuv) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npos; i += gridDim.x * blockDim.x) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)npos; i += (size_t)gridDim.x * blockDim.x) {
     const float4 p = p4[i];
     const int o = (int)vorder[i];
     const float4 n = o < nnrm ? n4[o] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -517,7 +517,7 @@ __global__ void k_pack_vertices(float4* __restrict__ pk, const float4* __restric
 int launch_pack_vertices(float4* pk, const float4* p4, const uint32_t* vorder, const float4* n4, const float2* uv,
                          int npos, int nnrm, int nuv, cudaStream_t s) {
   if (npos <= 0) return 0;
-  k_pack_vertices<<<std::min((npos + 255) / 256, 4096), 256, 0, s>>>(pk, p4, vorder, n4, uv, npos, nnrm, nuv);
+  k_pack_vertices<<<item_blocks(npos), 256, 0, s>>>(pk, p4, vorder, n4, uv, npos, nnrm, nuv);
   return (int)cudaGetLastError();
 }
 

@@ -198,10 +198,10 @@ __global__ void k_bounds_init(int* bounds) {
 // bounds[0..2] minima, [3..5] maxima of the finite coordinates, as ordered ints.
 __global__ void __launch_bounds__(256) k_bounds(const float* __restrict__ pos, int n, int* __restrict__ bounds) {
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      const float c = pos[3 * (size_t)i + k];
+      const float c = pos[3 * i + k];
       if (fabsf(c) <= FLT_MAX) {
         lo[k] = fminf(lo[k], c);
         hi[k] = fmaxf(hi[k], c);
@@ -239,15 +239,15 @@ __device__ __forceinline__ uint32_t cell_of(const int* __restrict__ bounds, cons
 __global__ void __launch_bounds__(256) k_cells(const float* __restrict__ pos, const int32_t* __restrict__ faces, int n,
                                                const int* __restrict__ bounds, uint32_t* __restrict__ cells,
                                                uint32_t* __restrict__ codes) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
     float m[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       if (faces) {
-        const int32_t* f = faces + 9 * (size_t)i;
+        const int32_t* f = faces + 9 * i;
         m[k] = (pos[3 * (size_t)f[0] + k] + pos[3 * (size_t)f[3] + k] + pos[3 * (size_t)f[6] + k]) / 3.f;
       } else {
-        m[k] = pos[3 * (size_t)i + k];
+        m[k] = pos[3 * i + k];
       }
     }
     codes[i] = cell_of(bounds, m);
@@ -304,9 +304,9 @@ __global__ void __launch_bounds__(256) k_place_positions(const float* __restrict
                                                          float* __restrict__ py, float* __restrict__ pz,
                                                          float4* __restrict__ p4, uint32_t* __restrict__ vorder,
                                                          uint32_t* __restrict__ place) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
     const uint32_t at = cells ? atomicAdd(&cells[codes[i]], 1u) : (uint32_t)i;
-    const float x = pos[3 * (size_t)i], y = pos[3 * (size_t)i + 1], z = pos[3 * (size_t)i + 2];
+    const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
     px[at] = x;
     py[at] = y;
     pz[at] = z;
@@ -319,17 +319,17 @@ __global__ void __launch_bounds__(256) k_place_positions(const float* __restrict
 __global__ void __launch_bounds__(256) k_place_faces(const int32_t* __restrict__ faces, int n, uint32_t* __restrict__ cells,
                                                      const uint32_t* __restrict__ codes, const uint32_t* __restrict__ place,
                                                      int4* __restrict__ fv, int4* __restrict__ fvt, int4* __restrict__ fvn) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
     const uint32_t at = cells ? atomicAdd(&cells[codes[i]], 1u) : (uint32_t)i;
-    const int32_t* r = faces + 9 * (size_t)i;
-    fv[at] = make_int4((int)place[r[0]], (int)place[r[3]], (int)place[r[6]], i);
+    const int32_t* r = faces + 9 * i;
+    fv[at] = make_int4((int)place[r[0]], (int)place[r[3]], (int)place[r[6]], (int)i);
     fvt[at] = make_int4(r[1], r[4], r[7], 0);
     fvn[at] = make_int4(r[2], r[5], r[8], 0);
   }
 }
 
 int launch_mesh_order(const MeshOrder& o, cudaStream_t s) {
-  const int pg = std::max(1, std::min((o.npos + 255) / 256, 4096)), fg = std::max(1, std::min((o.nfaces + 255) / 256, 4096));
+  const int pg = item_blocks(o.npos), fg = item_blocks(o.nfaces);
   const bool sorted = o.nfaces >= kOrderedFaces;
   int* bounds = reinterpret_cast<int*>(o.cells + kMeshCells);
   auto group = [&](const int32_t* faces, int n, int grid) {
@@ -359,8 +359,8 @@ int launch_mesh_order(const MeshOrder& o, cudaStream_t s) {
 __global__ void __launch_bounds__(256) k_split_normals(const float* __restrict__ nrm, int n, float* __restrict__ nx,
                                                        float* __restrict__ ny, float* __restrict__ nz,
                                                        float4* __restrict__ n4) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float x = nrm[3 * (size_t)i], y = nrm[3 * (size_t)i + 1], z = nrm[3 * (size_t)i + 2];
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
+    const float x = nrm[3 * i], y = nrm[3 * i + 1], z = nrm[3 * i + 2];
     nx[i] = x;
     ny[i] = y;
     nz[i] = z;
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(256) k_split_normals(const float* __restrict__
 }
 int launch_split_normals(const float* nrm, int n, float* nx, float* ny, float* nz, float4* n4, cudaStream_t s) {
   if (n <= 0) return 0;
-  k_split_normals<<<std::min((n + 255) / 256, 4096), 256, 0, s>>>(nrm, n, nx, ny, nz, n4);
+  k_split_normals<<<item_blocks(n), 256, 0, s>>>(nrm, n, nx, ny, nz, n4);
   return (int)cudaGetLastError();
 }
 
@@ -748,10 +748,10 @@ __device__ __forceinline__ void face_payload(const DView& v, int f, int nf4, int
     float px, py, pz, nx = 0.f, ny = 0.f, nz = 0.f;
     float2 t = make_float2(0.f, 0.f);
     if (v.pk) {
-      const float4 a = __ldg(&v.pk[2 * pi[k]]);
+      const float4 a = __ldg(&v.pk[2 * (size_t)pi[k]]);
       px = a.x; py = a.y; pz = a.z; nx = a.w;
       if (need_nrm || need_uv) {
-        const float4 b = __ldg(&v.pk[2 * pi[k] + 1]);
+        const float4 b = __ldg(&v.pk[2 * (size_t)pi[k] + 1]);
         ny = b.x; nz = b.y; t = make_float2(b.z, b.w);
       }
     } else {
