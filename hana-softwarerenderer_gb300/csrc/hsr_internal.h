@@ -50,7 +50,8 @@ constexpr uint32_t kErrCapacity = kErrRecOverflow | kErrClipOverflow | kErrBinOv
 // writing (an overflow is re-run with larger scratch; a scan that gave up has no tile lists).
 constexpr uint32_t kErrNoDraw = kErrCapacity | kErrScanTimeout;
 // Default poll limits of the bounded waits (Scratch::poll_limit overrides both).
-constexpr long kDepWaitPolls = 1L << 23;   // raster: a shadow map's tiles (~1-2 s)
+constexpr int kPollNs = 64;                // sleep between two polls
+constexpr long kDepWaitPolls = 1L << 24;   // raster: a shadow map's tiles (1-2 s)
 constexpr long kScanWaitPolls = 1L << 22;  // scan: a predecessor block's prefix
 
 // Record flags.

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
           atomicOr(&sc.ctl->error, kErrScanTimeout);
           break;
         }
-        __nanosleep(64);
+        __nanosleep(kPollNs);
       }
       __threadfence();
       if ((int)blk == nblocks - 1) sc.ctl->rec_extra += (uint32_t)ld_volatile64(sc.split + 1);
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
             atomicOr(&sc.ctl->error, kErrScanTimeout);
             break;
           }
-          __nanosleep(64);
+          __nanosleep(kPollNs);
         }
       }
     } else if (blk == 0) {
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
             if (lane == 0) atomicOr(&sc.ctl->error, kErrScanTimeout);
             break;
           }
-          __nanosleep(64);
+          __nanosleep(kPollNs);
           continue;
         }
         unsigned long long sum = (use >> lane & 1u) ? s & kValMask : 0ull;

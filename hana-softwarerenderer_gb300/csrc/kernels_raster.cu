@@ -53,7 +53,7 @@ __device__ __forceinline__ void wait_at_least(const Scratch& sc, const uint32_t*
       atomicOr(&sc.ctl->error, kErrWaitTimeout);
       return;
     }
-    __nanosleep(64);
+    __nanosleep(kPollNs);
   }
 }
 
