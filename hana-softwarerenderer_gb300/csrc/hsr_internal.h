@@ -241,6 +241,11 @@ inline int item_blocks(int n) {
   return (int)(want < 4096 ? want : 4096);
 }
 
+// First of n records that share k of `parts` takes, the shares as even as they come (no product that a
+// long list could carry past 32 bits).
+__host__ __device__ constexpr uint32_t share_begin(uint32_t n, uint32_t k, uint32_t parts) {
+  return n / parts * k + (k < n % parts ? k : n % parts);
+}
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.
 // `from` is mapped host memory or device memory; sizes are multiples of 16.
 // The order a mesh is kept in (see k_place_positions): raw device copies of the caller's arrays in,

@@ -353,8 +353,8 @@ __device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& 
     // this warp's records: all of the tile's list, or its share of it
     uint32_t b = 0, end = n;
     if (SHARED) {
-      b = (n * (uint32_t)warp) / WARPS;
-      end = (n * (uint32_t)(warp + 1)) / WARPS;
+      b = share_begin(n, (uint32_t)warp, WARPS);
+      end = share_begin(n, (uint32_t)warp + 1u, WARPS);
     }
     {  // every pixel starts from the clear depth, or from nothing where the buffer's is read later
       const unsigned long long k0 = clear ? buffer_key(v.clear_depth) : ~0ull;

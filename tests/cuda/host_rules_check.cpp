@@ -1,0 +1,34 @@
+// Host check of the kernels' arithmetic rules (hsr_internal.h): prints one line per failure.
+#include <cstdio>
+#include <initializer_list>
+
+#include "hsr_internal.h"
+
+using namespace hsr;
+
+static int failures = 0;
+#define CHECK(c)                                        \
+  do {                                                  \
+    if (!(c)) {                                         \
+      std::printf("line %d: %s\n", __LINE__, #c);       \
+      failures++;                                       \
+    }                                                   \
+  } while (0)
+
+// The shares of a list partition it, in order, whatever its length.
+static void shares() {
+  for (uint32_t parts : {4u, 8u})
+    for (uint32_t n : {0u, 1u, 3u, 4u, 7u, 8u, 9u, 1000u, 1u << 29, (1u << 29) + 1u, 1u << 30, 0x7fffffffu, 0xfffffffeu}) {
+      CHECK(share_begin(n, 0, parts) == 0u);
+      CHECK(share_begin(n, parts, parts) == n);
+      for (uint32_t k = 0; k < parts; k++) {
+        const uint32_t b = share_begin(n, k, parts), e = share_begin(n, k + 1, parts);
+        CHECK(b <= e && e - b <= n / parts + 1u);
+      }
+    }
+}
+
+int main() {
+  shares();
+  return failures != 0;
+}
