@@ -246,6 +246,15 @@ inline int item_blocks(int n) {
 __host__ __device__ constexpr uint32_t share_begin(uint32_t n, uint32_t k, uint32_t parts) {
   return n / parts * k + (k < n % parts ? k : n % parts);
 }
+// Warps of the scatter that share the same 32 records: up to kMaxSharers where records are few, and no
+// more than there are.
+constexpr uint32_t kMaxSharers = 16;
+__host__ __device__ constexpr uint32_t scatter_sharers(uint32_t nrec, uint32_t warps) {
+  uint32_t parts = warps * 32u / (nrec ? nrec : 1u);
+  if (parts > kMaxSharers) parts = kMaxSharers;
+  if (parts > warps) parts = warps;
+  return parts ? parts : 1u;
+}
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.
 // `from` is mapped host memory or device memory; sizes are multiples of 16.
 // The order a mesh is kept in (see k_place_positions): raw device copies of the caller's arrays in,

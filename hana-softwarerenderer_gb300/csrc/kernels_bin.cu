@@ -283,14 +283,13 @@ int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStr
 // (large triangles), up to kMaxSharers warps take the same 32 and share their pairs' steps, each
 // with an atomic's round trip (1000x600 with shadow, 3,779 records of 15 tiles each: 22.5 -> 12.3 us, 2560x1440
 // close-up 16.4 -> 10.2 us; a quarter million records and more keep their warps to themselves).
-constexpr uint32_t kMaxSharers = 16;
 __device__ __forceinline__ void scatter_records(const DView* views, int T, const Scratch& sc, uint32_t block,
                                                 uint32_t nblocks) {
   const int lane = threadIdx.x & 31;
   const uint32_t nrec = min(sc.ctl->rec_count + sc.ctl->rec_extra, sc.rec_cap);
   if (sc.ctl->error & kErrNoDraw) return;
   const uint32_t warps = nblocks * (blockDim.x >> 5);
-  const int parts = (int)max(min(warps * 32u / max(nrec, 1u), kMaxSharers), 1u);
+  const int parts = (int)scatter_sharers(nrec, warps);
   const uint32_t me = block * (blockDim.x >> 5) + (threadIdx.x >> 5), stride = warps / (uint32_t)parts * 32u;
   if (me / (uint32_t)parts * 32u >= stride) return;
   const int part = (int)(me % (uint32_t)parts);

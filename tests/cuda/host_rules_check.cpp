@@ -28,7 +28,18 @@ static void shares() {
     }
 }
 
+// Every group of 32 records has its warps, whatever the grid, and each warp's step is a whole group.
+static void sharers() {
+  for (uint32_t warps : {1u, 2u, 8u, 15u, 16u, 17u, 40u, 9728u})
+    for (uint32_t nrec : {0u, 1u, 31u, 32u, 33u, 100u, 5000u, 1u << 20, 0xfffff000u}) {
+      const uint32_t parts = scatter_sharers(nrec, warps), groups = warps / parts;
+      CHECK(parts >= 1u && parts <= kMaxSharers && groups >= 1u);
+      CHECK(parts == 1u || groups * 32u >= nrec || parts * nrec <= warps * 32u);
+    }
+}
+
 int main() {
   shares();
+  sharers();
   return failures != 0;
 }
