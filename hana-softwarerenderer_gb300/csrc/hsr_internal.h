@@ -209,7 +209,8 @@ struct Scratch {
   uint32_t* tile_off;       // [ntiles]
   uint32_t* ne_off;         // [ntiles + 1] non-empty tiles before each tile
   uint32_t* tile_list;      // [ntiles] the non-empty tiles in tile order (ne_tiles of them)
-  unsigned long long* split;        // parts of huge triangles split, their sub-records (two words, kSplitWords bytes behind ctl)
+  unsigned long long* split;        // parts of huge triangles split, their sub-records, the splitters' beats
+                                    // (three words, kSplitWords bytes behind ctl)
   unsigned long long* scan_status;  // [scan blocks]
   uint32_t* bins;   uint32_t bin_cap;
   int32_t ntiles;

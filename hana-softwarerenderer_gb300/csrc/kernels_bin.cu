@@ -66,11 +66,13 @@ int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t 
 // tiles (same triangle constants and seq, pixel range clipped to the block, each with its own copy
 // of the payload, since a record's payload index is its own index), and every tile of the
 // rectangle is counted once.  The sub-ranges partition the triangle's pixel range, so each pixel is
-// still tested exactly once.  `parts` warps share the triangle.  Returns a lane's number of tiles.
+// still tested exactly once.  `parts` warps share the triangle.  Every kStepsToBeat steps the warp counts up
+// a word that the waiting blocks watch.
 // (A warp and not a CTA each: most queued triangles have some tens of tiles, and what takes the time
 // is the chain of loads from the queue to the view.)
-__device__ __forceinline__ uint32_t split_triangle(const DView* views, int T, const Scratch& sc, const BigItem& bi,
-                                                   uint32_t first, int part, int parts) {
+constexpr uint32_t kStepsToBeat = 1024;  // a millisecond or so, whatever the triangle's size
+__device__ __forceinline__ void split_triangle(const DView* views, int T, const Scratch& sc, const BigItem& bi,
+                                               uint32_t first, int part, int parts) {
   const RasterRec b = bi.rec;
   const DView& v = views[b.view & kRecViewMask];
   int tx0, ty0, ntw, nt;
@@ -82,16 +84,20 @@ __device__ __forceinline__ uint32_t split_triangle(const DView* views, int T, co
   const int i0 = part * 32 + (int)(threadIdx.x & 31u), step = parts * 32;
   if ((uint64_t)base + (uint64_t)nsub > (uint64_t)sc.rec_cap) {
     if (i0 == 0) atomicOr(&sc.ctl->error, kErrRecOverflow);
-    return 0u;
+    return;
   }
+  uint32_t steps = 0;
+  auto beat = [&] {  // (the first lane has the most steps)
+    if ((++steps & (kStepsToBeat - 1u)) == 0u && (threadIdx.x & 31u) == 0u) atomicAdd(sc.split + 2, 1ull);
+  };
   const int nf4 = payload_f4(v.shader);
-  for (int k = i0; k < nsub * nf4; k += step)
+  for (int k = i0; k < nsub * nf4; k += step, beat())
     reinterpret_cast<float4*>(&sc.pay[base + (uint32_t)(k / nf4)])[k % nf4] =
         reinterpret_cast<const float4*>(&bi.pay)[k % nf4];
   if (i0 == 0 && nf4) atomicAdd(&sc.ctl->pay_bytes, 16ull * (unsigned long long)(nf4 * nsub));
   const int x0 = (int)(b.xr & 0xffffu), x1 = (int)(b.xr >> 16);
   const int y0 = (int)(b.yr & 0xffffu), y1 = (int)(b.yr >> 16);
-  for (int sidx = i0; sidx < nsub; sidx += step) {
+  for (int sidx = i0; sidx < nsub; sidx += step, beat()) {
     const int bx = sidx % nbx, by = sidx / nbx;
     const int stx0 = tx0 + bx * kSubTilesX, stx1 = min(tx0 + ntw - 1, stx0 + kSubTilesX - 1);
     const int sty0 = ty0 + by * kSubTilesY, sty1 = min(ty0 + nth - 1, sty0 + kSubTilesY - 1);
@@ -101,9 +107,8 @@ __device__ __forceinline__ uint32_t split_triangle(const DView* views, int T, co
     w.pad = 0u;
     store_rec(&sc.recs[base + (uint32_t)sidx], w);
   }
-  for (int k = i0; k < nt; k += step)
+  for (int k = i0; k < nt; k += step, beat())
     atomicAdd(&sc.tile_count[v.tile_base + (ty0 + k / ntw) * v.tiles_x + tx0 + k % ntw], 1u);
-  return (uint32_t)(nt / step) + 1u;
 }
 
 // Sub-records of the queued huge triangles, then the scan, in one grid: blocks take tickets; where
@@ -118,7 +123,6 @@ __device__ __forceinline__ uint32_t split_triangle(const DView* views, int T, co
 // 65.8 -> 64.2 us, of six objects in 1280x720 224 -> 219, of a recorded 1280x720 frame 178.7 -> 175.9.
 constexpr uint32_t kMaxParts = 256;
 constexpr uint32_t kScanWarps = kScanThreads / 32;
-constexpr uint32_t kStepsToReport = 4096;  // a splitter reports at least every few milliseconds
 __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T, Scratch sc, uint32_t splitters) {
   __shared__ unsigned long long warp_sums[kScanThreads / 32];
   __shared__ unsigned long long s_prefix;
@@ -139,17 +143,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
       const bool skip = (sc.ctl->error & kErrCapacity) != 0u;  // nothing will be drawn
       // (the clipper's count is final, and grows by the sub-records' only when all parts are done)
       const uint32_t base = sc.ctl->rec_count + sc.ctl->rec_extra;
-      uint32_t mine = 0, steps = 0;  // the CTA's parts done, and a thread's tiles in them
+      uint32_t mine = 0;  // the CTA's parts
       for (uint32_t u0 = blk * kScanWarps; u0 < units; u0 += first * kScanWarps) {
         const uint32_t u = u0 + (uint32_t)warp;
-        if (!skip && u < units) steps += split_triangle(views, T, sc, sc.bigq[u / parts], base, (int)(u % parts), (int)parts);
+        if (!skip && u < units) split_triangle(views, T, sc, sc.bigq[u / parts], base, (int)(u % parts), (int)parts);
         mine += min((uint32_t)kScanWarps, units - u0);
-        if (!__syncthreads_or(steps >= kStepsToReport || u0 + first * kScanWarps >= units)) continue;
-        if (threadIdx.x == 0) {
-          __threadfence();
-          atomicAdd(split_done, (unsigned long long)mine);
-        }
-        mine = steps = 0;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(split_done, (unsigned long long)mine);
       }
       return;
     }
@@ -157,10 +160,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
     if (blk >= (uint32_t)nblocks) return;
     if (threadIdx.x == 0) {
       unsigned long long seen = 0;
-      for (long spins = 0;;) {  // the limit counts from the last report
-        const unsigned long long s = ld_volatile64(split_done);
+      for (long spins = 0;;) {  // the limit counts from the last sign of a splitter
+        const unsigned long long s = ld_volatile64(split_done), beats = ld_volatile64(sc.split + 2);
         if (s >= units) break;
-        if (s != seen) { seen = s; spins = 0; }
+        if (s + beats != seen) { seen = s + beats; spins = 0; }
         if (++spins > limit) {
           atomicOr(&sc.ctl->error, kErrScanTimeout);
           break;

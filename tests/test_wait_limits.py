@@ -17,3 +17,18 @@ def test_a_dependency_wait_lasts_a_second_before_it_gives_up():
     assert polls * ns >= 1e9
     for f in ("kernels_raster.cu", "kernels_bin.cu"):
         assert set(re.findall(r"__nanosleep\(([^)]*)\)", _src(f))) == {"kPollNs"}
+
+
+def test_splitters_show_themselves_whatever_the_size_of_a_triangle():
+    """The scan's wait for the splitters counts from their last sign.  With many triangles queued a warp
+    takes each alone, up to 2^26 / 32 steps of it, so the sign cannot wait for the triangle's end: each
+    loop over its tiles or sub-records gives one every kStepsToBeat steps."""
+    s = _src("kernels_bin.cu")
+    body = re.search(r"void split_triangle\(.*?\n}\n", s, re.S).group(0)
+    loops = re.findall(r"for \(int \w+ = i0;[^\n]*", body)
+    assert len(loops) == 3 and all("beat())" in lp for lp in loops), loops
+    steps = int(re.search(r"kStepsToBeat = (\d+);", s).group(1))
+    ns = int(re.search(r"constexpr int kPollNs = (\d+);", _src("hsr_internal.h")).group(1))
+    polls = 1 << int(re.search(r"constexpr long kScanWaitPolls = 1L << (\d+);", _src("hsr_internal.h")).group(1))
+    assert steps & (steps - 1) == 0 and polls * ns >= 100e3 * steps  # 100 us a step (an atomic or a 64-byte store)
+    assert re.search(r"s \+ beats != seen", s)
