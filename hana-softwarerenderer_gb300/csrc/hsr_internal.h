@@ -257,23 +257,27 @@ __host__ __device__ constexpr uint32_t scatter_sharers(uint32_t nrec, uint32_t w
   return parts ? parts : 1u;
 }
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.
-// `from` is mapped host memory or device memory; sizes are multiples of 16.
-// The order a mesh is kept in (see k_place_positions): raw device copies of the caller's arrays in,
-// the mesh's arrays out.
-constexpr int kMeshCells = 1 << 18;
-constexpr int kOrderedFaces = 1 << 15;  // smaller meshes keep the caller's order (they fit the caches)
-struct MeshOrder {
-  const float* pos; int npos;        // [npos][3]
-  const int32_t* faces; int nfaces;  // [nfaces][3 corners][v, vt, vn]
-  uint32_t* cells;                   // scratch: kMeshCells + 8 words
-  uint32_t* codes;                   // scratch: max(npos, nfaces) words
-  uint32_t* place;                   // scratch: npos words
+// A mesh's position and face arrays, which a mesh of kOrderedFaces faces or more keeps in an order of
+// the library's own (see k_place_positions).
+struct MeshArrays {
   float *px, *py, *pz;
   float4* p4;
   uint32_t* vorder;                  // [npos] the caller's index of each position
   int4 *fv, *fvt, *fvn;
 };
-int launch_mesh_order(const MeshOrder& o, cudaStream_t s);
+constexpr int kMeshCells = 1 << 18;
+constexpr int kOrderedFaces = 1 << 15;  // smaller meshes keep the caller's order (they fit the caches)
+struct MeshOrder {                   // the caller's arrays on the device, and scratch
+  const float* pos; int npos;        // [npos][3]
+  const int32_t* faces; int nfaces;  // [nfaces][3 corners][v, vt, vn]
+  uint32_t* cells;                   // kMeshCells + 8 words
+  uint32_t* codes;                   // max(npos, nfaces) words
+  uint32_t* place;                   // npos words
+};
+int launch_mesh_order(const MeshOrder& o, const MeshArrays& m, cudaStream_t s);
+// Pieces of the caller's arrays, in the caller's order: items first, first + 1, ..., n of them.
+int launch_place_positions(const float* pos, int first, int n, const MeshArrays& m, cudaStream_t s);
+int launch_place_faces(const int32_t* faces, int first, int n, const MeshArrays& m, cudaStream_t s);
 int launch_split_normals(const float* nrm, int n, float* nx, float* ny, float* nz, float4* n4, cudaStream_t s);
 // `from` is mapped host memory or device memory; sizes are multiples of 16.
 int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s);

@@ -548,6 +548,103 @@ int Runtime::clear_target(TargetObj* t, const uint8_t rgba[4], float depth) {
   return e == cudaSuccess ? HSR_OK : cuda_fail(e, "clear");
 }
 
+// Host array to device memory on the library's stream (callers synchronise before they return).
+static cudaError_t stage(const void* src, size_t bytes, void* dst) {
+  return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g_rt->stream) : cudaSuccess;
+}
+
+// A host array of n items of `item` bytes through the device in pieces: place(piece, first, count) is
+// called for each, in stream order.  The pieces share one block of the stream-ordered pool, which stays
+// reserved there afterwards: at most 36 MiB.
+constexpr int kStagePiece = 1 << 20;
+template <class F>
+static cudaError_t stage_pieces(const void* src, int n, size_t item, F place) {
+  if (n <= 0) return cudaSuccess;
+  cudaStream_t st = g_rt->stream;
+  char* tmp = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&tmp, item * (size_t)std::min(n, kStagePiece), st);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return e;
+  }
+  for (int64_t first = 0; first < n && e == cudaSuccess; first += kStagePiece) {
+    const int count = (int)std::min<int64_t>(n - first, kStagePiece);
+    e = stage((const char*)src + item * (size_t)first, item * (size_t)count, tmp);
+    if (e == cudaSuccess) e = (cudaError_t)place(tmp, (int)first, count);
+  }
+  cudaFreeAsync(tmp, st);
+  return e;
+}
+
+static int upload_failed(cudaError_t e, const char* what) {
+  if (e == cudaErrorMemoryAllocation) return fail(HSR_ERR_OUT_OF_MEMORY, std::string("mesh: device allocation for the ") + what + " failed");
+  return cuda_fail(e, "mesh upload");
+}
+
+// The caller's normals into the mesh's arrays (and the packed vertices, which carry them too).
+static int place_normals(MeshObj* m, const float* nrm) {
+  cudaStream_t st = g_rt->stream;
+  cudaError_t e = stage_pieces(nrm, m->nnrm, sizeof(float) * 3, [&](const char* piece, int first, int count) {
+    return launch_split_normals((const float*)piece, count, m->nx + first, m->ny + first, m->nz + first, m->n4 + first, st);
+  });
+  if (e == cudaSuccess && m->pk)
+    e = (cudaError_t)launch_pack_vertices(m->pk, m->p4, m->vorder, m->n4, m->uv, m->npos, m->nnrm, m->nuv, st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? HSR_OK : upload_failed(e, "normals");
+}
+
+// The caller's positions and faces into the mesh's arrays in the library's order.  The raw arrays, codes and
+// places (a 4M-triangle soup: 385 MB) come from a pool of their own that keeps nothing: the memory
+// goes back to the device when the stream has been waited for.  False, with nothing written, where
+// they cannot be had.
+static bool order_mesh(MeshObj* m, const MeshArrays& to, const float* pos, const int32_t* faces, cudaError_t& e) {
+  cudaStream_t st = g_rt->stream;
+  const size_t npos = (size_t)m->npos, nfaces = (size_t)m->nfaces;
+  const size_t b_pos = align_up(sizeof(float) * 3 * npos, 256), b_faces = align_up(sizeof(int32_t) * 9 * nfaces, 256);
+  const size_t b_cells = sizeof(uint32_t) * (kMeshCells + 64), b_codes = align_up(sizeof(uint32_t) * std::max(npos, nfaces), 256);
+  char* tmp = nullptr;
+  if ((g_rt->faults & HSR_FAULT_UPLOAD_SCRATCH) ||
+      cudaMallocFromPoolAsync((void**)&tmp, b_pos + b_faces + b_cells + b_codes + sizeof(uint32_t) * npos + 256,
+                              g_rt->upload_pool, st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  MeshOrder o = {};
+  o.pos = (const float*)tmp;
+  o.npos = m->npos;
+  o.faces = (const int32_t*)(tmp + b_pos);
+  o.nfaces = m->nfaces;
+  o.cells = (uint32_t*)(tmp + b_pos + b_faces);
+  o.codes = (uint32_t*)(tmp + b_pos + b_faces + b_cells);
+  o.place = (uint32_t*)(tmp + b_pos + b_faces + b_cells + b_codes);
+  e = stage(pos, sizeof(float) * 3 * npos, tmp);
+  if (e == cudaSuccess) e = stage(faces, sizeof(int32_t) * 9 * nfaces, tmp + b_pos);
+  if (e == cudaSuccess) e = (cudaError_t)launch_mesh_order(o, to, st);
+  cudaFreeAsync(tmp, st);
+  return true;
+}
+
+// The caller's positions and faces into the mesh's arrays: ordered where the mesh is large and the
+// scratch can be had, else as they come.
+static int place_mesh(MeshObj* m, const float* pos, const int32_t* faces) {
+  cudaStream_t st = g_rt->stream;
+  const MeshArrays to = {m->px, m->py, m->pz, m->p4, m->vorder, m->fv, m->fvt, m->fvn};
+  cudaError_t e = cudaSuccess;
+  if (m->nfaces < kOrderedFaces || !order_mesh(m, to, pos, faces, e)) {
+    e = stage_pieces(pos, m->npos, sizeof(float) * 3, [&](const char* piece, int first, int count) {
+      return launch_place_positions((const float*)piece, first, count, to, st);
+    });
+    if (e == cudaSuccess)
+      e = stage_pieces(faces, m->nfaces, sizeof(int32_t) * 9, [&](const char* piece, int first, int count) {
+        return launch_place_faces((const int32_t*)piece, first, count, to, st);
+      });
+  }
+  const cudaError_t es = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? HSR_OK : upload_failed(e, "positions and faces");
+}
+
 }  // namespace hsr
 
 using namespace hsr;
@@ -590,6 +687,12 @@ int hsr_init(int device) {
   if (e != cudaSuccess) { delete rt; return cuda_fail(e, "cudaStreamCreate"); }
   e = cudaMallocHost((void**)&rt->fixed_host, kFixedHostBytes);
   if (e != cudaSuccess) { delete rt; return cuda_fail(e, "hsr_init: page-locked staging"); }
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  e = cudaMemPoolCreate(&rt->upload_pool, &props);  // (keeps nothing: its release threshold is zero)
+  if (e != cudaSuccess) { delete rt; return cuda_fail(e, "hsr_init: memory pool"); }
   for (int k = 0; k < Runtime::kEvents; k++) {
     e = cudaEventCreate(&rt->ev[k]);
     if (e != cudaSuccess) { delete rt; return cuda_fail(e, "cudaEventCreate"); }
@@ -609,73 +712,12 @@ int hsr_shutdown(void) {
   if (g_rt->arena.base) cudaFree(g_rt->arena.base);
   if (g_rt->staging.base) cudaFreeHost(g_rt->staging.base);
   cudaFreeHost(g_rt->fixed_host);
+  cudaMemPoolDestroy(g_rt->upload_pool);
   for (int k = 0; k < Runtime::kEvents; k++) cudaEventDestroy(g_rt->ev[k]);
   cudaStreamDestroy(g_rt->stream);
   delete g_rt;
   g_rt = nullptr;
   return HSR_OK;
-}
-
-// Host array to a temporary of the stream-ordered pool, on the library's stream (pageable memory: the
-// copy has left the host array when the call returns).
-static cudaError_t stage(const void* src, size_t bytes, void* dst) {
-  return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g_rt->stream) : cudaSuccess;
-}
-
-// The caller's normals into the mesh's arrays (and the packed vertices, which carry them too).
-static int place_normals(MeshObj* m, const float* nrm) {
-  cudaStream_t st = g_rt->stream;
-  const size_t bytes = sizeof(float) * 3 * (size_t)m->nnrm;
-  char* tmp = nullptr;
-  cudaError_t e = cudaSuccess;
-  if (bytes) {
-    e = cudaMallocAsync((void**)&tmp, bytes, st);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(HSR_ERR_OUT_OF_MEMORY, "mesh: device allocation for the normals failed");
-    }
-    e = stage(nrm, bytes, tmp);
-    if (e == cudaSuccess) e = (cudaError_t)launch_split_normals((const float*)tmp, m->nnrm, m->nx, m->ny, m->nz, m->n4, st);
-    cudaFreeAsync(tmp, st);
-  }
-  if (e == cudaSuccess && m->pk)
-    e = (cudaError_t)launch_pack_vertices(m->pk, m->p4, m->vorder, m->n4, m->uv, m->npos, m->nnrm, m->nuv, st);
-  const cudaError_t es = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = es;
-  return e == cudaSuccess ? HSR_OK : cuda_fail(e, "normal upload");
-}
-
-// The caller's positions and faces into the mesh's arrays, in the library's order.
-static int place_mesh(MeshObj* m, const float* pos, const int32_t* faces) {
-  cudaStream_t st = g_rt->stream;
-  const size_t npos = (size_t)m->npos, nfaces = (size_t)m->nfaces;
-  const size_t b_pos = align_up(sizeof(float) * 3 * npos, 256), b_faces = align_up(sizeof(int32_t) * 9 * nfaces, 256);
-  const size_t b_cells = sizeof(uint32_t) * (kMeshCells + 64), b_codes = align_up(sizeof(uint32_t) * std::max(npos, nfaces), 256);
-  char* tmp = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&tmp, b_pos + b_faces + b_cells + b_codes + sizeof(uint32_t) * npos + 256, st);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(HSR_ERR_OUT_OF_MEMORY, "mesh: device allocation for the mesh order failed");
-  }
-  MeshOrder o = {};
-  o.pos = (const float*)tmp;
-  o.npos = m->npos;
-  o.faces = (const int32_t*)(tmp + b_pos);
-  o.nfaces = m->nfaces;
-  o.cells = (uint32_t*)(tmp + b_pos + b_faces);
-  o.codes = (uint32_t*)(tmp + b_pos + b_faces + b_cells);
-  o.place = (uint32_t*)(tmp + b_pos + b_faces + b_cells + b_codes);
-  o.px = m->px; o.py = m->py; o.pz = m->pz;
-  o.p4 = m->p4;
-  o.vorder = m->vorder;
-  o.fv = m->fv; o.fvt = m->fvt; o.fvn = m->fvn;
-  e = stage(pos, sizeof(float) * 3 * npos, tmp);
-  if (e == cudaSuccess) e = stage(faces, sizeof(int32_t) * 9 * nfaces, tmp + b_pos);
-  if (e == cudaSuccess) e = (cudaError_t)launch_mesh_order(o, st);
-  cudaFreeAsync(tmp, st);
-  const cudaError_t es = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = es;
-  return e == cudaSuccess ? HSR_OK : cuda_fail(e, "mesh upload");
 }
 
 int hsr_mesh_upload(const float* pos, int32_t npos, const float* nrm, int32_t nnrm, const float* uv, int32_t nuv,
@@ -892,7 +934,7 @@ int hsr_set_tuning(const hsr_tuning* in) {
 
 int hsr_set_fault_injection(uint32_t faults, int32_t poll_limit) {
   RT_OR_FAIL();
-  if (faults & ~(uint32_t)(HSR_FAULT_DEPENDENCY_STALL | HSR_FAULT_SCAN_STALL))
+  if (faults & ~(uint32_t)(HSR_FAULT_DEPENDENCY_STALL | HSR_FAULT_SCAN_STALL | HSR_FAULT_UPLOAD_SCRATCH))
     return fail(HSR_ERR_INVALID_ARG, "set_fault_injection: unknown fault bit");
   if (poll_limit < 0) return fail(HSR_ERR_INVALID_ARG, "set_fault_injection: poll_limit must be >= 0");
   g_rt->faults = faults;

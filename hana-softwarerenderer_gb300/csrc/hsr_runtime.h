@@ -108,6 +108,7 @@ struct Runtime {
   Arena arena;
   Pinned staging;
   char* fixed_host = nullptr;  // page-locked, kFixedHostBytes: hsr_draw_noalloc's view descriptor and control block
+  cudaMemPool_t upload_pool = nullptr;  // scratch of a mesh upload, given back after it
   hsr_tuning tuning = {8, 4, 8, 4.0f};
   hsr_stats stats = {};
   uint64_t launches = 0;

@@ -297,40 +297,53 @@ __global__ void __launch_bounds__(1024) k_cell_scan(uint32_t* __restrict__ cells
   }
 }
 
-// Positions to their places (their own with cells null): SoA, float4, the caller's index of each
-// place and the place of each index.
-__global__ void __launch_bounds__(256) k_place_positions(const float* __restrict__ pos, int n, uint32_t* __restrict__ cells,
-                                                         const uint32_t* __restrict__ codes, float* __restrict__ px,
-                                                         float* __restrict__ py, float* __restrict__ pz,
-                                                         float4* __restrict__ p4, uint32_t* __restrict__ vorder,
-                                                         uint32_t* __restrict__ place) {
+// Positions first, first + 1, ... (raw) to their places (their own with cells null): SoA, float4, the
+// caller's index of each place and, where asked for, the place of each index.
+__global__ void __launch_bounds__(256) k_place_positions(const float* __restrict__ pos, int first, int n,
+                                                         uint32_t* __restrict__ cells, const uint32_t* __restrict__ codes,
+                                                         float* __restrict__ px, float* __restrict__ py,
+                                                         float* __restrict__ pz, float4* __restrict__ p4,
+                                                         uint32_t* __restrict__ vorder, uint32_t* __restrict__ place) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t at = cells ? atomicAdd(&cells[codes[i]], 1u) : (uint32_t)i;
+    const uint32_t own = (uint32_t)first + (uint32_t)i, at = cells ? atomicAdd(&cells[codes[i]], 1u) : own;
     const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
     px[at] = x;
     py[at] = y;
     pz[at] = z;
     p4[at] = make_float4(x, y, z, 0.f);
-    vorder[at] = (uint32_t)i;
-    place[i] = at;
+    vorder[at] = own;
+    if (place) place[own] = at;
   }
 }
 
-__global__ void __launch_bounds__(256) k_place_faces(const int32_t* __restrict__ faces, int n, uint32_t* __restrict__ cells,
-                                                     const uint32_t* __restrict__ codes, const uint32_t* __restrict__ place,
-                                                     int4* __restrict__ fv, int4* __restrict__ fvt, int4* __restrict__ fvn) {
+// Faces first, first + 1, ... (raw), likewise; their corners' positions have moved to `place` (null: not).
+__global__ void __launch_bounds__(256) k_place_faces(const int32_t* __restrict__ faces, int first, int n,
+                                                     uint32_t* __restrict__ cells, const uint32_t* __restrict__ codes,
+                                                     const uint32_t* __restrict__ place, int4* __restrict__ fv,
+                                                     int4* __restrict__ fvt, int4* __restrict__ fvn) {
+  auto at_place = [&](int32_t v) { return place ? (int)place[v] : v; };
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t at = cells ? atomicAdd(&cells[codes[i]], 1u) : (uint32_t)i;
+    const uint32_t own = (uint32_t)first + (uint32_t)i, at = cells ? atomicAdd(&cells[codes[i]], 1u) : own;
     const int32_t* r = faces + 9 * i;
-    fv[at] = make_int4((int)place[r[0]], (int)place[r[3]], (int)place[r[6]], (int)i);
+    fv[at] = make_int4(at_place(r[0]), at_place(r[3]), at_place(r[6]), (int)own);
     fvt[at] = make_int4(r[1], r[4], r[7], 0);
     fvn[at] = make_int4(r[2], r[5], r[8], 0);
   }
 }
 
-int launch_mesh_order(const MeshOrder& o, cudaStream_t s) {
+int launch_place_positions(const float* pos, int first, int n, const MeshArrays& m, cudaStream_t s) {
+  if (n <= 0) return 0;
+  k_place_positions<<<item_blocks(n), 256, 0, s>>>(pos, first, n, nullptr, nullptr, m.px, m.py, m.pz, m.p4, m.vorder, nullptr);
+  return (int)cudaGetLastError();
+}
+int launch_place_faces(const int32_t* faces, int first, int n, const MeshArrays& m, cudaStream_t s) {
+  if (n <= 0) return 0;
+  k_place_faces<<<item_blocks(n), 256, 0, s>>>(faces, first, n, nullptr, nullptr, nullptr, m.fv, m.fvt, m.fvn);
+  return (int)cudaGetLastError();
+}
+
+int launch_mesh_order(const MeshOrder& o, const MeshArrays& m, cudaStream_t s) {
   const int pg = item_blocks(o.npos), fg = item_blocks(o.nfaces);
-  const bool sorted = o.nfaces >= kOrderedFaces;
   int* bounds = reinterpret_cast<int*>(o.cells + kMeshCells);
   auto group = [&](const int32_t* faces, int n, int grid) {
     cudaError_t e = cudaMemsetAsync(o.cells, 0, sizeof(uint32_t) * kMeshCells, s);
@@ -339,19 +352,14 @@ int launch_mesh_order(const MeshOrder& o, cudaStream_t s) {
     k_cell_scan<<<1, 1024, 0, s>>>(o.cells);
     return cudaGetLastError();
   };
-  if (sorted) {
-    k_bounds_init<<<1, 32, 0, s>>>(bounds);
-    k_bounds<<<std::min(pg, 1024), 256, 0, s>>>(o.pos, o.npos, bounds);
-    const cudaError_t e = group(nullptr, o.npos, pg);
-    if (e != cudaSuccess) return (int)e;
-  }
-  k_place_positions<<<pg, 256, 0, s>>>(o.pos, o.npos, sorted ? o.cells : nullptr, o.codes, o.px, o.py, o.pz, o.p4, o.vorder,
-                                       o.place);
-  if (sorted) {
-    const cudaError_t e = group(o.faces, o.nfaces, fg);
-    if (e != cudaSuccess) return (int)e;
-  }
-  k_place_faces<<<fg, 256, 0, s>>>(o.faces, o.nfaces, sorted ? o.cells : nullptr, o.codes, o.place, o.fv, o.fvt, o.fvn);
+  k_bounds_init<<<1, 32, 0, s>>>(bounds);
+  k_bounds<<<std::min(pg, 1024), 256, 0, s>>>(o.pos, o.npos, bounds);
+  cudaError_t e = group(nullptr, o.npos, pg);
+  if (e != cudaSuccess) return (int)e;
+  k_place_positions<<<pg, 256, 0, s>>>(o.pos, 0, o.npos, o.cells, o.codes, m.px, m.py, m.pz, m.p4, m.vorder, o.place);
+  e = group(o.faces, o.nfaces, fg);
+  if (e != cudaSuccess) return (int)e;
+  k_place_faces<<<fg, 256, 0, s>>>(o.faces, 0, o.nfaces, o.cells, o.codes, o.place, m.fv, m.fvt, m.fvn);
   return (int)cudaGetLastError();
 }
 

@@ -231,6 +231,7 @@ def stats() -> dict:
 
 FAULT_DEPENDENCY_STALL = 1
 FAULT_SCAN_STALL = 2
+FAULT_UPLOAD_SCRATCH = 4
 
 
 def set_fault_injection(faults: int = 0, poll_limit: int = 0) -> None:

@@ -123,7 +123,11 @@ HSR_API int hsr_abi_version(void);
  * 0-based (v, vt, vn) index of each corner, the layout of Model::faces_ (model.h:11).
  * Indices are validated on the host.  Normals are used as stored: the reference
  * normalises them in place on every access (model.cpp:108-111), which is the identity
- * for normals that are fixed points of Vector3f::normalize(). */
+ * for normals that are fixed points of Vector3f::normalize().
+ * While the call runs it holds device scratch beside the mesh's own arrays: for 2^15 faces and
+ * more, 16-20 bytes a position and 36-40 a face, which are given back before it returns (a mesh whose
+ * scratch cannot be had is kept in the caller's order, with the same results); else, and for
+ * hsr_mesh_update_normals, up to 36 MiB, which stay in the device's stream-ordered pool. */
 HSR_API int hsr_mesh_upload(const float* pos, int32_t npos, const float* nrm, int32_t nnrm,
                     const float* uv, int32_t nuv, const int32_t* faces, int32_t nfaces,
                     hsr_mesh* out);
@@ -272,9 +276,12 @@ HSR_API int hsr_autotune(const hsr_draw_desc* descs, int32_t n, int32_t reps, hs
  *                               HSR_ERR_TIMEOUT and the device stays usable;
  *   HSR_FAULT_SCAN_STALL        the tile-count scan's first block withholds its prefix and
  *                               waits for a flag nothing sets, so every look-back runs out:
- *                               the call returns HSR_ERR_TIMEOUT and writes no target. */
+ *                               the call returns HSR_ERR_TIMEOUT and writes no target;
+ *   HSR_FAULT_UPLOAD_SCRATCH    hsr_mesh_upload finds no memory for the scratch that orders a
+ *                               large mesh: the mesh keeps the caller's order (same results). */
 #define HSR_FAULT_DEPENDENCY_STALL 1u
 #define HSR_FAULT_SCAN_STALL 2u
+#define HSR_FAULT_UPLOAD_SCRATCH 4u
 HSR_API int hsr_set_fault_injection(uint32_t faults, int32_t poll_limit);
 
 /* ---- statistics of the last completed draw sequence (for tests and benchmarks) ------- */
