@@ -256,6 +256,15 @@ __host__ __device__ constexpr uint32_t scatter_sharers(uint32_t nrec, uint32_t w
   if (parts > warps) parts = warps;
   return parts ? parts : 1u;
 }
+// What of a sequence's empty tiles the scatter's grid clears: `clear_bytes`, the planes of the views that
+// clear, of the three planes of all views' pixels (several draws into one target clear it once).
+inline float clear_share(size_t clear_bytes, size_t pixels) { return (float)clear_bytes / (12.f * (float)(pixels ? pixels : 1)); }
+// Of how many blocks of that grid one scatters while the others clear: two, or three where the pixels to
+// clear (of three planes) outweigh the (record, tile) pairs (see k_scatter).
+constexpr float kClearHeavy = 10.f;
+__host__ __device__ constexpr uint32_t scatter_every(uint32_t empty_tiles, int tile, float share, uint32_t pairs) {
+  return (float)empty_tiles * (float)(tile * tile) * share >= kClearHeavy * (float)pairs ? 3u : 2u;
+}
 // Kernel launchers (kernels_*.cu).  All return cudaError_t as int.
 // A mesh's position and face arrays, which a mesh of kOrderedFaces faces or more keeps in an order of
 // the library's own (see k_place_positions).
@@ -288,8 +297,7 @@ bool clips_with_emit(size_t faces);  // the emit pass's grid also clips (no laun
 int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms, cudaStream_t s);
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
 int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStream_t s);
-int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int clear_chunks, uint32_t plane_bytes,
-                   cudaStream_t s);
+int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int clear_chunks, float clear_share, cudaStream_t s);
 int launch_raster(const DView* views, int tile, Scratch sc, int grid, int warps, cudaStream_t s);
 int scan_blocks(int ntiles);
 

@@ -239,8 +239,10 @@ int Runtime::plan_build(const hsr_draw_desc* descs, int n, Plan& p, bool in_orde
     v.cch_base = p.ncch;
     p.nvch += v.vch_count;
     p.nsch += (m->nfaces + kSetupChunk - 1) / kSetupChunk;
-    p.clear_bytes += (size_t)tg->w * (size_t)tg->h * (4u + (tg->depth ? 4u : 0u) + (tg->prim ? 4u : 0u));
-    if (d.flags & HSR_DRAW_CLEAR) p.ncch += (int)(((size_t)tg->w * (size_t)tg->h + kClearChunk - 1) / kClearChunk);
+    if (d.flags & HSR_DRAW_CLEAR) {
+      p.clear_bytes += (size_t)tg->w * (size_t)tg->h * (4u + (tg->depth ? 4u : 0u) + (tg->prim ? 4u : 0u));
+      p.ncch += (int)(((size_t)tg->w * (size_t)tg->h + kClearChunk - 1) / kClearChunk);
+    }
   }
   for (int k = 0; k < n; k++) {
     // the readers of a target wait for every view that writes it (a chain already marked is marked whole)
@@ -363,7 +365,7 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
   // above this batch's record count)
   const size_t want = ncch ? (size_t)num_sms * 8 : std::min<size_t>((rec_cap + 255) / 256, (size_t)num_sms * 8);
   kr = launch_scatter(dviews, tile, sc, (int)std::max<size_t>(want, 1), ncch,
-                      (uint32_t)(clear_bytes / std::max<size_t>(total_pixels, 1)), s);
+                      clear_share(clear_bytes, total_pixels), s);
   if (kr) return cuda_fail((cudaError_t)kr, "scatter kernel");
   mark(8);
   for (int g = 0, ng = split ? split->n : 1; g < ng; g++) {

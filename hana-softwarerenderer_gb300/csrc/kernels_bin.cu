@@ -446,18 +446,16 @@ __device__ __forceinline__ void clear_empty_tiles(const DView* views, int T, int
 // (record, tile) pairs, two of three do (16 views, 15 pixels a pair: 92 -> 76 us; at 6 a pair, 64
 // requests, that is 299 -> 354).
 constexpr int kClearMinBlocks = 3;
-constexpr unsigned long long kClearHeavy = 10;  // pixels of three planes per pair
 
 __global__ void __launch_bounds__(256) k_scatter(const DView* views, int T, Scratch sc, int nchunks,
-                                                 uint32_t plane_bytes) {
+                                                 float clear_share) {
   __shared__ int32_t s_cbase[kSharedViews];
   const uint32_t b = blockIdx.x, g = gridDim.x;
   chain_wait();
   const uint32_t ne = sc.ctl->ne_tiles, nt = (uint32_t)sc.ntiles;
   if (ne >= nt) nchunks = 0;  // every tile is the raster's: all blocks scatter
-  const unsigned long long px = (unsigned long long)(nt - min(ne, nt)) * (unsigned)(T * T) * plane_bytes / 12u;
-  const uint32_t every = px >= kClearHeavy * sc.ctl->bin_total ? 3u : 2u;  // 3: two clear and one scatters
-  const uint32_t first = b / every * (every - 1u);                         // clearing blocks before this group
+  const uint32_t every = scatter_every(nt - min(ne, nt), T, clear_share, sc.ctl->bin_total);
+  const uint32_t first = b / every * (every - 1u);  // clearing blocks before this group
   if (nchunks > 0 && b % every != 0u) {  // block-uniform
     const bool in_shared = sc.nviews <= kSharedViews;
     if (in_shared)
@@ -473,10 +471,10 @@ __global__ void __launch_bounds__(256) k_scatter(const DView* views, int T, Scra
 }
 
 // `grid` blocks of 256 threads (at least kClearMinBlocks when the batch clears, so both parts have
-// blocks); `plane_bytes`: bytes cleared per pixel on average.
-int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int nchunks, uint32_t plane_bytes, cudaStream_t s) {
+// blocks).
+int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int nchunks, float clear_share, cudaStream_t s) {
   if (nchunks > 0 && grid < kClearMinBlocks) grid = kClearMinBlocks;
-  return launch_chained(k_scatter, grid > 0 ? grid : 1, 256, 0, s, views, tile, sc, nchunks, plane_bytes);
+  return launch_chained(k_scatter, grid > 0 ? grid : 1, 256, 0, s, views, tile, sc, nchunks, clear_share);
 }
 
 }  // namespace hsr

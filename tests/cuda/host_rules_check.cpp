@@ -38,8 +38,20 @@ static void sharers() {
     }
 }
 
+// Six draws into one 1280x720 target, five pixels to clear a pair and draw: what the five that do not
+// clear leave empty is not to be cleared.  One draw of 15 pixels a pair: two blocks of three clear.
+static void clears() {
+  const size_t px = 1280 * 720, tiles = px / 64;
+  const uint32_t empty = (uint32_t)(tiles / 2);
+  CHECK(scatter_every(6 * empty, 8, clear_share(12 * px, 6 * px), (uint32_t)(px / 2 / 5)) == 2u);
+  CHECK(scatter_every(empty, 8, clear_share(12 * px, px), (uint32_t)(px / 2 / 15)) == 3u);
+  CHECK(scatter_every(empty, 8, clear_share(4 * px, px), (uint32_t)(px / 2 / 15)) == 2u);  // colour alone
+  CHECK(clear_share(0, 0) == 0.f);
+}
+
 int main() {
   shares();
   sharers();
+  clears();
   return failures != 0;
 }
