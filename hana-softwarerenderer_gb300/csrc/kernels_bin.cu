@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
         mine += min((uint32_t)kScanWarps, units - u0);
       }
       __syncthreads();
-      if (threadIdx.x == 0) {
+      if (threadIdx.x == 0 && !(sc.faults & HSR_FAULT_SCAN_STALL)) {  // injected stall: no report
         __threadfence();
         atomicAdd(split_done, (unsigned long long)mine);
       }
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
     const unsigned long long agg = __shfl_sync(kFull, wi, kScanThreads / 32 - 1);  // the block's; publish, look back
     unsigned long long* st = sc.scan_status;
     unsigned long long prefix = 0;
-    if (blk == 0 && (sc.faults & HSR_FAULT_SCAN_STALL)) {
-      // injected stall: withhold the prefix and wait on a word nothing sets (its own)
+    if (blk == 0 && nbig == 0u && (sc.faults & HSR_FAULT_SCAN_STALL)) {
+      // injected stall (the splitters' where there are any): withhold the prefix and wait on a word nothing sets (its own)
       if (lane == 0) {
         long spins = 0;
         while ((ld_volatile64(&st[0]) >> 62) == 0) {

@@ -74,13 +74,9 @@ __device__ __forceinline__ void wait_target(const Scratch& sc, const DView* view
 // Wait for tile `lt` of the earlier views into this view's target.  Views of one target share their
 // tile grid and a tile reads no pixel but its own, so the last of them that has records there is
 // the only one to wait for (it waited for those before it).  A finished tile's fill cursor, spent
-// after the binning, holds kTileDone.
+// after the binning, holds kTileDone (HSR_FAULT_DEPENDENCY_STALL withholds it).
 constexpr uint32_t kTileDone = 0xffffffffu;
 __device__ __forceinline__ void wait_tile(const Scratch& sc, const DView* views, int dep, int lt) {
-  if (sc.faults & HSR_FAULT_DEPENDENCY_STALL) {
-    wait_target(sc, views, dep);
-    return;
-  }
   for (int d = dep; d >= 0; d = views[d].dep1) {
     const int t = views[d].tile_base + lt;
     if (sc.tile_count[t] == 0u) continue;
@@ -608,7 +604,8 @@ __device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& 
         if (SHARED) __syncthreads(); else __syncwarp();
         if (SHARED ? threadIdx.x == 0 : lane == 0) {
           if (v.has_dependents & kTargetReaders) atomicAdd(&sc.view_done[vi], sm.done[warp]);
-          if (v.has_dependents & kTileReaders) atomicExch(&sc.tile_fill[t], kTileDone);
+          if ((v.has_dependents & kTileReaders) && !(sc.faults & HSR_FAULT_DEPENDENCY_STALL))
+            atomicExch(&sc.tile_fill[t], kTileDone);
           sm.done[warp] = 0u;
         }
       }

@@ -272,11 +272,15 @@ HSR_API int hsr_autotune(const hsr_draw_desc* descs, int32_t n, int32_t reps, hs
  * has given up, the others of that sequence stop waiting too.  faults is a mask of:
  *   HSR_FAULT_DEPENDENCY_STALL  raster tiles of a draw that reads another draw's target (its
  *                               shadow map) wait for one finished tile more than that draw
- *                               has, so the wait ends only by running out: the call returns
- *                               HSR_ERR_TIMEOUT and the device stays usable;
+ *                               has, and a finished tile of a draw that a later one draws over
+ *                               is not reported, so the waits end only by running out: the
+ *                               call returns HSR_ERR_TIMEOUT and the device stays usable;
  *   HSR_FAULT_SCAN_STALL        the tile-count scan's first block withholds its prefix and
- *                               waits for a flag nothing sets, so every look-back runs out:
- *                               the call returns HSR_ERR_TIMEOUT and writes no target;
+ *                               waits for a flag nothing sets, so every look-back runs out;
+ *                               where triangles of many tiles are split first, the blocks
+ *                               that split them do not report instead, and the scan's wait for
+ *                               them runs out: the call returns HSR_ERR_TIMEOUT and writes
+ *                               no target;
  *   HSR_FAULT_UPLOAD_SCRATCH    hsr_mesh_upload finds no memory for the scratch that orders a
  *                               large mesh: the mesh keeps the caller's order (same results). */
 #define HSR_FAULT_DEPENDENCY_STALL 1u

@@ -32,3 +32,13 @@ def test_splitters_show_themselves_whatever_the_size_of_a_triangle():
     polls = 1 << int(re.search(r"constexpr long kScanWaitPolls = 1L << (\d+);", _src("hsr_internal.h")).group(1))
     assert steps & (steps - 1) == 0 and polls * ns >= 100e3 * steps  # 100 us a step (an atomic or a 64-byte store)
     assert re.search(r"s \+ beats != seen", s)
+
+
+def test_injected_stalls_reach_the_waits_they_are_for():
+    """A withheld report, not another wait in its place: of a finished tile to the next draw into its target,
+    and of the splitters to the scan."""
+    r, b = _src("kernels_raster.cu"), _src("kernels_bin.cu")
+    body = re.search(r"void wait_tile\(.*?\n}\n", r, re.S).group(0)
+    assert "faults" not in body and "wait_at_least(sc, &sc.tile_fill[t], kTileDone)" in body
+    assert re.search(r"!\(sc\.faults & HSR_FAULT_DEPENDENCY_STALL\)\)\s*atomicExch\(&sc\.tile_fill\[t\], kTileDone\)", r)
+    assert re.search(r"!\(sc\.faults & HSR_FAULT_SCAN_STALL\)\) \{[^}]*atomicAdd\(split_done", b)
