@@ -91,3 +91,66 @@ def test_upload_gives_its_scratch_back(gpu):
     gpu.Mesh(mesh).release()
     torch.cuda.synchronize()
     assert before - torch.cuda.mem_get_info()[0] <= 64 << 20
+
+
+def _grid(cells, seed, split):
+    """A height field of 2 * cells^2 triangles; `split`: uvs and normals in arrays of their own order."""
+    m = scenes.grid_mesh(cells, cells, seed)
+    if split:
+        rng = np.random.default_rng(seed)
+        m.faces = m.faces.copy()
+        for k, name in ((1, "uv"), (2, "nrm")):
+            at = rng.permutation(len(m.pos)).astype(np.int32)
+            v = np.empty_like(getattr(m, name))
+            v[at] = getattr(m, name)
+            setattr(m, name, v)
+            m.faces[:, :, k] = at[m.faces[:, :, k]]
+    return m
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("cells", [20, 127, 128, 200])  # 2^15 faces at 128
+@pytest.mark.parametrize("shader", [scenes.GROUND, scenes.BLINN])
+def test_normals_replaced_after_the_upload(gpu, cells, split, shader):
+    """The same bytes as a mesh uploaded with those normals, and the oracle's picture."""
+    w, h = 320, 200
+    mesh = _grid(cells, cells, split)
+    rng = np.random.default_rng(cells)
+    new = scenes.fixed_point_normals((mesh.nrm + rng.normal(0, 0.3, mesh.nrm.shape)).astype(np.float32))
+    sd = U.shader_data((0.4, 1.3, 1.9), w, h)
+    tex = scenes.noise_texture(64, 64, 4, 3)
+    got = _draw(gpu, mesh, shader, sd, w, h, tex, update=new)
+    with_new = scenes.Mesh(mesh.pos, new, mesh.uv, mesh.faces)
+    _equal(got, _draw(gpu, with_new, shader, sd, w, h, tex))
+    exp = _oracle(with_new, shader, sd, w, h, tex)
+    assert (exp["prim"] > 0).mean() > 0.1
+    assert not np.array_equal(exp["color"], _oracle(mesh, shader, sd, w, h, tex)["color"])
+    golden_io.assert_pass(got, exp, "main", f"normals {cells}", 1)
+
+
+@pytest.mark.parametrize("kind", ["inf", "nan", "huge", "all-nan", "one-point"])
+def test_positions_without_a_place_in_the_grid(faults, kind):
+    """Positions that are not finite, span more than a float, or none at all: the order changes nothing."""
+    w, h = 300, 200
+    mesh = _grid(150, 5, False)
+    mesh.pos = mesh.pos.copy()
+    rng = np.random.default_rng(6)
+    some = rng.choice(len(mesh.pos), len(mesh.pos) // 20, replace=False)
+    at = (some, rng.integers(0, 3, len(some)))
+    if kind == "inf":
+        mesh.pos[at] = rng.choice([np.inf, -np.inf], len(some))
+    elif kind == "nan":
+        mesh.pos[at] = np.nan
+    elif kind == "huge":
+        mesh.pos[at] = rng.choice([3.4e38, -3.4e38, 1e-42], len(some))
+    elif kind == "all-nan":
+        mesh.pos[:] = np.nan
+    else:
+        mesh.pos[:] = mesh.pos[7]
+    sd = U.shader_data((0.4, 1.3, 1.9), w, h)
+    got = _draw(faults, mesh, scenes.GROUND, sd, w, h)
+    exp = _oracle(mesh, scenes.GROUND, sd, w, h)
+    assert (exp["prim"] > 0).any() == (kind in ("inf", "nan", "huge"))
+    golden_io.assert_pass(got, exp, "main", kind, 1)
+    faults.set_fault_injection(faults.FAULT_UPLOAD_SCRATCH, 0)
+    _equal(got, _draw(faults, mesh, scenes.GROUND, sd, w, h))
