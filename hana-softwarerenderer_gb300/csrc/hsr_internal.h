@@ -296,7 +296,9 @@ int launch_setup(const DView* views, int nviews, int nchunks, bool own_vertices,
 bool clips_with_emit(size_t faces);  // the emit pass's grid also clips (no launch_post)
 int launch_emit(const DView* views, int tile, Scratch sc, bool clip, int num_sms, cudaStream_t s);
 int launch_post(const DView* views, int tile, Scratch sc, int grid, cudaStream_t s);
-int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStream_t s);
+// One grid for both parts, or (to time them) a grid of `splitters` blocks and a grid that scans.
+enum { kSplitAndScan, kSplitAlone, kScanAlone };
+int launch_scan(const DView* views, int tile, Scratch sc, int splitters, int part, cudaStream_t s);
 int launch_scatter(const DView* views, int tile, Scratch sc, int grid, int clear_chunks, float clear_share, cudaStream_t s);
 int launch_raster(const DView* views, int tile, Scratch sc, int grid, int warps, cudaStream_t s);
 int scan_blocks(int ntiles);

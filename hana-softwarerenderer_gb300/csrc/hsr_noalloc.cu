@@ -183,7 +183,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   if (!kr) kr = launch_setup(dview, 1, nsch, own, sc, rt->num_sms * 8, s);
   if (!kr) kr = launch_emit(dview, T, sc, clips_with_emit(faces), rt->num_sms, s);
   if (!kr && !clips_with_emit(faces)) kr = launch_post(dview, T, sc, rt->num_sms * 4, s);
-  if (!kr) kr = launch_scan(dview, T, sc, rt->num_sms * 2, s);
+  if (!kr) kr = launch_scan(dview, T, sc, rt->num_sms * 2, kSplitAndScan, s);
   if (!kr) kr = launch_scatter(dview, T, sc, rt->num_sms * 8, ncch, 1.f, s);
   if (!kr) kr = launch_raster(dview, T, sc, rt->num_sms * rt->tuning.ctas_per_sm, rt->tuning.warps_per_cta, s);
   if (kr) return cuda_fail((cudaError_t)kr, "draw_noalloc: kernel launch");

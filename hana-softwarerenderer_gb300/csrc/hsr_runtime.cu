@@ -349,15 +349,17 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
   kr = launch_setup(dviews, n, nsch, own, sc, num_sms * 8, s);
   if (kr) return cuda_fail((cudaError_t)kr, "setup kernel");
   mark(3);
-  const bool one_grid = clips_with_emit(total_faces);
+  const bool one_grid = clips_with_emit(total_faces) && !apart;
   kr = launch_emit(dviews, tile, sc, one_grid, num_sms, s);
   if (kr) return cuda_fail((cudaError_t)kr, "emit kernel");
   mark(4);
   kr = one_grid ? 0 : launch_post(dviews, tile, sc, num_sms * 4, s);
   if (kr) return cuda_fail((cudaError_t)kr, "post kernel");
   mark(5);
+  kr = apart ? launch_scan(dviews, tile, sc, num_sms * 2, kSplitAlone, s) : 0;
+  if (kr) return cuda_fail((cudaError_t)kr, "split kernel");
   mark(6);
-  kr = launch_scan(dviews, tile, sc, num_sms * 2, s);
+  kr = launch_scan(dviews, tile, sc, num_sms * 2, apart ? kScanAlone : kSplitAndScan, s);
   if (kr) return cuda_fail((cudaError_t)kr, "scan kernel");
   mark(7);
   // grid-stride over the records: one full wave of 256-thread blocks (fewer when there are
@@ -387,7 +389,7 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
 }
 
 int Plan::kernel_count() const {
-  return 1 + (nvch && !culls_own_vertices(total_faces, total_pos) ? 1 : 0) + (nsch ? 1 : 0) + (clips_with_emit(total_faces) ? 1 : 2) + 3;
+  return 1 + (nvch && !culls_own_vertices(total_faces, total_pos) ? 1 : 0) + (nsch ? 1 : 0) + (clips_with_emit(total_faces) && !apart ? 1 : 2) + (apart ? 1 : 0) + 3;
 }
 
 // Grow the capacity an overflow reported; returns false if nothing overflowed.
@@ -460,6 +462,7 @@ int Runtime::run_sequence(const hsr_draw_desc* descs, int n) {
   Plan p;
   int rc = plan_build(descs, n, p);
   if (rc != HSR_OK) return rc;
+  p.apart = profiling;
   for (int attempt = 0; attempt < 6; attempt++) {
     p.layout();
     rc = arena.reserve(p.dev_bytes);
@@ -491,8 +494,6 @@ int Runtime::run_sequence(const hsr_draw_desc* descs, int n) {
     for (int k = 0; k < HSR_KERNEL_COUNT; k++) {
       float km = timing.kernel_ms[k] = 0.f;
       if (k == 0 && culls_own_vertices(p.total_faces, p.total_pos)) continue;  // part of the cull pass
-      if (k == 4) continue;  // split in the scan's grid
-      if (k == 3 && clips_with_emit(p.total_faces)) continue;  // clipped in the emit pass's grid
       if (profiling) cudaEventElapsedTime(&km, ev[k + 1], ev[k + 2]);
       timing.kernel_ms[k] = km;
     }

@@ -73,6 +73,7 @@ struct Plan {
   std::vector<DView> views;
   std::vector<Off> offs;
   int nvch = 0, nsch = 0, ncch = 0;  // vertex / setup / clear chunks of the batch (bases in each DView)
+  bool apart = false;                // the clipper and the splitters in launches of their own, to time them
   uint32_t stash_warps = 0;          // raster warps with a stash (the device's SMs x kStashWarpsPerSm)
   size_t view_bytes = 0, total_faces = 0, total_tiles = 0, total_pos = 0, total_nrm = 0, total_pixels = 0, clear_bytes = 0;
   size_t rec_cap = 0, clip_cap = 0, bin_cap = 0, big_cap = 0;

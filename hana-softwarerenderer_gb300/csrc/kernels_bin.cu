@@ -123,7 +123,8 @@ __device__ __forceinline__ void split_triangle(const DView* views, int T, const 
 // 65.8 -> 64.2 us, of six objects in 1280x720 224 -> 219, of a recorded 1280x720 frame 178.7 -> 175.9.
 constexpr uint32_t kMaxParts = 256;
 constexpr uint32_t kScanWarps = kScanThreads / 32;
-__global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T, Scratch sc, uint32_t splitters) {
+__global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T, Scratch sc, uint32_t splitters,
+                                                           int part) {
   __shared__ unsigned long long warp_sums[kScanThreads / 32];
   __shared__ unsigned long long s_prefix;
   __shared__ uint32_t s_block;
@@ -134,12 +135,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
   chain_wait();
   if (threadIdx.x == 0) s_block = atomicAdd(&sc.ctl->scan_ticket, 1u);
   __syncthreads();
-  uint32_t blk = s_block;
+  // (kScanAlone: the splitters' grid before this one took the first tickets)
+  uint32_t blk = s_block - (part == kScanAlone ? splitters : 0u);
   const uint32_t nbig = min(sc.ctl->big_count, sc.big_cap);
   if (nbig > 0u) {
     const uint32_t parts = min(max(splitters * kScanWarps / nbig, 1u), kMaxParts), units = nbig * parts;
     const uint32_t first = min(splitters, (units + kScanWarps - 1) / kScanWarps);
-    if (blk < first) {
+    if (part != kScanAlone && blk < first) {
       const bool skip = (sc.ctl->error & kErrCapacity) != 0u;  // nothing will be drawn
       // (the clipper's count is final, and grows by the sub-records' only when all parts are done)
       const uint32_t base = sc.ctl->rec_count + sc.ctl->rec_extra;
@@ -156,7 +158,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
       }
       return;
     }
-    blk -= first;
+    if (part == kSplitAlone) return;
+    if (part == kSplitAndScan) blk -= first;
     if (blk >= (uint32_t)nblocks) return;
     if (threadIdx.x == 0) {
       unsigned long long seen = 0;
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
     }
     __syncthreads();
   }
-  if (blk >= (uint32_t)nblocks) return;
+  if (part == kSplitAlone || blk >= (uint32_t)nblocks) return;
   const int base = (int)blk * kScanTile + (int)threadIdx.x * kScanItems;
   uint32_t vals[kScanItems];
   static_assert(kScanItems == 4, "one 16-byte load");
@@ -277,8 +280,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const DView* views, int T
   }
 }
 
-int launch_scan(const DView* views, int tile, Scratch sc, int splitters, cudaStream_t s) {
-  return launch_chained(k_scan, splitters + scan_blocks_hd(sc.ntiles), kScanThreads, 0, s, views, tile, sc, (uint32_t)splitters);
+int launch_scan(const DView* views, int tile, Scratch sc, int splitters, int part, cudaStream_t s) {
+  const int grid = (part == kScanAlone ? 0 : splitters) + (part == kSplitAlone ? 0 : scan_blocks_hd(sc.ntiles));
+  return launch_chained(k_scan, grid, kScanThreads, 0, s, views, tile, sc, (uint32_t)splitters, part);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -378,15 +378,15 @@ HSR_API int hsr_server_inject_alloc_failures(hsr_server s, int32_t n);
 /* ---- timing of the last completed draw sequence (CUDA events on the library stream) --
  * batch_ms spans the upload of the view descriptors to the end of the raster kernel;
  * kernel_ms holds one entry per kernel of the launch sequence, in launch order, filled when
- * profiling is on:
+ * profiling is on.  Clip and split then are launches of their own; without profiling a sequence of
+ * at most 2^21 faces clips in the emit pass's grid, and triangles are split in the scan's:
  *   [0] vertex   screen vertices (k_vertex; 0 for a sequence of at most 2^18 faces or of a position a face
  *                or more, whose cull pass computes them)
  *   [1] cull     fast accept, cull, viewport, bounding box, record (k_setup)
  *   [2] emit     shading payloads and tile counts of the surviving triangles (k_emit)
- *   [3] clip     homogeneous clipper for faces crossing a plane (k_post; 0 for a sequence of at most
- *                2^21 faces, which clips in the emit pass's grid)
- *   [4] split    0: the scan's grid splits the triangles that touch many tiles
- *   [5] scan     sub-records of those, prefix sums over the tile counts (k_scan)
+ *   [3] clip     homogeneous clipper for faces crossing a plane (k_post)
+ *   [4] split    sub-records of triangles touching many tiles (k_scan's first blocks)
+ *   [5] scan     prefix sums over the tile counts (k_scan)
  *   [6] scatter  tile lists, and the clear of tiles without triangles (k_scatter)
  *   [7] raster   coverage, depth test, shading, writes (k_raster) */
 #define HSR_KERNEL_COUNT 8
