@@ -198,8 +198,8 @@ constexpr int kSharedViews = 256;  // views whose chunk / tile bases kernels cop
 // Scratch of one launch sequence (device pointers, sized by the host).
 struct Scratch {
   Ctl* ctl;
-  uint32_t* view_done;      // [nviews] tiles finished per view, then [2 * kRasterGroups] tile counters
-                            // and the count of finished raster CTAs
+  uint32_t* view_done;      // [nviews] tiles finished per view, then [kRasterGroups] tile counters and the
+                            // count of finished raster CTAs
   RasterRec* recs;  uint32_t rec_cap;
   Payload* pay;             // [rec_cap]
   int2* clipq;      uint32_t clip_cap;   // (view, face) of faces that need clipping
@@ -215,8 +215,7 @@ struct Scratch {
   uint32_t* bins;   uint32_t bin_cap;
   int32_t ntiles;
   int32_t nviews;
-  // the raster launch's part of the tiles, [tile_lo, tile_hi), and the two counters that hand out its
-  // tiles (to warps, and at the end of the list to CTAs)
+  // the raster launch's part of the tiles, [tile_lo, tile_hi), and the counter that hands them out
   int32_t tile_lo, tile_hi;
   uint32_t* claim;
   // where the raster's last CTA (counted by `finished`) stores the control block: mapped host
@@ -290,7 +289,7 @@ int launch_place_faces(const int32_t* faces, int first, int n, const MeshArrays&
 int launch_split_normals(const float* nrm, int n, float* nx, float* ny, float* nz, float4* n4, cudaStream_t s);
 // `from` is mapped host memory or device memory; sizes are multiples of 16.
 int launch_prep(const void* from, void* to, size_t copy, void* counters, size_t zero, int max_grid, cudaStream_t s);
-int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s);
+int launch_vertex(const DView* views, int nviews, int nchunks, cudaStream_t s);
 bool culls_own_vertices(size_t faces, size_t positions);  // the cull pass needs no launch_vertex
 int launch_setup(const DView* views, int nviews, int nchunks, bool own_vertices, Scratch sc, int grid, cudaStream_t s);
 bool clips_with_emit(size_t faces);  // the emit pass's grid also clips (no launch_post)

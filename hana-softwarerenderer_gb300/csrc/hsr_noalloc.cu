@@ -129,7 +129,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   const size_t o_clip = off; off = nal(off + sizeof(float4) * (size_t)std::max(m->npos, 1));
   const size_t o_zero = off;
   const size_t o_ctl = off; off = nal(off + sizeof(Ctl));
-  const size_t o_done = off; off = nal(off + sizeof(uint32_t) * (1 + 2 + 1));
+  const size_t o_done = off; off = nal(off + sizeof(uint32_t) * (1 + 1 + 1));
   const size_t o_cnt = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_fill = off; off = nal(off + sizeof(uint32_t) * tiles);
   const size_t o_stat = off; off = nal(off + sizeof(unsigned long long) * (size_t)std::max(nscan, 1));
@@ -170,7 +170,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   sc.nviews = 1;
   sc.tile_hi = sc.ntiles;
   sc.claim = sc.view_done + 1;
-  sc.finished = sc.view_done + 3;
+  sc.finished = sc.view_done + 2;
   sc.ctl_out = (Ctl*)(h + host_bytes);
 
   // ---- the launch sequence of hsr_draw on the static scratch ------------------------------
@@ -179,7 +179,7 @@ static int noalloc_draw(Runtime* rt, const hsr_draw_desc& d) {
   const bool own = culls_own_vertices(faces, (size_t)m->npos);
   // the view, and the counters start at zero every call
   int kr = launch_prep(h, dev, host_bytes, dev + o_zero, zero_bytes, rt->num_sms * 4, s);
-  if (!kr && !own) kr = launch_vertex(dview, 1, nvch, rt->num_sms * 8, s);
+  if (!kr && !own) kr = launch_vertex(dview, 1, nvch, s);
   if (!kr) kr = launch_setup(dview, 1, nsch, own, sc, rt->num_sms * 8, s);
   if (!kr) kr = launch_emit(dview, T, sc, clips_with_emit(faces), rt->num_sms, s);
   if (!kr && !clips_with_emit(faces)) kr = launch_post(dview, T, sc, rt->num_sms * 4, s);

@@ -275,7 +275,7 @@ void Plan::layout() {
   o_vout = off; off = align_up(off + view_bytes, 256);
   o_zero = off;
   o_ctl = off; off = align_up(off + sizeof(Ctl), 256);
-  o_done = off; off = align_up(off + sizeof(uint32_t) * ((size_t)n + 2 * kRasterGroups + 1), 256);
+  o_done = off; off = align_up(off + sizeof(uint32_t) * ((size_t)n + kRasterGroups + 1), 256);
   o_cnt = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_fill = off; off = align_up(off + sizeof(uint32_t) * total_tiles, 256);
   o_stat = off; off = align_up(off + sizeof(unsigned long long) * std::max(nscan, 1), 256);
@@ -321,7 +321,7 @@ void Plan::bind(char* dev_base, char* host_base) {
   sc.tile_hi = sc.ntiles;
   sc.claim = sc.view_done + n;
   sc.ctl_out = (Ctl*)(host + host_bytes);
-  sc.finished = sc.view_done + n + 2 * kRasterGroups;
+  sc.finished = sc.view_done + n + kRasterGroups;
   sc.stash = stash_warps ? (float*)(dev + o_stash) : nullptr;
   sc.stash_warps = stash_warps;
 }
@@ -343,7 +343,7 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
   if (kr) return cuda_fail((cudaError_t)kr, "prep kernel");
   mark(1);
   const bool own = culls_own_vertices(total_faces, total_pos);
-  kr = own ? 0 : launch_vertex(dviews, n, nvch, num_sms * 8, s);
+  kr = own ? 0 : launch_vertex(dviews, n, nvch, s);
   if (kr) return cuda_fail((cudaError_t)kr, "vertex kernel");
   mark(2);
   kr = launch_setup(dviews, n, nsch, own, sc, num_sms * 8, s);
@@ -375,7 +375,7 @@ int Plan::enqueue(cudaStream_t s, int num_sms, const hsr_tuning& tu, cudaEvent_t
     if (split) {
       part.tile_lo = g > 0 ? views[split->end[g - 1]].tile_base : 0;
       part.tile_hi = split->end[g] < n ? views[split->end[g]].tile_base : sc.ntiles;
-      part.claim = sc.view_done + n + 2 * g;
+      part.claim = sc.view_done + n + g;
       if (g < ng - 1) part.ctl_out = nullptr;
     }
     kr = launch_raster(dviews, tile, part, num_sms * tu.ctas_per_sm, tu.warps_per_cta, s);

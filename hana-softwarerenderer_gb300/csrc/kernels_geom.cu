@@ -418,8 +418,7 @@ __global__ void __launch_bounds__(256) k_vertex(const DView* views, int nviews) 
   vertex_chunk_work(views[ch.view], ch);
 }
 
-int launch_vertex(const DView* views, int nviews, int nchunks, int grid, cudaStream_t s) {
-  (void)grid;
+int launch_vertex(const DView* views, int nviews, int nchunks, cudaStream_t s) {
   if (nchunks <= 0) return 0;
   return launch_chained(k_vertex, nchunks, 256, 0, s, views, nviews);
 }

@@ -291,7 +291,7 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
 template <int T, int WARPS, bool SHARED, bool HIDE>
 __device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& sc,
                                              RasterSmem<T, WARPS>& sm, const int32_t* tbase, uint32_t nlist,
-                                             const uint32_t* tile_list, uint32_t* claim) {
+                                             const uint32_t* tile_list) {
   constexpr int NPIX = T * T;
   constexpr int PPL = NPIX / 32;
   constexpr bool kKeep = TileState<NPIX>::kKeep;
@@ -319,11 +319,11 @@ __device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& 
   const uint32_t upto = (2u << lane) - 1u;  // this lane and those below
   uint32_t li = 0;  // position in the list
   if (SHARED) {
-    if (threadIdx.x == 0) sm.claim = atomicAdd(claim, 1u);
+    if (threadIdx.x == 0) sm.claim = atomicAdd(sc.claim, 1u);
     __syncthreads();
     li = sm.claim;
   } else {
-    if (lane == 0) li = atomicAdd(claim, 1u);
+    if (lane == 0) li = atomicAdd(sc.claim, 1u);
     li = __shfl_sync(kFull, li, 0);
   }
   uint32_t t = li < nlist ? tile_list[li] : ntiles;
@@ -578,7 +578,7 @@ __device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& 
       sm.frags[warp] += frags;
     }
     if (!SHARED) {
-      if (lane == 0) li = atomicAdd(claim, 1u);
+      if (lane == 0) li = atomicAdd(sc.claim, 1u);
       li = __shfl_sync(kFull, li, 0);
       if (li < nlist) {
         t_next = tile_list[li];
@@ -612,7 +612,7 @@ __device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& 
     }
     if (SHARED) {
       __syncthreads();  // the merged state and the claim word are free again
-      if (threadIdx.x == 0) sm.claim = atomicAdd(claim, 1u);
+      if (threadIdx.x == 0) sm.claim = atomicAdd(sc.claim, 1u);
       __syncthreads();
       li = sm.claim;
       if (li < nlist) t_next = tile_list[li];
@@ -630,16 +630,14 @@ __device__ __forceinline__ void raster_tiles(const DView* views, const Scratch& 
   }
 }
 
-// The list's tiles by warps, or (`shared` of them: all or none) by CTAs.  Written as if both could run:
-// as one branch the compiler lays the loops out together, and the first one is 1-2 % slower.
+// The list's tiles by warps, or (`shared`) by CTAs.  (The barrier between the two keeps the compiler from
+// laying the loops out together, with 168 bytes of spills more for 8x8 tiles.)
 template <int T, int WARPS, bool HIDE>
 __device__ __forceinline__ void raster_list(const DView* views, const Scratch& sc, RasterSmem<T, WARPS>& sm,
-                                            const int32_t* tbase, uint32_t nlist, uint32_t shared, const uint32_t* list) {
-  if (shared < nlist) raster_tiles<T, WARPS, false, HIDE>(views, sc, sm, tbase, nlist - shared, list, sc.claim);
-  if (shared > 0u) {
-    __syncthreads();
-    raster_tiles<T, WARPS, true, HIDE>(views, sc, sm, tbase, shared, list + (nlist - shared), sc.claim + 1);
-  }
+                                            const int32_t* tbase, uint32_t nlist, bool shared, const uint32_t* list) {
+  if (!shared) raster_tiles<T, WARPS, false, HIDE>(views, sc, sm, tbase, nlist, list);
+  __syncthreads();
+  if (shared) raster_tiles<T, WARPS, true, HIDE>(views, sc, sm, tbase, nlist, list);
 }
 
 // With few non-empty tiles most warps have none and the sequence lasts as long as its longest tile:
@@ -670,7 +668,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 7 : 32 / WARPS) k_ras
     const uint32_t* list = sc.tile_list + lo;
     // uniform over the grid: every warp of every CTA has a stash, or none does
     const bool stashes = TileState<T * T>::kKeep || !sc.stash || gridDim.x * (uint32_t)WARPS <= sc.stash_warps;
-    const uint32_t shared = stashes && nlist <= kSharedTilesPerCta * gridDim.x ? nlist : 0u;
+    const bool shared = stashes && nlist <= kSharedTilesPerCta * gridDim.x;
     if (sc.ctl->box_px < kHideCandidates * (float)(T * T) * (float)sc.ctl->ne_tiles)
       raster_list<T, WARPS, false>(views, sc, sm, tbase, nlist, shared, list);
     else
