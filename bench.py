@@ -24,7 +24,9 @@ serve     10,000 Poisson arrivals at two offered loads (80% of the plain path's 
           the server and for the plain path.
 roofline  every kernel of the batched step: algorithmic bytes per launch / its CUDA-event
           duration, against the measured HBM copy bandwidth; the headline is the kernel with
-          the largest share.
+          the largest share.  The kernels' times come from passes of their own after the timed
+          ones (hsr_set_profiling puts an event after each kernel and times the clipper and the
+          splitter as launches of their own).
 frame_1080p / batched_views_64   the single 1080p frame and the 64-view batched launch.
 cpu_baseline  the oracle (C restatement of the reference) on this host's cores, bounded
           sample of the same request stream.
@@ -164,14 +166,16 @@ def kernel_bytes(t: dict) -> dict:
     """Algorithmic bytes per launch of each kernel of one launch sequence (the floor a kernel
     must move to or from HBM; intermediate results the design keeps in L2 still count).
 
-    vertex : 12 B position read + 16 B screen vertex written per position.
-    cull   : 16 B face indices per face + 16 B screen vertex per position (each gathered
-             once) + a 64 B record written per triangle that reaches the raster.
-    emit   : per surviving triangle 32 B of its record and 16 B face indices read, a 4 B
-             payload index written, and the shading payload written (payload_bytes, counted
-             by the kernels: 0-128 B by shader); the packed position, normal and uv (one
-             32 B sector) of each vertex of a surviving triangle read once, records / 2
-             vertices (a closed triangle mesh has half as many vertices as faces).
+    vertex : 12 B position read + 16 B screen vertex written per position; nothing where the cull
+             pass computes them (at most 2^18 faces, or a position a face or more).
+    cull   : 16 B face indices per face + 16 B screen vertex (12 B position where it computes
+             them) per position, each gathered once + a 64 B record written per triangle that
+             reaches the raster.
+    emit   : per surviving triangle 32 B of its record and 16 B face indices read and the shading
+             payload written (payload_bytes, counted by the kernels: 0-128 B by shader); the
+             packed position, normal and uv (one 32 B sector) of each vertex of a surviving
+             triangle read once, records / 2 vertices (a closed triangle mesh has half as many
+             vertices as faces).
     clip   : per clipped face 48 B of indices and 3 x 56 B of corner attributes.
     split  : per split triangle its 192 B queue entry read.
     scan   : 4 B read + 12 B written per tile (offset, non-empty prefix, list entry).
@@ -185,10 +189,11 @@ def kernel_bytes(t: dict) -> dict:
     px, rec, pairs = t["pixels"], t["records"], t["bin_pairs"]
     rpx = t.get("raster_pixels", px)
     pay = t.get("payload_bytes", rec * 128)
+    own = t["faces"] <= 1 << 18 or t["vertices"] >= t["faces"]  # culls_own_vertices (kernels_geom.cu)
     return {
-        "vertex": t["vertices"] * 28 + t["normals"] * 28,
-        "cull": t["faces"] * 16 + t["vertices"] * 16 + rec * 64,
-        "emit": rec * 52 + pay + (rec // 2) * 32,
+        "vertex": 0 if own else t["vertices"] * 28,
+        "cull": t["faces"] * 16 + t["vertices"] * (12 if own else 16) + rec * 64,
+        "emit": rec * 48 + pay + (rec // 2) * 32,
         "clip": t["clipped_faces"] * (48 + 3 * 56),
         "split": t.get("split_triangles", 0) * 192,
         "scan": t.get("tiles", px / 64.0) * 16,
@@ -282,7 +287,6 @@ def run_ours(args, world, rank, local):
         vb = hserve.ViewBatch(rp, chunks[0])
         tuned = hsr.autotune(vb.descs, reps=2)  # outside the timed region
         vb.release()
-    hsr.set_profiling(True)
     retries0 = None
 
     # ---- value: one launch sequence of 64 requests per step ------------------------------
@@ -305,8 +309,6 @@ def run_ours(args, world, rank, local):
         if not timed:
             continue
         step_ms.append(t["batch_ms"])
-        for k, v in t["kernel_ms"].items():
-            kernel_ms[k].append(v)
         launches += int(t["launches"])
         h2d.append(int(t["h2d_bytes"]))
         d2h.append(sum(r.width * r.height * 4 for r in chunk) + int(t["d2h_bytes"]))
@@ -320,8 +322,18 @@ def run_ours(args, world, rank, local):
     total_s = dist_max(sum(step_ms) / 1000.0, world)
     value = world * frames / total_s
     counts = {k: v / args.steps for k, v in counts_sum.items()}  # per step
-    roof = roofline(kernel_ms, counts, "serve_batch64")
+    # the kernels' own times: the same steps again, with an event after each kernel
+    hsr.set_profiling(True)
+    for chunk in chunks[args.warmup:]:
+        vb = hserve.ViewBatch(rp, chunk)
+        flush.zero_()
+        torch.cuda.synchronize()
+        vb.draw_all()
+        for k, v in hsr.last_timing()["kernel_ms"].items():
+            kernel_ms[k].append(v)
+        vb.release()
     hsr.set_profiling(False)
+    roof = roofline(kernel_ms, counts, "serve_batch64")
 
     # ---- e2e: the same requests through hsr_server (all submitted at once) ----------------
     timed_reqs = [r for c in chunks[args.warmup:] for r in c]
@@ -426,6 +438,31 @@ def serve_poisson(rp, reqs, plain_fps: float, server_fps: float, args) -> dict:
     return res
 
 
+def device_times(render, steps: int, flush):
+    """`steps` timed draws after three others, L2 flushed before each: their device times, then each
+    kernel's times from as many profiled draws, and the last draw's counts."""
+    import torch
+
+    import hsr
+
+    ms, kms, t = [], {k: [] for k in hsr.KERNELS}, None
+    for profile in (False, True):
+        hsr.set_profiling(profile)
+        for i in range(3 + steps):
+            flush.zero_()
+            torch.cuda.synchronize()
+            render()
+            t = hsr.last_timing()
+            if i < 3:
+                continue
+            if not profile:
+                ms.append(t["batch_ms"])
+            for k, v in t["kernel_ms"].items() if profile else ():
+                kms[k].append(v)
+    hsr.set_profiling(False)
+    return ms, kms, t
+
+
 def run_frame(args) -> dict:
     """The single 1080p frame with its 2048^2 shadow pass (device time + plain calls)."""
     import torch
@@ -440,18 +477,7 @@ def run_frame(args) -> dict:
     old = hsr.get_tuning()
     if not args.tile:
         hsr.autotune(g.descs, reps=3)
-    hsr.set_profiling(True)
-    for _ in range(3):
-        g.render()
-    ms, kms, t = [], {k: [] for k in hsr.KERNELS}, None
-    for _ in range(args.steps):
-        flush.zero_()
-        torch.cuda.synchronize()
-        g.render()
-        t = hsr.last_timing()
-        ms.append(t["batch_ms"])
-        for k, v in t["kernel_ms"].items():
-            kms[k].append(v)
+    ms, kms, t = device_times(g.render, args.steps, flush)
     plain = []
     for _ in range(max(3, args.steps // 2)):
         flush.zero_()
@@ -459,7 +485,6 @@ def run_frame(args) -> dict:
         s0 = time.perf_counter()
         g.render(batched=False)
         plain.append((time.perf_counter() - s0) * 1000.0)
-    hsr.set_profiling(False)
     counts = {k: int(t[k]) for k in COUNT_KEYS}
     res = {"workload": FRAME_WORKLOAD, "frames_per_s": round(1000.0 / statistics.mean(ms), 2),
            "ms_p50": round(float(np.percentile(ms, 50)), 4), "ms_p99": round(float(np.percentile(ms, 99)), 4),
@@ -486,19 +511,7 @@ def run_soup(args) -> dict:
     flush = torch.empty(512 * 1024 * 1024, dtype=torch.uint8, device="cuda")
     old = hsr.get_tuning()
     tuned = hsr.autotune(g.descs, reps=2) if not args.tile else None
-    hsr.set_profiling(True)
-    for _ in range(3):
-        g.render()
-    ms, kms, t = [], {k: [] for k in hsr.KERNELS}, None
-    for _ in range(max(5, args.steps // 3)):
-        flush.zero_()
-        torch.cuda.synchronize()
-        g.render()
-        t = hsr.last_timing()
-        ms.append(t["batch_ms"])
-        for k, v in t["kernel_ms"].items():
-            kms[k].append(v)
-    hsr.set_profiling(False)
+    ms, kms, t = device_times(g.render, max(5, args.steps // 3), flush)
     counts = {k: int(t[k]) for k in COUNT_KEYS}
     s = statistics.mean(ms) / 1000.0
     res = {"workload": SOUP_WORKLOAD, "frames_per_s": round(1.0 / s, 2), "ms": round(s * 1000.0, 4),
