@@ -341,7 +341,7 @@ __device__ __forceinline__ uint32_t sub_records(int ntw, int nth) {
   return (uint32_t)((ntw + kSubTilesX - 1) / kSubTilesX) * (uint32_t)((nth + kSubTilesY - 1) / kSubTilesY);
 }
 
-// Tile rectangle of a record; T is a power of two (8 or 16).
+// Tile rectangle of a record; T is a power of two (8, 16 or 32).
 __device__ __forceinline__ void rec_tiles(const RasterRec& r, int T, int& tx0, int& ty0, int& ntw, int& nt) {
   const int ts = __ffs(T) - 1;
   const int x0 = (int)(r.xr & 0xffffu), x1 = (int)(r.xr >> 16);

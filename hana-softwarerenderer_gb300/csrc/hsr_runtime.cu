@@ -267,8 +267,9 @@ void Plan::layout() {
   big_cap = std::min<size_t>(big_cap, 0xfffff000u);
   bin_cap = std::min<size_t>(bin_cap, 0xfffff000u);
   nscan = scan_blocks((int)total_tiles);
-  // [views | chunks | per-view vertex outputs | ctl | view_done | tile_count | tile_fill |
-  //  scan_status | tile_off | ne_off | tile_list | recs | clipbuf | bins]; the zeroed part is one memset
+  // [views | per-view vertex outputs | ctl | view_done, claims | tile_count | tile_fill | scan_status |
+  //  tile_off | ne_off | tile_list | recs | payloads | clipq | bigq | bins | stash]; k_prep zeroes the part
+  // from ctl to scan_status
   size_t off = 0;
   o_views = off; off = align_up(off + sizeof(DView) * n, 256);
   host_bytes = off;

@@ -117,7 +117,7 @@ struct Runtime {
   bool profiling = false;
   uint32_t faults = 0;     // hsr_set_fault_injection: HSR_FAULT_* for hsr_draw / hsr_draw_batch
   int32_t poll_limit = 0;  // and the bounded waits' poll limit (0: default)
-  static constexpr int kEvents = HSR_KERNEL_COUNT + 2;  // start, after the memset, after each kernel
+  static constexpr int kEvents = HSR_KERNEL_COUNT + 2;  // start, after k_prep, after each kernel
   cudaEvent_t ev[kEvents] = {};
   hsr_timing timing = {};
 

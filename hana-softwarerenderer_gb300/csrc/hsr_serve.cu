@@ -324,7 +324,9 @@ static void group_requests(Slot& s, const std::vector<SrvReq*>& batch, std::vect
   size_t total = 0;
   for (const SrvReq* q : s.reqs) total += copied(q);
   const int ng = (int)std::min<size_t>({(size_t)kRasterGroups, 1 + total / kGroupBytes, s.reqs.size()});
-  // the groups' shares of the bytes, summed: decreasing, as what the last one leaves to copy shows
+  // the groups' shares of the bytes, summed: decreasing, as what the last one leaves to copy shows.  Nine
+  // mixes of 24 to 64 requests (63-194 MB copied): equal shares are 0-3.5 % slower than these,
+  // steeper ones (0.55, 0.82, 0.95) between 1.5 % faster and 4 % slower
   static const double kShare[kRasterGroups][kRasterGroups] = {
       {1.0}, {0.7, 1.0}, {0.5, 0.85, 1.0}, {0.4, 0.7, 0.9, 1.0}};
   s.split.n = ng;

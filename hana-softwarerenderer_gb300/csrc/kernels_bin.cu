@@ -4,8 +4,9 @@
 //
 // k_prep    the launch sequence's first kernel: view descriptors from the host's page-locked
 //           staging, counters to zero.
-// k_scan    sub-records of triangles that touch more than kMaxRecordTiles tiles, then exclusive prefix sums of the per-tile counts and of the non-empty tiles, single
-//           pass with decoupled look-back, and the list of non-empty tiles in tile order;
+// k_scan    sub-records of triangles that touch more than kMaxRecordTiles tiles, then exclusive
+//           prefix sums of the per-tile counts and of the non-empty tiles, single pass with
+//           decoupled look-back, and the list of non-empty tiles in tile order;
 //           block order comes from a ticket so a block only waits on blocks that already
 //           run, and every wait is bounded (error bit + give up, never a hang).
 // k_scatter writes record indices into the per-tile lists with warp-aggregated atomics;

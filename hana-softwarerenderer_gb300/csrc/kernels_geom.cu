@@ -864,7 +864,7 @@ __device__ void clip_face(bool active, const DView& v, int view, int face, int T
 // Emit pass over the records of k_setup (dense: one thread per surviving triangle): the
 // shading payload, the tile counts, and the hand-over of huge triangles to k_scan (their
 // slot becomes a hole the binning skips).  Grid-stride with warp-uniform trip counts, so
-// the warp collectives of append_small see every lane.
+// the warp collectives of append_counts see every lane.
 __device__ __forceinline__ void emit_records(const DView* views, int T, const Scratch& sc, uint32_t block,
                                              uint32_t nblocks) {
   const int lane = threadIdx.x & 31;

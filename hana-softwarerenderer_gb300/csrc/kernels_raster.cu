@@ -128,9 +128,13 @@ __device__ __forceinline__ uint32_t lowest_depth(const RasterRec& r) {
 // Candidates per pixel of the visited tiles (the records' bounding boxes, added up by the emit pass)
 // from which covered candidates are tested against lowest_depth before they are queued (HIDE): a
 // shared load and a compare a candidate, which save the divisions and the atomic of the hidden
-// ones.  The 4M-triangle soup has 26 a pixel (raster 784 -> 666 us); meshes have about 3, where
-// nearly every covered candidate wins when it is tested and the test costs 2-3 % (64 requests
-// 1,730 -> 1,786 us).
+// ones.  Raster without and with the test, soups in 1920x1080 by candidates a pixel, tile 8 | 16:
+//    5.6   86 -> 89 us  |  88 ->  88          20.7  197 -> 168 us | 240 -> 199
+//    7.3  102 -> 102    | 113 -> 110          61    447 -> 332    | 559 -> 408
+//   14.2  154 -> 143    | 180 -> 160         205  1,417 -> 963    | 1,700 -> 1,153
+// So the two are equal at 7 or a little below, and 10 leaves meshes out (about 3 a pixel), where nearly
+// every covered candidate wins when it is tested (64 requests 1,730 -> 1,786 us).  The 4M-triangle
+// soup has 26: 784 -> 666 us.
 constexpr float kHideCandidates = 10.f;
 
 // Pixel of candidate i: q = i - m.x counts a record's range in row-major order, width w;
