@@ -392,6 +392,10 @@ __device__ __forceinline__ void vertex_chunk_work(const DView& v, const Chunk& c
   // contiguous span; the loads of a thread are issued before any is used
   constexpr int kPer = kVertexChunk / 256;
   const int i0 = ch.begin + (int)threadIdx.x;
+  float mvp[16];  // loaded once (read again after each store: 64 requests 83 -> 103 us)
+#pragma unroll
+  for (int k = 0; k < 16; k++) mvp[k] = v.mvp[k];
+  float4* const sv = v.sv;
   float xs[kPer], ys[kPer], zs[kPer];
 #pragma unroll
   for (int k = 0; k < kPer; k++) {
@@ -405,7 +409,7 @@ __device__ __forceinline__ void vertex_chunk_work(const DView& v, const Chunk& c
   for (int k = 0; k < kPer; k++) {
     const int i = i0 + 256 * k;
     if (i >= ch.end) break;
-    v.sv[i] = screen_vertex(mat_vec(v.mvp, xs[k], ys[k], zs[k], 1.f));
+    sv[i] = screen_vertex(mat_vec(mvp, xs[k], ys[k], zs[k], 1.f));
   }
 }
 

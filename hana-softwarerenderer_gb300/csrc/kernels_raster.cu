@@ -208,6 +208,11 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
   constexpr int NF4 = payload_f4_of<S>();
   const int lane = threadIdx.x & 31;
   uint32_t shaded = 0;
+  // (the compiler reads a descriptor's field again after a store: 64 requests 1,554 -> 1,567 us)
+  const int W = v.W, H = v.H;
+  uint32_t* const color = v.color;
+  float* const depth = v.depth;
+  uint32_t* const prims = v.prim;
 #pragma unroll 1
   for (int q = q0; q < PPL; q += qstep) {
     // the next row's payloads start on their way to L1 while this row is shaded (a whole tile's at
@@ -218,11 +223,11 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
     }
     const int p = lane + 32 * q;
     const int x = ox + p % T, y = oy + p / T;
-    if (x >= v.W || y >= v.H) continue;
-    const size_t idx = (size_t)y * v.W + x;
+    if (x >= W || y >= H) continue;
+    const size_t idx = (size_t)y * W + x;
     uint32_t ri = st.win[p].y;
     // without the fused clear the buffer's depth enters here, after the fragments' minimum
-    if (!clear && ri != kNone && st.key(p) >= buffer_key(__ldcg(&v.depth[idx]))) ri = kNone;
+    if (!clear && ri != kNone && st.key(p) >= buffer_key(__ldcg(&depth[idx]))) ri = kNone;
     if (ri != kNone) {
       shaded++;
       float b0, b1, b2;
@@ -253,14 +258,14 @@ __device__ __forceinline__ uint32_t shade_tile(const DView& v, const Scratch& sc
         for (int k = 0; k < NF4; k++) reinterpret_cast<float4*>(P)[k] = src[k];
       }
       const uint32_t prim = v.prim_base + (seq >> kSeqFaceShift) + 1u;
-      const uint32_t alpha = clear ? v.clear_rgba : __ldcg(&v.color[idx]);
-      v.color[idx] = pack_rgb(fragment_s<S>(v, P, b0, b1, b2, prim, bt), alpha);
-      if (v.depth) v.depth[idx] = from_ord(st.z[p]);
-      if (v.prim) v.prim[idx] = prim;
+      const uint32_t alpha = clear ? v.clear_rgba : __ldcg(&color[idx]);
+      color[idx] = pack_rgb(fragment_s<S>(v, P, b0, b1, b2, prim, bt), alpha);
+      if (depth) depth[idx] = from_ord(st.z[p]);
+      if (prims) prims[idx] = prim;
     } else if (clear) {
-      v.color[idx] = v.clear_rgba;
-      if (v.depth) v.depth[idx] = v.clear_depth;
-      if (v.prim) v.prim[idx] = 0u;
+      color[idx] = v.clear_rgba;
+      if (depth) depth[idx] = v.clear_depth;
+      if (prims) prims[idx] = 0u;
     }
   }
   return shaded;
