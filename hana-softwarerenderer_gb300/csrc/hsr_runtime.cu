@@ -599,9 +599,9 @@ static int place_normals(MeshObj* m, const float* nrm) {
 }
 
 // The caller's positions and faces into the mesh's arrays in the library's order.  The raw arrays, codes and
-// places (a 4M-triangle soup: 385 MB) come from a pool of their own that keeps nothing: the memory
-// goes back to the device when the stream has been waited for.  False, with nothing written, where
-// they cannot be had.
+// places (a 4M-triangle soup: 385 MB) come from a pool of their own, and go back to the device
+// when the stream has been waited for, but for kUploadPoolKeep.  False, with nothing written, where they
+// cannot be had.
 static bool order_mesh(MeshObj* m, const MeshArrays& to, const float* pos, const int32_t* faces, cudaError_t& e) {
   cudaStream_t st = g_rt->stream;
   const size_t npos = (size_t)m->npos, nfaces = (size_t)m->nfaces;
@@ -695,8 +695,10 @@ int hsr_init(int device) {
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = device;
-  e = cudaMemPoolCreate(&rt->upload_pool, &props);  // (keeps nothing: its release threshold is zero)
+  e = cudaMemPoolCreate(&rt->upload_pool, &props);
   if (e != cudaSuccess) { delete rt; return cuda_fail(e, "hsr_init: memory pool"); }
+  uint64_t upload_keep = kUploadPoolKeep;
+  cudaMemPoolSetAttribute(rt->upload_pool, cudaMemPoolAttrReleaseThreshold, &upload_keep);
   for (int k = 0; k < Runtime::kEvents; k++) {
     e = cudaEventCreate(&rt->ev[k]);
     if (e != cudaSuccess) { delete rt; return cuda_fail(e, "cudaEventCreate"); }

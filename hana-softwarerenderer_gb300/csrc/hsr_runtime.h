@@ -97,6 +97,9 @@ struct Plan {
 int first_reclear(const hsr_draw_desc* d, int n);
 
 constexpr size_t kFixedHostBytes = 4096;
+// What Runtime::upload_pool keeps for the next upload: the scratch of a mesh of half a million faces (82k
+// faces upload in 1.40 ms where the pool keeps nothing, in 1.31 ms with it).
+constexpr size_t kUploadPoolKeep = (size_t)32 << 20;
 
 struct Runtime {
   int device = 0;

@@ -125,9 +125,10 @@ HSR_API int hsr_abi_version(void);
  * normalises them in place on every access (model.cpp:108-111), which is the identity
  * for normals that are fixed points of Vector3f::normalize().
  * While the call runs it holds device scratch beside the mesh's own arrays: for 2^15 faces and
- * more, 16-20 bytes a position and 36-40 a face, which are given back before it returns (a mesh whose
- * scratch cannot be had is kept in the caller's order, with the same results); else, and for
- * hsr_mesh_update_normals, up to 36 MiB, which stay in the device's stream-ordered pool. */
+ * more, 16-20 bytes a position and 36-40 a face, which are given back before it returns but for 32 MiB
+ * (a mesh whose scratch cannot be had is kept in the caller's order, with the same results);
+ * else, and for hsr_mesh_update_normals, up to 36 MiB, which stay in the device's stream-ordered
+ * pool. */
 HSR_API int hsr_mesh_upload(const float* pos, int32_t npos, const float* nrm, int32_t nnrm,
                     const float* uv, int32_t nuv, const int32_t* faces, int32_t nfaces,
                     hsr_mesh* out);
